@@ -80,30 +80,20 @@ __device__ __forceinline__ float2 ld(const float2 *__restrict__ v, int c) { retu
 #define DF_ZCHUNK(A)                                                   \
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;          \
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;          \
-    const int k0 = blockIdx.z * DF_KZ + 1;                            \
-    const int k1 = min(k0 + DF_KZ - 1, (A).hi.n2);                    \
+    const int k0 = blockIdx.z * kz + 1;                               \
+    const int k1 = min(k0 + kz - 1, (A).hi.n2);                       \
     const bool in = i <= (A).hi.n0 && j <= (A).hi.n1;
-
-constexpr int DF_KZ = 32;
 
 // operator coefficient of cell c from its hi (FP32 copy) and lo parts
 __device__ __forceinline__ float2 cf(const float *hi, const float *lo, int c) { return make_float2(hi[c], lo[c]); }
 
 }  // namespace
 
-Launch3 df_launch(const DfOp &A)
-{
-    Launch3 l;
-    l.block = dim3(32, 4, 1);
-    l.grid = dim3((A.hi.n0 + 31) / 32, (A.hi.n1 + 3) / 4, (A.hi.n2 + DF_KZ - 1) / DF_KZ);
-    return l;
-}
-
 // q = A p, and the block partials of (p, q) (FP64 products and sums) and of
 // the sum of q (for the mean of A p in all-Neumann systems, which is zero in
 // exact arithmetic: double-float per thread, FP64 across threads)
 __global__ void __launch_bounds__(128, 8) k_spmv_df(DfOp A, const float2 *__restrict__ p, float2 *__restrict__ q,
-                                                 double *__restrict__ part, int n0)
+                                                 double *__restrict__ part, int n0, int kz)
 {
     DF_ZCHUNK(A);
     double v = 0.0;
@@ -143,7 +133,7 @@ __global__ void __launch_bounds__(128, 8) k_spmv_df(DfOp A, const float2 *__rest
 // (r, z) for beta: r double-float, z the FP32 preconditioned residual; FP64
 // products and sums
 __global__ void __launch_bounds__(128) k_dot_rz_df(DfOp A, const float2 *__restrict__ r, const float *__restrict__ z,
-                                                   double *__restrict__ part)
+                                                   double *__restrict__ part, int kz)
 {
     DF_ZCHUNK(A);
     double v = 0.0;
@@ -162,7 +152,7 @@ __global__ void __launch_bounds__(128) k_dot_rz_df(DfOp A, const float2 *__restr
 __global__ void __launch_bounds__(128) k_cg_update_df(DfOp A, float2 *__restrict__ x, float2 *__restrict__ r,
                                                       const float2 *__restrict__ p, const float2 *__restrict__ q,
                                                       float *__restrict__ rlow, float *__restrict__ x0, float first,
-                                                      const double *__restrict__ scal, double *__restrict__ part)
+                                                      const double *__restrict__ scal, double *__restrict__ part, int kz)
 {
     DF_ZCHUNK(A);
     double v = 0.0;
@@ -189,7 +179,7 @@ __global__ void __launch_bounds__(128) k_cg_update_df(DfOp A, float2 *__restrict
 
 // p = z + beta p (p = z on the first call)
 __global__ void __launch_bounds__(128) k_pupdate_df(DfOp A, const float *__restrict__ z, float2 *__restrict__ p,
-                                                    const double *__restrict__ scal, int first)
+                                                    const double *__restrict__ scal, int first, int kz)
 {
     DF_ZCHUNK(A);
     if (!in) return;
@@ -231,9 +221,9 @@ __global__ void k_df_to_double(const float2 *src, double *dst, int n)
 void df_spmv_dot(const DfOp &A, const float2 *p, float2 *q, Reducer &R, bool singular, cudaStream_t st,
                  int *launches, KTimer *kt)
 {
-    Launch3 l = df_launch(A);
+    const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     const int id = kt_begin(kt, KC_SPMV, st);
-    k_spmv_df<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks);
+    k_spmv_df<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks, l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     reduce_alpha(R, (int)nblocks(l), singular, st, launches);
@@ -241,8 +231,8 @@ void df_spmv_dot(const DfOp &A, const float2 *p, float2 *q, Reducer &R, bool sin
 
 void df_dot_rz(const DfOp &A, const float2 *r, const float *z, Reducer &R, cudaStream_t st, int *launches)
 {
-    Launch3 l = df_launch(A);
-    k_dot_rz_df<<<l.grid, l.block, 0, st>>>(A, r, z, R.partials);
+    const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
+    k_dot_rz_df<<<l.grid, l.block, 0, st>>>(A, r, z, R.partials, l.kz);
     *launches += 1;
     reduce_beta(R, (int)nblocks(l), st, launches);
 }
@@ -250,9 +240,9 @@ void df_dot_rz(const DfOp &A, const float2 *r, const float *z, Reducer &R, cudaS
 void df_cg_update(const DfOp &A, float2 *x, float2 *r, const float2 *p, const float2 *q, float *rlow, float *x0,
                   double first, Reducer &R, cudaStream_t st, int *launches, KTimer *kt)
 {
-    Launch3 l = df_launch(A);
+    const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     const int id = kt_begin(kt, KC_CGUPDATE, st);
-    k_cg_update_df<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, x0, (float)first, R.scal, R.partials);
+    k_cg_update_df<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, x0, (float)first, R.scal, R.partials, l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     reduce_to(R, (int)nblocks(l), S_RR, st, launches);
@@ -261,8 +251,8 @@ void df_cg_update(const DfOp &A, float2 *x, float2 *r, const float2 *p, const fl
 void df_pupdate(const DfOp &A, const float *z, float2 *p, const double *scal, bool first, cudaStream_t st,
                 int *launches)
 {
-    Launch3 l = df_launch(A);
-    k_pupdate_df<<<l.grid, l.block, 0, st>>>(A, z, p, scal, first ? 1 : 0);
+    const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
+    k_pupdate_df<<<l.grid, l.block, 0, st>>>(A, z, p, scal, first ? 1 : 0, l.kz);
     *launches += 1;
 }
 

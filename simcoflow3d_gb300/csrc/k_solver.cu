@@ -88,30 +88,20 @@ void reduce_to(Reducer &R, int nblocks, int slot, cudaStream_t st, int *launches
 // ---------------------------------------------------------------------------
 // FP64 CG kernels on the fine level
 
-// Fine-level FP64 kernels march KZ cells along k per thread: the k-neighbours
-// stay in registers and the FP64 block reduction (costly on this GPU's FP64
-// pipe) is paid once per KZ cells.
-constexpr int KZ = 32;
-
-inline Launch3 launch_zchunk(int n0, int n1, int n2)
-{
-    Launch3 l;
-    l.block = dim3(32, 4, 1);
-    l.grid = dim3((n0 + 31) / 32, (n1 + 3) / 4, (n2 + KZ - 1) / KZ);
-    return l;
-}
-
+// Fine-level CG kernels march kz cells along k per thread (launch_march):
+// the k-neighbours stay in registers and the FP64 block reduction (costly on
+// this GPU's FP64 pipe) is paid once per kz cells.
 #define ZCHUNK_IJK(L)                                                  \
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;          \
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;          \
-    const int k0 = blockIdx.z * KZ + 1;                               \
-    const int k1 = min(k0 + KZ - 1, (L).n2);                          \
+    const int k0 = blockIdx.z * kz + 1;                               \
+    const int k1 = min(k0 + kz - 1, (L).n2);                          \
     const bool in = i <= (L).n0 && j <= (L).n1;
 
 // q = A p and the block partials of (p, q) and of the sum of q (q is zero on
 // inactive cells, whose p is zero and which couple to nothing).
 __global__ void __launch_bounds__(128) k_spmv_dot(LevelView<double> A, const double *__restrict__ p,
-                                                  double *__restrict__ q, double *__restrict__ part, int n0)
+                                                  double *__restrict__ q, double *__restrict__ part, int n0, int kz)
 {
     ZCHUNK_IJK(A);
     double v = 0.0, sq = 0.0;
@@ -170,9 +160,9 @@ void reduce_alpha(Reducer &R, int nblocks, bool singular, cudaStream_t st, int *
 void cg_spmv_dot(const LevelView<double> &A, const double *p, double *q, Reducer &R, bool singular,
                  cudaStream_t st, int *launches, KTimer *kt)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
+    const March l = launch_march(A.n0, A.n1, A.n2);
     const int id = kt_begin(kt, KC_SPMV, st);
-    k_spmv_dot<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks);
+    k_spmv_dot<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks, l.kz);
     kt_end(kt, id, st);
     k_reduce_alpha<<<1, 1024, 0, st>>>(R.partials, (int)nblocks(l), R.max_blocks, R.scal, singular ? 1 : 0);
     *launches += 2;
@@ -187,7 +177,7 @@ __global__ void __launch_bounds__(128) k_cg_update(LevelView<double> A, double *
                                                    double *__restrict__ r, const double *__restrict__ p,
                                                    const double *__restrict__ q, T *__restrict__ rlow,
                                                    LevelView<T> L0, T *__restrict__ x0, T first,
-                                                   const double *__restrict__ scal, double *__restrict__ part)
+                                                   const double *__restrict__ scal, double *__restrict__ part, int kz)
 {
     ZCHUNK_IJK(A);
     double v = 0.0;
@@ -213,22 +203,22 @@ void cg_update(const LevelView<double> &A, double *x, double *r, const double *p
                const LevelView<T> &L0, T *x0, double first, Reducer &R, cudaStream_t st, int *launches,
                KTimer *kt)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
+    const March l = launch_march(A.n0, A.n1, A.n2);
     const int id = kt_begin(kt, KC_CGUPDATE, st);
-    k_cg_update<T><<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, L0, x0, (T)first, R.scal, R.partials);
+    k_cg_update<T><<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, L0, x0, (T)first, R.scal, R.partials, l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     reduce_to(R, (int)nblocks(l), S_RR, st, launches);
 }
 
 // (r, z): in mixed mode r is taken from its FP32 copy (the V-cycle's rhs) and
-// the products are formed in FP32, accumulated per thread in FP32 over KZ
+// the products are formed in FP32, accumulated per thread in FP32 over kz
 // cells and across threads in FP64; z is an FP32 preconditioner output, so
 // this loses nothing that matters for beta.  FP64 mode: FP64 throughout.
 template <typename T>
 __global__ void __launch_bounds__(128) k_dot_rz(LevelView<double> A, const double *__restrict__ r,
                                                 const T *__restrict__ rlow, const T *__restrict__ z,
-                                                double *__restrict__ part)
+                                                double *__restrict__ part, int kz)
 {
     ZCHUNK_IJK(A);
     double v = 0.0;
@@ -250,8 +240,8 @@ template <typename T>
 void cg_dot_rz(const LevelView<double> &A, const double *r, const T *rlow, const T *z, Reducer &R, cudaStream_t st,
                int *launches)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
-    k_dot_rz<T><<<l.grid, l.block, 0, st>>>(A, r, rlow, z, R.partials);
+    const March l = launch_march(A.n0, A.n1, A.n2);
+    k_dot_rz<T><<<l.grid, l.block, 0, st>>>(A, r, rlow, z, R.partials, l.kz);
     k_reduce<<<1, 1024, 0, st>>>(R.partials, (int)nblocks(l), R.scal, 0, RM_BETA);
     *launches += 2;
 }
@@ -264,7 +254,8 @@ void reduce_beta(Reducer &R, int nblocks, cudaStream_t st, int *launches)
 
 template <typename T>
 __global__ void __launch_bounds__(128) k_pupdate(LevelView<double> A, const T *__restrict__ z,
-                                                 double *__restrict__ p, const double *__restrict__ scal, int first)
+                                                 double *__restrict__ p, const double *__restrict__ scal, int first,
+                                                 int kz)
 {
     ZCHUNK_IJK(A);
     if (!in) return;
@@ -280,8 +271,8 @@ template <typename T>
 void cg_pupdate(const LevelView<double> &A, const T *z, double *p, const double *scal, bool first, cudaStream_t st,
                 int *launches)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
-    k_pupdate<T><<<l.grid, l.block, 0, st>>>(A, z, p, scal, first ? 1 : 0);
+    const March l = launch_march(A.n0, A.n1, A.n2);
+    k_pupdate<T><<<l.grid, l.block, 0, st>>>(A, z, p, scal, first ? 1 : 0, l.kz);
     *launches += 1;
 }
 
@@ -313,7 +304,8 @@ __global__ void __launch_bounds__(1024) k_reduce2(const double *__restrict__ par
 }
 
 __global__ void __launch_bounds__(128) k_sum_count(LevelView<double> A, const unsigned char *__restrict__ act,
-                                                   const double *__restrict__ v, double *__restrict__ part, int n0)
+                                                   const double *__restrict__ v, double *__restrict__ part, int n0,
+                                                   int kz)
 {
     ZCHUNK_IJK(A);
     double s = 0.0, cnt = 0.0;
@@ -333,7 +325,7 @@ __global__ void __launch_bounds__(128) k_sum_count(LevelView<double> A, const un
 
 __global__ void __launch_bounds__(128) k_center_norm(LevelView<double> A, const unsigned char *__restrict__ act,
                                                      double *__restrict__ b, const double *__restrict__ scal,
-                                                     int singular, double *__restrict__ part)
+                                                     int singular, double *__restrict__ part, int kz)
 {
     ZCHUNK_IJK(A);
     double s = 0.0;
@@ -359,8 +351,8 @@ void reduce2_to(Reducer &R, int nblocks, int mode, cudaStream_t st, int *launche
 void active_mean(const LevelView<double> &A, const unsigned char *active, const double *v, Reducer &R,
                  cudaStream_t st, int *launches)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
-    k_sum_count<<<l.grid, l.block, 0, st>>>(A, active, v, R.partials, R.max_blocks);
+    const March l = launch_march(A.n0, A.n1, A.n2);
+    k_sum_count<<<l.grid, l.block, 0, st>>>(A, active, v, R.partials, R.max_blocks, l.kz);
     *launches += 1;
     reduce2_to(R, (int)nblocks(l), 0, st, launches);
 }
@@ -368,14 +360,14 @@ void active_mean(const LevelView<double> &A, const unsigned char *active, const 
 void rhs_prologue(const LevelView<double> &A, const unsigned char *active, double *b, bool singular, Reducer &R,
                   cudaStream_t st, int *launches)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
+    const March l = launch_march(A.n0, A.n1, A.n2);
     const int nb = (int)nblocks(l);
     if (singular) {
-        k_sum_count<<<l.grid, l.block, 0, st>>>(A, active, b, R.partials, R.max_blocks);
+        k_sum_count<<<l.grid, l.block, 0, st>>>(A, active, b, R.partials, R.max_blocks, l.kz);
         k_reduce2<<<1, 1024, 0, st>>>(R.partials, nb, R.max_blocks, R.scal, 0);
         *launches += 2;
     }
-    k_center_norm<<<l.grid, l.block, 0, st>>>(A, active, b, R.scal, singular ? 1 : 0, R.partials);
+    k_center_norm<<<l.grid, l.block, 0, st>>>(A, active, b, R.scal, singular ? 1 : 0, R.partials, l.kz);
     k_reduce<<<1, 1024, 0, st>>>(R.partials, nb, R.scal, S_BB, RM_STORE);
     *launches += 2;
 }
@@ -383,7 +375,7 @@ void rhs_prologue(const LevelView<double> &A, const unsigned char *active, doubl
 __global__ void __launch_bounds__(128) k_final_residual(LevelView<double> A, const unsigned char *__restrict__ act,
                                                         const double *__restrict__ b, const double *__restrict__ x,
                                                         double *__restrict__ r, int singular,
-                                                        double *__restrict__ part, int n0)
+                                                        double *__restrict__ part, int n0, int kz)
 {
     ZCHUNK_IJK(A);
     double s = 0.0, sx = 0.0;
@@ -408,15 +400,15 @@ __global__ void __launch_bounds__(128) k_final_residual(LevelView<double> A, con
 void final_residual(const LevelView<double> &A, const unsigned char *active, const double *b, const double *x,
                     double *r, bool singular, Reducer &R, cudaStream_t st, int *launches)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
+    const March l = launch_march(A.n0, A.n1, A.n2);
     const int nb = (int)nblocks(l);
-    k_final_residual<<<l.grid, l.block, 0, st>>>(A, active, b, x, r, singular ? 1 : 0, R.partials, R.max_blocks);
+    k_final_residual<<<l.grid, l.block, 0, st>>>(A, active, b, x, r, singular ? 1 : 0, R.partials, R.max_blocks, l.kz);
     k_reduce2<<<1, 1024, 0, st>>>(R.partials, nb, R.max_blocks, R.scal, 1);
     *launches += 2;
 }
 
 __global__ void __launch_bounds__(128) k_shift(LevelView<double> A, const unsigned char *__restrict__ act,
-                                               double *__restrict__ x, const double *__restrict__ scal)
+                                               double *__restrict__ x, const double *__restrict__ scal, int kz)
 {
     ZCHUNK_IJK(A);
     if (!in) return;
@@ -429,8 +421,8 @@ __global__ void __launch_bounds__(128) k_shift(LevelView<double> A, const unsign
 void shift_solution(const LevelView<double> &A, const unsigned char *active, double *x, const double *scal,
                     cudaStream_t st, int *launches)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
-    k_shift<<<l.grid, l.block, 0, st>>>(A, active, x, scal);
+    const March l = launch_march(A.n0, A.n1, A.n2);
+    k_shift<<<l.grid, l.block, 0, st>>>(A, active, x, scal, l.kz);
     *launches += 1;
 }
 
@@ -1679,8 +1671,8 @@ void probe_prolong(MgLevel<T> &F, MgLevel<T> &C, const ChebCoef &cc, cudaStream_
 
 void probe_spmv(const LevelView<double> &A, const double *p, double *q, Reducer &R, cudaStream_t st)
 {
-    Launch3 l = launch_zchunk(A.n0, A.n1, A.n2);
-    k_spmv_dot<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks);
+    const March l = launch_march(A.n0, A.n1, A.n2);
+    k_spmv_dot<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks, l.kz);
 }
 
 template void probe_smooth<float>(MgLevel<float> &, const ChebCoef &, cudaStream_t);

@@ -94,6 +94,30 @@ inline Launch3 launch_interior(int n0, int n1, int n2)
     return l;
 }
 
+// A launch of 32 x 4 columns per block whose threads march kz cells along k.
+// A longer march pays a block's FP64 reduction and first loads less often,
+// but a column segment is a serial chain (about 1.4 us per cell and launch of
+// the double-float SpMV): kz is the longest of 32, 16, .., 2 that still fills
+// one wave of eight blocks on each of the 152 SMs.  Measured, projections at
+// fixed 32 / one wave / four waves: 40^3 mixed 2.00 / 1.46 / 1.45 ms, 64^3 FP64
+// 3.27 / 2.64 / 2.64 ms, 147x93x121 mixed 4.77 / 4.12 / 4.65 ms, 256^3 mixed
+// 14.65 / 14.66 / 14.77 ms.
+struct March : Launch3 {
+    int kz;
+};
+constexpr long long MARCH_WAVE = 152 * 8;
+
+inline March launch_march(int n0, int n1, int n2)
+{
+    March l;
+    l.block = dim3(32, 4, 1);
+    const long long cols = (long long)((n0 + 31) / 32) * ((n1 + 3) / 4);
+    l.kz = 32;
+    while (l.kz > 2 && cols * ((n2 + l.kz - 1) / l.kz) < MARCH_WAVE) l.kz /= 2;
+    l.grid = dim3((n0 + 31) / 32, (n1 + 3) / 4, (n2 + l.kz - 1) / l.kz);
+    return l;
+}
+
 inline unsigned nblocks(const Launch3 &l) { return l.grid.x * l.grid.y * l.grid.z; }
 
 // Block-wide FP64 sum; result valid in thread 0.  blockDim.x*y*z <= 1024.
