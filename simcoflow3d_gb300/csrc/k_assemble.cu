@@ -76,12 +76,10 @@ __device__ __forceinline__ double lamda_of(const AsmArgs &a, int gc, int gn)
 // innermost), that assigned it within the same face call.  Each thread
 // marches one (i,j) column in k -- exactly a contiguous run of that loop
 // order -- and carries the twelve (face, W/D) values in registers.  For
-// parallelism a column is cut into segments of KSEG cells; segments are
-// contiguous runs of the loop order too.  Cells with no earlier assignment
+// parallelism a column is cut into segments of a.kseg cells (asm_kseg);
+// segments are contiguous runs of the loop order too.  Cells with no earlier assignment
 // inside their segment ("head" cells) are listed and resolved from
 // per-segment and per-group summaries (k_pocoef_heads).
-constexpr int KSEG = SCF_KSEG;
-
 namespace {
 __device__ __forceinline__ double beta_of(int pc, int pn, double lam, double betap, double betam)
 {
@@ -184,10 +182,10 @@ __global__ void __launch_bounds__(128) k_pocoef(AsmArgs a)
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     if (i > d.I || j > d.J) return;
-    const int nsk = (d.K + KSEG - 1) / KSEG, sk = blockIdx.z;
+    const int nsk = (d.K + a.kseg - 1) / a.kseg, sk = blockIdx.z;
     const int col = (i - 1) * d.J + (j - 1);   // column index in loop order
     const int seg = col * nsk + sk;            // segment index in loop order
-    const int kbeg = sk * KSEG + 1, kend = min(kbeg + KSEG - 1, d.K);
+    const int kbeg = sk * a.kseg + 1, kend = min(kbeg + a.kseg - 1, d.K);
     const int sy = d.gx, sz = d.gx * d.gy;
     const int goff[6] = {-1, -sy, -sz, 1, sy, sz};
     double carryW[6], carryD[6];
@@ -264,28 +262,28 @@ __global__ void __launch_bounds__(128) k_pocoef(AsmArgs a)
     a.col_mask[seg] = (unsigned short)m;
 }
 
-// Group summaries: the last assignment of each (face, W/D) stream within
-// 64 consecutive segments.
-__global__ void k_pocoef_groups(AsmArgs a, int ncol, int ngrp)
+// Group summaries: the last assignment of each (face, W/D) stream within 64
+// consecutive segments.  One warp per group: each lane reads two segments'
+// masks, a ballot per stream finds the last segment that assigned it, and
+// lane s fetches stream s's value.  (One thread walking the 64 segments was a
+// chain of dependent loads: 52 us at 147x93x121.)
+__global__ void __launch_bounds__(128) k_pocoef_groups(AsmArgs a, int ncol, int ngrp)
 {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (g >= ngrp) return;
-    double v[12];
+    const int c0 = g * 64;
+    const unsigned m0 = c0 + lane < ncol ? a.col_mask[c0 + lane] : 0u;
+    const unsigned m1 = c0 + 32 + lane < ncol ? a.col_mask[c0 + 32 + lane] : 0u;
+    int last = -1;
     unsigned m = 0;
 #pragma unroll
-    for (int s = 0; s < 12; ++s) v[s] = 0.0;
-    const int c1 = min(ncol, (g + 1) * 64);
-    for (int c = g * 64; c < c1; ++c) {
-        const unsigned cm = a.col_mask[c];
-        if (!cm) continue;
-#pragma unroll
-        for (int s = 0; s < 12; ++s)
-            if (cm & (1u << s)) v[s] = a.col_val[(long long)c * 12 + s];
-        m |= cm;
+    for (int s = 0; s < 12; ++s) {
+        const unsigned b0 = __ballot_sync(0xffffffffu, (m0 >> s) & 1u), b1 = __ballot_sync(0xffffffffu, (m1 >> s) & 1u);
+        if (b0 | b1) m |= 1u << s;
+        if (lane == s && (b0 | b1)) last = b1 ? c0 + 63 - __clz(b1) : c0 + 31 - __clz(b0);
     }
-#pragma unroll
-    for (int s = 0; s < 12; ++s) a.grp_val[(long long)g * 12 + s] = v[s];
-    a.grp_mask[g] = (unsigned short)m;
+    if (lane < 12) a.grp_val[(long long)g * 12 + lane] = last >= 0 ? a.col_val[(long long)last * 12 + lane] : 0.0;
+    if (lane == 0) a.grp_mask[g] = (unsigned short)m;
 }
 
 // Head cells: the carried value comes from the latest earlier segment (first
@@ -301,8 +299,8 @@ __global__ void k_pocoef_heads(AsmArgs a, unsigned count)
     const long long L = e >> 4;
     const int col = (int)(L / d.K), k = (int)(L % d.K) + 1;
     const int i = col / d.J + 1, j = col % d.J + 1;
-    const int nsk = (d.K + KSEG - 1) / KSEG;
-    const int seg = col * nsk + (k - 1) / KSEG;
+    const int nsk = (d.K + a.kseg - 1) / a.kseg;
+    const int seg = col * nsk + (k - 1) / a.kseg;
     const unsigned bit = 1u << s;
     double beta = a.stale_init;
     bool found = false;
@@ -459,7 +457,7 @@ __device__ __forceinline__ void op_issue(const AsmArgs &a, double *sd, int *si, 
 }
 
 // Matrix rows, FP32 copies and right-hand side of each cell (a block is
-// 32 x 4 columns, each thread marches one KSEG segment along k).  The
+// 32 x 4 columns, each thread marches one segment of a.kseg cells along k).  The
 // inputs of cell k+1 are copied into shared memory while cell k is
 // computed (two stages).
 template <bool MIXED>
@@ -473,7 +471,7 @@ __global__ void __launch_bounds__(OP_THREADS, 3) k_operator(AsmArgs a, OpArgs o)
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     if (i > d.I || j > d.J) return;
-    const int kbeg = blockIdx.z * KSEG + 1, kend = min(kbeg + KSEG - 1, d.K);
+    const int kbeg = blockIdx.z * a.kseg + 1, kend = min(kbeg + a.kseg - 1, d.K);
     const int *fl = a.flag;
     TermMemo tm[6];
 #pragma unroll
@@ -626,7 +624,7 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
         *launches += 1;
         *stale_count_host = 0;
     } else {
-        dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + KSEG - 1) / KSEG);
+        dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + a.kseg - 1) / a.kseg);
         k_phase<<<2 * 152 * 8, 256, 0, st>>>(a);
         k_pocoef<<<g, b, 0, st>>>(a);
         *launches += 2;
@@ -636,8 +634,8 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
     unsigned cnt = *stale_count_host;
     if (cnt > a.stale_cap) cnt = a.stale_cap;
     if (cnt) {
-        const int ncol = d.I * d.J * ((d.K + KSEG - 1) / KSEG), ngrp = (ncol + 63) / 64;
-        k_pocoef_groups<<<(ngrp + 127) / 128, 128, 0, st>>>(a, ncol, ngrp);
+        const int ncol = d.I * d.J * ((d.K + a.kseg - 1) / a.kseg), ngrp = (ncol + 63) / 64;
+        k_pocoef_groups<<<(ngrp + 3) / 4, 128, 0, st>>>(a, ncol, ngrp);
         k_pocoef_heads<<<(cnt + 127) / 128, 128, 0, st>>>(a, cnt);
         *launches += 2;
     }
@@ -649,7 +647,7 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
         k_pocoef_boundary<<<g, 256, 0, st>>>(a);
         *launches += 1;
     }
-    dim3 ob(32, 4), og((d.I + 31) / 32, (d.J + 3) / 4, (d.K + KSEG - 1) / KSEG);
+    dim3 ob(32, 4), og((d.I + 31) / 32, (d.J + 3) / 4, (d.K + a.kseg - 1) / a.kseg);
     // the staged inputs need more than the default 48 KB of dynamic shared
     // memory (set per device, so on every call)
     cudaFuncSetAttribute(k_operator<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OP_SMEM);

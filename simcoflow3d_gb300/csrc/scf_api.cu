@@ -311,6 +311,7 @@ AsmArgs asm_args(scf_ctx *ctx)
     a.flags = ctx->flags;
     a.phase = ctx->phase;
     a.rdt = 1.0 / ctx->dt;
+    a.kseg = asm_kseg(ctx->d.I, ctx->d.J, ctx->d.K);
     return a;
 }
 
@@ -1002,8 +1003,9 @@ int scf_ctx_create(scf_ctx **out, int32_t imax, int32_t jmax, int32_t kmax, cons
     A(ctx->stale_count, 1); A(ctx->flags, 4);
     ctx->stale_cap = (unsigned)(n < (1LL << 30) ? n : (1LL << 30));
     A(ctx->stale_list, ctx->stale_cap);
-    // per-segment summaries of the coefficient kernel (segments of 32 cells)
-    const long long ncol = (long long)imax * jmax * ((kmax + SCF_KSEG - 1) / SCF_KSEG), ngrp = (ncol + 63) / 64;
+    // per-segment summaries of the coefficient kernel
+    const int kseg = asm_kseg(imax, jmax, kmax);
+    const long long ncol = (long long)imax * jmax * ((kmax + kseg - 1) / kseg), ngrp = (ncol + 63) / 64;
     A(ctx->col_val, 12 * ncol); A(ctx->col_mask, ncol); A(ctx->grp_val, 12 * ngrp); A(ctx->grp_mask, ngrp);
     A(ctx->phase, ng);
     A(ctx->diag, ng); A(ctx->dinv, ng); A(ctx->cE, ng); A(ctx->cN, ng); A(ctx->cT, ng); A(ctx->extra, ng);

@@ -2,8 +2,19 @@
 #pragma once
 #include "scf_common.cuh"
 
-// Cells per thread segment of the column-marching assembly kernels.
-constexpr int SCF_KSEG = 32;
+// Cells per thread segment of the column-marching assembly kernels: the
+// longest of 32, 16, 8, 4 that still gives four blocks to each of the 152 SMs
+// (two waves of k_pocoef, one of k_operator).  A segment start forms every
+// coefficient anew (the memo is empty), a long segment is a serial chain of
+// loads: 40^3 1.49 ms per projection at 32 cells, 1.27 ms at 4; 147x93x121
+// 4.08 at 32, 4.02 at 8; from 256x128x128 up 32 is chosen and nothing changes.
+inline int asm_kseg(int I, int J, int K)
+{
+    const long long cols = (long long)((I + 31) / 32) * ((J + 3) / 4);
+    int kseg = 32;
+    while (kseg > 4 && cols * ((K + kseg - 1) / kseg) < 152 * 4) kseg /= 2;
+    return kseg;
+}
 
 // Inputs of the assembly (device mirrors of scf_poisson_in) plus scratch.
 struct AsmArgs {
@@ -28,6 +39,7 @@ struct AsmArgs {
     unsigned *flags;
     unsigned char *phase;   // ghosted, 1 wet / 2 dry / 0 neither
     double rdt;             // 1/dt
+    int kseg;               // cells per column segment (asm_kseg)
 };
 
 // Level-0 operator outputs (ghosted layout).
