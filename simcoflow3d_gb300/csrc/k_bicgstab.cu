@@ -9,9 +9,9 @@
 //   S: s = r - alpha v, formed at the 7 points; t = A s; t.s, t.t; omega
 //   X: s again, x += alpha p + omega s, r = s - omega t; r0.r, r.r; beta,
 //      and the stopping test
-// s is never stored.  Each thread marches KZ cells of one (i, j) column and
+// s is never stored.  Each thread marches d.kz cells of one (i, j) column and
 // keeps its share of the dot products in registers, so a block writes one
-// partial sum per dot for 128 x KZ cells; after each of P, S and X one
+// partial sum per dot for 128 x kz cells; after each of P, S and X one
 // block of 1024 threads sums the partials in a fixed order (so every run is
 // bitwise reproducible) and updates the scalars, which stay in device
 // memory.  (Summing them in the last block of the pass instead was slower:
@@ -25,7 +25,6 @@ namespace pred {
 namespace {
 
 constexpr int NT = 128;
-constexpr int KZ = 16;
 
 // Sum of up to 4 values over the block; thread 0 writes them to
 // partials[4 * block + q].  The products and the warp sums are formed in A
@@ -68,8 +67,8 @@ struct M6 {
 #define COLUMN                                                                \
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;                  \
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;                  \
-    const int k0 = blockIdx.z * KZ + 1;                                       \
-    const int k1 = min(k0 + KZ - 1, d.K);                                     \
+    const int k0 = blockIdx.z * d.kz + 1;                                     \
+    const int k1 = min(k0 + d.kz - 1, d.K);                                   \
     const bool in = i <= d.I && j <= d.J;                                     \
     const long long c0 = i + d.sy * j + d.sz * k0;
 
@@ -297,8 +296,16 @@ M6<T> m6(const T *const m[6])
 
 }  // namespace
 
+int march_len(int I, int J, int K, long long blocks)
+{
+    const long long cols = (long long)((I + 31) / 32) * ((J + 3) / 4);
+    int kz = 16;
+    while (kz > 1 && cols * ((K + kz - 1) / kz) < blocks) kz /= 2;
+    return kz;
+}
+
 dim3 solver_block() { return dim3(32, 4, 1); }
-dim3 solver_grid(const Dims &d) { return dim3((d.I + 31) / 32, (d.J + 3) / 4, (d.K + KZ - 1) / KZ); }
+dim3 solver_grid(const Dims &d) { return dim3((d.I + 31) / 32, (d.J + 3) / 4, (d.K + d.kz - 1) / d.kz); }
 
 template <typename T>
 void bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first, Reduce &R,

@@ -324,7 +324,11 @@ __global__ void k_pred_bc(double *pred, MomDev in, Dims d, int comp)
 void mom_assemble(const MomDev &in, const MomParams &o, int comp, const Dims &d, const MomSys &S, bool want32,
                   cudaStream_t st)
 {
-    const int kz = 16;
+    // two and a half waves of four blocks per SM; the row memo starts empty
+    // in each segment, but the march is a serial chain: 67x53x75 FP64 3.35 ms
+    // per call at 16 cells, 2.85 at 2; 128x112x96 mixed 4.76 at 16, 4.53 at 4,
+    // 4.73 at 2
+    const int kz = march_len(d.I, d.J, d.K, 152 * 10);
     const dim3 grid((d.I + 31) / 32, (d.J + 3) / 4, (d.K + kz - 1) / kz);
     k_mom_assemble<<<grid, dim3(32, 4, 1), 0, st>>>(in, o, comp, d, S, want32 ? 1 : 0, kz);
 }

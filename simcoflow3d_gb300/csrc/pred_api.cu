@@ -324,6 +324,10 @@ extern "C" int scf_mom_create(scf_mom_ctx **out, int32_t imax, int32_t jmax, int
     d.sy = imax + 2;
     d.sz = (long long)(imax + 2) * (jmax + 2);
     d.ng = d.sz * (kmax + 2);
+    // one wave of five blocks per SM: 67x53x75 FP64 3.36 ms per call at 16
+    // cells per segment, 3.04 at 4 and 3.50 at 1; 128x112x96 mixed 4.76 at 16,
+    // 4.64 at 8, 4.78 at 4; 16 from about 128^3 up
+    d.kz = march_len(imax, jmax, kmax, 152 * 5);
     auto fail = [&](int rc) {
         scf_mom_destroy(ctx);
         return rc;

@@ -43,6 +43,7 @@ struct MomSys {
 struct Dims {
     int I, J, K;          // interior sizes of the pressure grid
     long long sy, sz, ng; // ghosted strides and size
+    int kz;               // cells per column segment of the solver kernels
 };
 
 // Scalars of one BiCGStab run, in device memory.
@@ -94,7 +95,10 @@ void set_target(BcgScalars *sc, double target, cudaStream_t st);
 // Launch shape of the per-cell kernels (assembly checks).
 dim3 interior_block();
 dim3 interior_grid(const Dims &d);
-// Launch shape of the solver kernels (KZ-cell column segments); Reduce
+// Cells per column segment: the longest of 16, 8, .., 1 that gives at least
+// `blocks` blocks of 32 x 4 columns.
+int march_len(int I, int J, int K, long long blocks);
+// Launch shape of the solver kernels (d.kz-cell column segments); Reduce
 // holds one partial per dot per block of this grid.
 dim3 solver_block();
 dim3 solver_grid(const Dims &d);
