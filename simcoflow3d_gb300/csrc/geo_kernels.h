@@ -4,9 +4,6 @@
 #include <algorithm>
 #include "scf_common.cuh"
 
-// Cells per thread segment of the column-marching face kernel.
-constexpr int GEO_KSEG = 32;
-
 // One cell family on the device, in the host arrays' layouts (scf_geometry.h):
 // ghosted arrays of d.ng cells, interior arrays of d.n cells, ",3" arrays
 // with the component as the slowest index.

@@ -253,7 +253,7 @@ __device__ __forceinline__ Face face_resolve(FullMemo &mm, const FaceIn &in, Fac
 }
 
 // CellGeoCal's face loop and shared-face averaging (CutCell.f90:402-531).
-// A block is 32 x 4 columns; each thread marches a GEO_KSEG-cell segment of
+// A block is 32 x 4 columns; each thread marches a kseg-cell segment of
 // its (i,j) column.  For cell (i,j,k) it needs its six faces (WlLh takes
 // them all) and finishes the three faces it shares with its lower
 // neighbours: the W face with the E face of (i-1,j,k), the S face with the N
@@ -271,7 +271,7 @@ __device__ __forceinline__ Face face_resolve(FullMemo &mm, const FaceIn &in, Fac
 // one barrier only.
 constexpr int GEO_QCAP = 256;
 
-__global__ void __launch_bounds__(128) k_geo_faces(GeoFam t, Dims d, int *exact_count)
+__global__ void __launch_bounds__(128) k_geo_faces(GeoFam t, Dims d, int *exact_count, int kseg)
 {
     __shared__ FaceIn q_in[2][GEO_QCAP];
     __shared__ Face q_out[2][GEO_QCAP];
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(128) k_geo_faces(GeoFam t, Dims d, int *exact_
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const bool live = i <= d.I && j <= d.J;
-    const int kbeg = blockIdx.z * GEO_KSEG + 1, kend = min(kbeg + GEO_KSEG - 1, d.K);
+    const int kbeg = blockIdx.z * kseg + 1, kend = min(kbeg + kseg - 1, d.K);
     const long long NG = d.ng, NN = d.n;
     if (tid < 2) q_count[tid] = 0;
     __syncthreads();
@@ -645,15 +645,26 @@ __global__ void __launch_bounds__(256) k_geo_moex(GeoFam P, GeoFam U, GeoFam V, 
 // NumberExternalCell (CutCell.f90:753-786).  The numbering runs over
 // (i, j, k) with k fastest; an (i,j) column is a contiguous run of it.
 // Pass 1: active cells per column; pass 2 (one block): exclusive prefix over
-// the columns in (i, j) order; pass 3: each column numbers its cells.
+// the columns in (i, j) order; pass 3: each column numbers its cells.  One
+// thread walks a column, POSNU_U loads in flight at a time (one at a time, the
+// pass is the latency of nk dependent-looking loads: 47 us at 96^3).
+constexpr int POSNU_U = 8;
 __global__ void __launch_bounds__(256) k_posnu_count(GeoFam t, Dims d, int *colcount)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int ni = d.I - t.iu, nj = d.J - t.iv, nk = d.K - t.iw;
     if (i > ni || j > nj) return;
-    int c = 0;
-    for (int k = 1; k <= nk; ++k) c += t.ct[nidx(d, i, j, k)] != 2;
+    const int n0 = nidx(d, i, j, 1), s = d.I * d.J;
+    int c = 0, k = 0;
+    for (; k + POSNU_U <= nk; k += POSNU_U) {   // the group's loads are in flight together
+        int v[POSNU_U];
+#pragma unroll
+        for (int q = 0; q < POSNU_U; ++q) v[q] = t.ct[n0 + (k + q) * s];
+#pragma unroll
+        for (int q = 0; q < POSNU_U; ++q) c += v[q] != 2;
+    }
+    for (; k < nk; ++k) c += t.ct[n0 + k * s] != 2;
     colcount[(i - 1) * nj + (j - 1)] = c;
 }
 
@@ -689,10 +700,18 @@ __global__ void __launch_bounds__(256) k_posnu_write(GeoFam t, Dims d, const int
     const int ni = d.I - t.iu, nj = d.J - t.iv, nk = d.K - t.iw;
     if (i > ni || j > nj) return;
     int p = colstart[(i - 1) * nj + (j - 1)];
-    for (int k = 1; k <= nk; ++k) {
-        const long long q = (long long)(i - 1) + (long long)ni * ((j - 1) + (long long)nj * (k - 1));
-        t.posnu[q] = t.ct[nidx(d, i, j, k)] != 2 ? p++ : -1;
+    const int n0 = nidx(d, i, j, 1), s = d.I * d.J;
+    int *out = t.posnu + (i - 1) + (long long)ni * (j - 1);
+    const long long so = (long long)ni * nj;
+    int k = 0;
+    for (; k + POSNU_U <= nk; k += POSNU_U) {
+        int v[POSNU_U];
+#pragma unroll
+        for (int q = 0; q < POSNU_U; ++q) v[q] = t.ct[n0 + (k + q) * s];
+#pragma unroll
+        for (int q = 0; q < POSNU_U; ++q) out[(k + q) * so] = v[q] != 2 ? p++ : -1;
     }
+    for (; k < nk; ++k) out[k * so] = t.ct[n0 + k * s] != 2 ? p++ : -1;
 }
 
 }  // namespace
@@ -705,9 +724,16 @@ void launch_cell_geo(const GeoFam &t, const Dims &d, int *exact_count, cudaStrea
                      cudaEvent_t *ev)
 {
     k_geo_define<<<grid_for(d.ng, 256), 256, 0, st>>>(t, d);
-    dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + GEO_KSEG - 1) / GEO_KSEG);
+    // Cells per segment: the longest of 32, 16, .., 2 that gives two waves of
+    // the face kernel's three blocks per SM.  A segment start evaluates one
+    // face more, a long segment is a serial chain of loads and queue barriers:
+    // 96^3 (host call) 10.8 ms at 32 cells, 9.7 at 4, 9.8 at 2.
+    const long long cols = (long long)((d.I + 31) / 32) * ((d.J + 3) / 4);
+    int kseg = 32;
+    while (kseg > 2 && cols * ((d.K + kseg - 1) / kseg) < 152 * 6) kseg /= 2;
+    dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + kseg - 1) / kseg);
     if (ev) cudaEventRecord(ev[0], st);
-    k_geo_faces<<<g, b, 0, st>>>(t, d, exact_count);
+    k_geo_faces<<<g, b, 0, st>>>(t, d, exact_count, kseg);
     if (ev) cudaEventRecord(ev[1], st);
     *launches += 2;
     if (!t.moex) {
