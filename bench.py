@@ -956,7 +956,7 @@ def clsvof_workload(n: int):
 
 # algorithmic bytes per interior cell of one launch: the fields a kernel must
 # read and write once (neighbours come from cache)
-CLSVOF_BYTES = {"sweep_first": 40, "sweep_later": 56, "reconstruct": 40}
+CLSVOF_BYTES = {"sweep_first": 40, "sweep_later": 56, "normals": 54}
 
 
 def clsvof_cpu_ms(n_full: int, sample_n: int = 64):
@@ -1008,9 +1008,10 @@ def run_clsvof(args):
     cells = n ** 3
     kinds = ("reconstruct", "sweep", "walls", "redistance")
     kms = {k: sum(t["ms_kernels"][q] for t in timed) / len(timed) for q, k in enumerate(kinds)}
-    # per step: 18 sweeps (6 first, 12 later) and 24 reconstructions
+    # per step: 18 sweeps (6 first, 12 later) and 24 reconstructions, of which
+    # the 18 before the sweeps touch the partly filled cells only
     sweep_bytes = 6 * cells * (CLSVOF_BYTES["sweep_first"] + 2 * CLSVOF_BYTES["sweep_later"])
-    rec_bytes = 24 * cells * CLSVOF_BYTES["reconstruct"]
+    rec_bytes = 6 * cells * CLSVOF_BYTES["normals"]
     top = max(("sweep", "reconstruct"), key=lambda k: kms[k])
     tb = {"sweep": sweep_bytes, "reconstruct": rec_bytes}[top]
     launches = {"sweep": 18, "reconstruct": 24}[top]
@@ -1038,7 +1039,7 @@ def run_clsvof(args):
                 "h2d_bytes_per_step": int(e2e[-1]["bytes_h2d"]), "d2h_bytes_per_step": int(e2e[-1]["bytes_d2h"]),
                 "ms_h2d": round(statistics.mean(r["ms_h2d"] for r in e2e), 3),
                 "ms_d2h": round(statistics.mean(r["ms_d2h"] for r in e2e), 3)},
-        "roofline": {"bound": "hbm", "kernel": {"sweep": "k_sweep", "reconstruct": "k_reconstruct"}[top],
+        "roofline": {"bound": "hbm", "kernel": {"sweep": "k_sweep", "reconstruct": "k_normals"}[top],
                      "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
                      "peak_kind": peak_kind, "bytes_per_launch": tb // launches,
                      "ms_per_launch": round(kms[top] / launches, 5),

@@ -64,8 +64,9 @@ typedef struct scf_clsvof_stats {
     int32_t steps;                 /* time steps run by the last call            */
     int32_t gpu_launches;          /* kernels launched by the last run           */
     double ms_kernels[4];          /* with scf_clsvof_set_timing: the summed
-                                      times of k_reconstruct, k_sweep, k_walls
-                                      and the three redistancing kernels       */
+                                      times of the reconstruction kernels, the
+                                      sweeps, k_walls and the three
+                                      redistancing kernels                     */
 } scf_clsvof_stats;
 
 typedef struct scf_clsvof_ctx scf_clsvof_ctx;

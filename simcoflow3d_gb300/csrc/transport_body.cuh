@@ -21,8 +21,13 @@
 
 #if defined(__CUDACC__)
 #define TR_HD __host__ __device__ inline
+// Never inlined: FP64 work behind a branch that is rarely taken.  The compiler
+// turns a short inline branch into unconditional arithmetic and a select, and
+// FP64 operations are what bounds these kernels.
+#define TR_RARE __host__ __device__ __noinline__
 #else
 #define TR_HD inline
+#define TR_RARE inline
 #endif
 
 #if defined(TR_HOST_CHECK)
@@ -88,6 +93,25 @@ TR_HD double from_bits(uint64_t u)
     c.u = u;
     return c.d;
 }
+
+// Tests and sign changes on the 32-bit halves: the compiler turns their
+// 64-bit forms back into FP64 comparisons and negations.
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ uint32_t hi32(double v) { return (uint32_t)__double2hiint(v); }
+__device__ __forceinline__ uint32_t lo32(double v) { return (uint32_t)__double2loint(v); }
+__device__ __forceinline__ double from_halves(uint32_t hi, uint32_t lo) { return __hiloint2double((int)hi, (int)lo); }
+#else
+TR_HD uint32_t hi32(double v) { return (uint32_t)(bits_of(v) >> 32); }
+TR_HD uint32_t lo32(double v) { return (uint32_t)bits_of(v); }
+TR_HD double from_halves(uint32_t hi, uint32_t lo) { return from_bits(((uint64_t)hi << 32) | lo); }
+#endif
+TR_HD int exp_of(double v) { return (int)(hi32(v) >> 20) & 0x7ff; }
+TR_HD bool is_zero(double v) { return ((hi32(v) & 0x7fffffffu) | lo32(v)) == 0; }
+TR_HD bool is_plus_zero(double v) { return (hi32(v) | lo32(v)) == 0; }
+TR_HD bool is_one(double v) { return ((hi32(v) ^ 0x3ff00000u) | lo32(v)) == 0; }
+TR_HD bool is_finite(double v) { return exp_of(v) != 0x7ff; }
+TR_HD bool same_bits(double a, double b) { return ((hi32(a) ^ hi32(b)) | (lo32(a) ^ lo32(b))) == 0; }
+TR_HD double flip_if(double v, bool f) { return from_halves(hi32(v) ^ (f ? 0x80000000u : 0u), lo32(v)); }
 
 // x / d.  When d is a normal power of two its reciprocal is exact and
 // x * (1/d) is the same correctly rounded quotient, without an FP64
@@ -251,13 +275,42 @@ TR_HD bool is_interface(const Dims &D, const double *vfl, int i, int j, int k)
     return flag;
 }
 
-// |grad phi| - 1 of a difference triple, the test Normal_Vector_Irre uses.
-TR_HD double off_unit(double vx, double vy, double vz) { return fabs(1.0 - sqrt(vx * vx + vy * vy + vz * vz)); }
-
-TR_HD int side_of(double qm, double qp)
+// Normal_Vector_Irre's test | |grad phi| - 1 | < ETA on the sum of squares of a
+// difference triple, without the square root: the rounded |1 - sqrt(s)| is below
+// ETA exactly for OFF_LO <= s <= OFF_HI (sqrt and the subtraction are
+// monotonic, so two bisections give the interval's ends).
+constexpr double OFF_LO = 0x1.b6147ae147ae2p-1, OFF_HI = 0x1.27d70a3d70a3ep+0;
+TR_HD double norm2(double vx, double vy, double vz) { return vx * vx + vy * vy + vz * vz; }
+TR_HD int side_of(double sm, double sp)
 {
-    return (qm < ETA && qp >= ETA) ? -1 : (qm >= ETA && qp < ETA) ? 1 : 0;
+    const bool m_in = sm >= OFF_LO && sm <= OFF_HI, m_off = sm < OFF_LO || sm > OFF_HI;   // neither for NaN
+    const bool p_in = sp >= OFF_LO && sp <= OFF_HI, p_off = sp < OFF_LO || sp > OFF_HI;
+    return (m_in && p_off) ? -1 : (m_off && p_in) ? 1 : 0;
 }
+
+// Neighbours of a cell by constant strides from its own index.
+struct Around {
+    const Dims &D;
+    int i, j, k;
+    size_t g0, n0, gy, gz, ny, nz;
+    TR_HD Around(const Dims &D_, int i_, int j_, int k_)
+        : D(D_), i(i_), j(j_), k(k_), g0(D_.g(i_, j_, k_)), n0(D_.n(i_, j_, k_)), gy((size_t)(D_.I + 2)),
+          gz((size_t)(D_.I + 2) * (size_t)(D_.J + 2)), ny((size_t)D_.I), nz((size_t)D_.I * (size_t)D_.J)
+    {
+    }
+    TR_HD size_t g(int a, int b, int c) const   // ghosted, offsets a, b, c
+    {
+        const size_t t = g0 + (ptrdiff_t)a + (ptrdiff_t)b * (ptrdiff_t)gy + (ptrdiff_t)c * (ptrdiff_t)gz;
+        TR_CHECK(t == D.g(i + a, j + b, k + c), "ghosted neighbour");
+        return t;
+    }
+    TR_HD size_t n(int a, int b, int c) const   // interior
+    {
+        const size_t t = n0 + (ptrdiff_t)a + (ptrdiff_t)b * (ptrdiff_t)ny + (ptrdiff_t)c * (ptrdiff_t)nz;
+        TR_CHECK(t == D.n(i + a, j + b, k + c), "interior neighbour");
+        return t;
+    }
+};
 
 // Normal_Vector_Irre (2361-2456) for 1 < i < I, 1 < j < J, 1 < k < K: per
 // axis a one-sided difference towards the side whose neighbour's gradient
@@ -268,54 +321,54 @@ TR_HD int side_of(double qm, double qp)
 TR_HD void normal_irre(const Dims &D, const Geo &G, const double *phi, int i, int j, int k, double &nxx,
                        double &nyy, double &nzz)
 {
-    auto P = [&](int a, int b, int c) { return phi[D.g(a, b, c)]; };
-    auto X = [&](int a, int b, int c) { return G.x[D.n(a, b, c)]; };
-    auto Y = [&](int a, int b, int c) { return G.y[D.n(a, b, c)]; };
-    auto Z = [&](int a, int b, int c) { return G.z[D.n(a, b, c)]; };
+    const Around A(D, i, j, k);
+    auto P = [&](int a, int b, int c) { return phi[A.g(a, b, c)]; };
+    auto X = [&](int a, int b, int c) { return G.x[A.n(a, b, c)]; };
+    auto Y = [&](int a, int b, int c) { return G.y[A.n(a, b, c)]; };
+    auto Z = [&](int a, int b, int c) { return G.z[A.n(a, b, c)]; };
     auto Q = [](double num, double den) { return divd(num, den); };
-    double vx, vy, vz, qm, qp;
-    vx = i >= 3 ? Q(P(i, j, k) - P(i - 2, j, k), X(i, j, k) - X(i - 2, j, k))
-                : Q(P(i, j, k) - P(i - 1, j, k), X(i, j, k) - X(i - 1, j, k));
-    vy = Q(P(i - 1, j + 1, k) - P(i - 1, j - 1, k), Y(i - 1, j + 1, k) - Y(i - 1, j - 1, k));
-    vz = Q(P(i - 1, j, k + 1) - P(i - 1, j, k - 1), Z(i - 1, j, k + 1) - Z(i - 1, j, k - 1));
-    qm = off_unit(vx, vy, vz);
-    vx = i <= D.I - 2 ? Q(P(i + 2, j, k) - P(i, j, k), X(i + 2, j, k) - X(i, j, k))
-                      : Q(P(i + 1, j, k) - P(i, j, k), X(i + 1, j, k) - X(i, j, k));
-    vy = Q(P(i + 1, j + 1, k) - P(i + 1, j - 1, k), Y(i + 1, j + 1, k) - Y(i + 1, j - 1, k));
-    vz = Q(P(i + 1, j, k + 1) - P(i + 1, j, k - 1), Z(i + 1, j, k + 1) - Z(i + 1, j, k - 1));
-    qp = off_unit(vx, vy, vz);
-    const int sx = side_of(qm, qp);
-    vy = j >= 3 ? Q(P(i, j, k) - P(i, j - 2, k), Y(i, j, k) - Y(i, j - 2, k))
-                : Q(P(i, j, k) - P(i, j - 1, k), Y(i, j, k) - Y(i, j - 1, k));
-    vx = Q(P(i + 1, j - 1, k) - P(i - 1, j - 1, k), X(i + 1, j - 1, k) - X(i - 1, j - 1, k));
-    vz = Q(P(i, j - 1, k + 1) - P(i, j - 1, k - 1), Z(i, j - 1, k + 1) - Z(i, j - 1, k - 1));
-    qm = off_unit(vx, vy, vz);
-    vx = Q(P(i + 1, j + 1, k) - P(i - 1, j + 1, k), X(i + 1, j + 1, k) - X(i - 1, j + 1, k));
-    vy = j <= D.J - 2 ? Q(P(i, j + 2, k) - P(i, j, k), Y(i, j + 2, k) - Y(i, j, k))
-                      : Q(P(i, j + 1, k) - P(i, j, k), Y(i, j + 1, k) - Y(i, j, k));
-    vz = Q(P(i, j + 1, k + 1) - P(i, j + 1, k - 1), Z(i, j + 1, k + 1) - Z(i, j + 1, k - 1));
-    qp = off_unit(vx, vy, vz);
-    const int sy = side_of(qm, qp);
-    vx = Q(P(i + 1, j, k - 1) - P(i - 1, j, k - 1), X(i + 1, j, k - 1) - X(i - 1, j, k - 1));
-    vy = Q(P(i, j + 1, k - 1) - P(i, j - 1, k - 1), Y(i, j + 1, k - 1) - Y(i, j - 1, k - 1));
-    vz = k >= 3 ? Q(P(i, j, k) - P(i, j, k - 2), Z(i, j, k) - Z(i, j, k - 2))
-                : Q(P(i, j, k) - P(i, j, k - 1), Z(i, j, k) - Z(i, j, k - 1));
-    qm = off_unit(vx, vy, vz);
-    vx = Q(P(i + 1, j, k + 1) - P(i - 1, j, k + 1), X(i + 1, j, k + 1) - X(i - 1, j, k + 1));
-    vy = Q(P(i, j + 1, k + 1) - P(i, j - 1, k + 1), Y(i, j + 1, k + 1) - Y(i, j - 1, k + 1));
-    vz = k <= D.K - 2 ? Q(P(i, j, k + 2) - P(i, j, k), Z(i, j, k + 2) - Z(i, j, k))
-                      : Q(P(i, j, k + 1) - P(i, j, k), Z(i, j, k + 1) - Z(i, j, k));
-    qp = off_unit(vx, vy, vz);
-    const int sz = side_of(qm, qp);
-    nxx = sx == -1 ? Q(P(i, j, k) - P(i - 1, j, k), X(i, j, k) - X(i - 1, j, k))
-        : sx == 1  ? Q(P(i + 1, j, k) - P(i, j, k), X(i + 1, j, k) - X(i, j, k))
-                   : Q(P(i + 1, j, k) - P(i - 1, j, k), X(i + 1, j, k) - X(i - 1, j, k));
-    nyy = sy == -1 ? Q(P(i, j, k) - P(i, j - 1, k), Y(i, j, k) - Y(i, j - 1, k))
-        : sy == 1  ? Q(P(i, j + 1, k) - P(i, j, k), Y(i, j + 1, k) - Y(i, j, k))
-                   : Q(P(i, j + 1, k) - P(i, j - 1, k), Y(i, j + 1, k) - Y(i, j - 1, k));
-    nzz = sz == -1 ? Q(P(i, j, k) - P(i, j, k - 1), Z(i, j, k) - Z(i, j, k - 1))
-        : sz == 1  ? Q(P(i, j, k + 1) - P(i, j, k), Z(i, j, k + 1) - Z(i, j, k))
-                   : Q(P(i, j, k + 1) - P(i, j, k - 1), Z(i, j, k + 1) - Z(i, j, k - 1));
+    const double p0 = P(0, 0, 0), x0 = X(0, 0, 0), y0 = Y(0, 0, 0), z0 = Z(0, 0, 0);
+    double vx, vy, vz, sm, sp;
+    int o = i >= 3 ? -2 : -1;
+    vx = Q(p0 - P(o, 0, 0), x0 - X(o, 0, 0));
+    vy = Q(P(-1, 1, 0) - P(-1, -1, 0), Y(-1, 1, 0) - Y(-1, -1, 0));
+    vz = Q(P(-1, 0, 1) - P(-1, 0, -1), Z(-1, 0, 1) - Z(-1, 0, -1));
+    sm = norm2(vx, vy, vz);
+    o = i <= D.I - 2 ? 2 : 1;
+    vx = Q(P(o, 0, 0) - p0, X(o, 0, 0) - x0);
+    vy = Q(P(1, 1, 0) - P(1, -1, 0), Y(1, 1, 0) - Y(1, -1, 0));
+    vz = Q(P(1, 0, 1) - P(1, 0, -1), Z(1, 0, 1) - Z(1, 0, -1));
+    sp = norm2(vx, vy, vz);
+    const int sx = side_of(sm, sp);
+    o = j >= 3 ? -2 : -1;
+    vy = Q(p0 - P(0, o, 0), y0 - Y(0, o, 0));
+    vx = Q(P(1, -1, 0) - P(-1, -1, 0), X(1, -1, 0) - X(-1, -1, 0));
+    vz = Q(P(0, -1, 1) - P(0, -1, -1), Z(0, -1, 1) - Z(0, -1, -1));
+    sm = norm2(vx, vy, vz);
+    o = j <= D.J - 2 ? 2 : 1;
+    vx = Q(P(1, 1, 0) - P(-1, 1, 0), X(1, 1, 0) - X(-1, 1, 0));
+    vy = Q(P(0, o, 0) - p0, Y(0, o, 0) - y0);
+    vz = Q(P(0, 1, 1) - P(0, 1, -1), Z(0, 1, 1) - Z(0, 1, -1));
+    sp = norm2(vx, vy, vz);
+    const int sy = side_of(sm, sp);
+    vx = Q(P(1, 0, -1) - P(-1, 0, -1), X(1, 0, -1) - X(-1, 0, -1));
+    vy = Q(P(0, 1, -1) - P(0, -1, -1), Y(0, 1, -1) - Y(0, -1, -1));
+    o = k >= 3 ? -2 : -1;
+    vz = Q(p0 - P(0, 0, o), z0 - Z(0, 0, o));
+    sm = norm2(vx, vy, vz);
+    vx = Q(P(1, 0, 1) - P(-1, 0, 1), X(1, 0, 1) - X(-1, 0, 1));
+    vy = Q(P(0, 1, 1) - P(0, -1, 1), Y(0, 1, 1) - Y(0, -1, 1));
+    o = k <= D.K - 2 ? 2 : 1;
+    vz = Q(P(0, 0, o) - p0, Z(0, 0, o) - z0);
+    sp = norm2(vx, vy, vz);
+    const int sz = side_of(sm, sp);
+    // towards the minus side (-1, 0), the plus side (0, 1) or central (-1, 1)
+    int hi = sx == -1 ? 0 : 1, lo = sx == 1 ? 0 : -1;
+    nxx = Q(P(hi, 0, 0) - P(lo, 0, 0), X(hi, 0, 0) - X(lo, 0, 0));
+    hi = sy == -1 ? 0 : 1; lo = sy == 1 ? 0 : -1;
+    nyy = Q(P(0, hi, 0) - P(0, lo, 0), Y(0, hi, 0) - Y(0, lo, 0));
+    hi = sz == -1 ? 0 : 1; lo = sz == 1 ? 0 : -1;
+    nzz = Q(P(0, 0, hi) - P(0, 0, lo), Z(0, 0, hi) - Z(0, 0, lo));
 }
 
 // Interface_Reconstruct (1216-1309) of one cell: the unit normal and the
@@ -325,7 +378,9 @@ TR_HD void reconstruct(const Dims &D, const Geo &G, const double *vfl, const dou
                        double &n1, double &n2, double &n3, double &d1)
 {
     n1 = n2 = n3 = d1 = 0.0;
-    if (!is_interface(D, vfl, i, j, k)) return;
+    // a partly filled cell is an interface cell whatever its neighbours hold
+    const double v = vfl[D.g(i, j, k)];
+    if (!(v > VOFEPS && v < 1.0 - VOFEPS) && !is_interface(D, vfl, i, j, k)) return;
     if (i > 1 && i < D.I && j > 1 && j < D.J && k > 1 && k < D.K) {
         normal_irre(D, G, phi, i, j, k, n1, n2, n3);
     } else {
@@ -343,7 +398,7 @@ TR_HD void reconstruct(const Dims &D, const Geo &G, const double *vfl, const dou
         n1 = n1 / temp; n2 = n2 / temp; n3 = n3 / temp;
     }
     const size_t c = D.n(i, j, k);
-    d1 = find_distance(G.dx[c], G.dy[c], G.dz[c], n1, n2, n3, vfl[D.g(i, j, k)]);
+    d1 = find_distance(G.dx[c], G.dy[c], G.dz[c], n1, n2, n3, v);
 }
 
 // East/West/North/South/Top/Bottom_Flux (1553-1688): the liquid crossing
@@ -390,21 +445,53 @@ TR_HD size_t line_n(const Dims &D, int axis, int m, int a, int b)
     return axis == 0 ? D.n(m, a, b) : axis == 1 ? D.n(a, m, b) : D.n(a, b, m);
 }
 
-// The VOF flux through the face between cells q and q+1 of a line
-// (X_Sweep 835-860 and its y, z forms): a full or empty upstream cell
-// sends vfl*u*dt, a partial one its geometric cut.  z tests w >= 0 where x
-// and y test > 0.
+// Whether cell q is the upstream one of the face between cells q and q+1
+// of a line: z tests w >= 0 where x and y test > 0 (X_Sweep 835-860 and its
+// y, z forms).
+TR_HD bool face_down(int axis, double w) { return axis == 2 ? w >= 0.0 : w > 0.0; }
+
+// A partly filled cell, whose outflow is a geometric cut; a full or empty
+// upstream cell sends vfl*u*dt.
+TR_RARE bool partial_rare(double v) { return !(v >= 1.0 - VOFEPS || v <= VOFEPS); }
+TR_HD bool partial_cell(double v)
+{
+    if (is_plus_zero(v) || is_one(v)) return false;   // without FP64 compares
+    return partial_rare(v);
+}
+
+// The VOF flux through the face between cells q and q+1 of a line.
 TR_HD double vof_face(const Dims &D, const Geo &G, const SweepIn &S, int q, int a, int b)
 {
     const double w = S.vel[line_g(D, S.axis, q, a, b)];
-    const bool down = S.axis == 2 ? w >= 0.0 : w > 0.0;
+    const bool down = face_down(S.axis, w);
     const int up = down ? q : q + 1;
     const size_t gu = line_g(D, S.axis, up, a, b), nu = line_n(D, S.axis, up, a, b);
     const double v = S.vfl[gu];
-    if (v >= 1.0 - VOFEPS || v <= VOFEPS) return v * w * S.dtv;
+    if (!partial_cell(v)) return v * w * S.dtv;
     if (down) return face_flux(S.axis, +1, S.nx[gu], S.ny[gu], S.nz[gu], S.dis[gu], v, G.dx[nu], G.dy[nu], G.dz[nu],
                                w * S.dtv);
     return -face_flux(S.axis, -1, S.nx[gu], S.ny[gu], S.nz[gu], S.dis[gu], v, G.dx[nu], G.dy[nu], G.dz[nu], -w * S.dtv);
+}
+
+// The geometric fluxes a partial cell (i, j, k) with plane n.x = s sends
+// through its faces along the axis: fh where it is upstream of its high
+// face, fl where it is upstream of its low face (0 otherwise; nothing reads
+// those).
+TR_HD void partial_fluxes(const Dims &D, const Geo &G, const SweepIn &S, int i, int j, int k, double n1, double n2,
+                          double n3, double s, double &fl, double &fh)
+{
+    const int ax = S.axis, n = D.len(ax), m = ax == 0 ? i : ax == 1 ? j : k;
+    const size_t g = D.g(i, j, k), c = D.n(i, j, k);
+    const double v = S.vfl[g], dx = G.dx[c], dy = G.dy[c], dz = G.dz[c];
+    fl = fh = 0.0;
+    if (m <= n - 1) {
+        const double w = S.vel[g];
+        if (face_down(ax, w)) fh = face_flux(ax, +1, n1, n2, n3, s, v, dx, dy, dz, w * S.dtv);
+    }
+    if (m >= 2) {
+        const double w = S.vel[ax == 0 ? D.g(i - 1, j, k) : ax == 1 ? D.g(i, j - 1, k) : D.g(i, j, k - 1)];
+        if (!face_down(ax, w)) fl = -face_flux(ax, -1, n1, n2, n3, s, v, dx, dy, dz, -w * S.dtv);
+    }
 }
 
 // The level-set flux u*phi_face*dt through the face on the high side of
@@ -450,51 +537,50 @@ TR_HD double ls_face(const Dims &D, const Geo &G, const SweepIn &S, const double
     return w * ls * dtv;
 }
 
-// One cell of one sweep, gathered: the VOF and level set after the
-// sweep's face fluxes (added in the order the reference's face loops add
-// them to this cell), then the sub-step's divergence term -- the first
+// One cell of one sweep from the fluxes through its low and high faces (VOF
+// vl, vh; level set ll, lh), added in the order the reference's face loops
+// add them to this cell, then the sub-step's divergence term -- the first
 // sweep divides by 1 - dtv/d (u_m - u_{m-1}), the later two add dtv/d
 // times the first sweep's result times that difference -- and the clip of
-// the VOF to 0 and 1 within 1e-14 (Clsvof_Scheme 486-780).  Needs n >= 3.
-TR_HD void sweep_cell(const Dims &D, const Geo &G, const SweepIn &S, int i, int j, int k, double &vf_out,
-                      double &ls_out)
+// the VOF to 0 and 1 within 1e-14 (Clsvof_Scheme 486-780).  Needs n >= 3;
+// vl and ll are not read at m = 1, vh not at m = n.
+TR_HD void sweep_update(const Dims &D, const Geo &G, const SweepIn &S, int i, int j, int k, double vl, double vh,
+                        double ll, double lh, double &vf_out, double &ls_out)
 {
     const int ax = S.axis, n = D.len(ax);
     const int m = ax == 0 ? i : ax == 1 ? j : k;
     const int a = ax == 0 ? j : i, b = ax == 2 ? j : k;
     const double *d = ax == 0 ? G.dx : ax == 1 ? G.dy : G.dz;
-    const double *c = ax == 0 ? G.x : ax == 1 ? G.y : G.z;
     const size_t g = D.g(i, j, k), nc = D.n(i, j, k);
     const double dm = d[nc];
+    const size_t gm = ax == 0 ? D.g(i - 1, j, k) : ax == 1 ? D.g(i, j - 1, k) : D.g(i, j, k - 1);
+    const double ug = S.vel[g], um = S.vel[gm];
     // VOF (X_Sweep 835-875)
-    double tv = S.vfl[g];
-    if (m >= 2) tv = tv + divd(vof_face(D, G, S, m - 1, a, b), dm);
-    if (m <= n - 1) tv = tv - divd(vof_face(D, G, S, m, a, b), dm);
+    const double v0 = S.vfl[g];
+    double tv = v0;
+    if (m >= 2) tv = tv + divd(vl, dm);
+    if (m <= n - 1) tv = tv - divd(vh, dm);
     if (m == 1) {
-        const size_t gw = ax == 0 ? D.g(0, j, k) : ax == 1 ? D.g(i, 0, k) : D.g(i, j, 0);
-        const double flux = S.vfl[g] * S.vel[gw] * S.dtv;
+        const double flux = v0 * um * S.dtv;
         tv = tv + divd(flux, dm);
     }
     if (m == n) {
-        const double flux = S.vfl[g] * S.vel[g] * S.dtv;
+        const double flux = v0 * ug * S.dtv;
         tv = tv - divd(flux, dm);
     }
     // level set (X_Sweep 877-947)
     double tl = S.phi[g];
-    if (m >= 3) tl = tl + divd(ls_face(D, G, S, d, c, m - 1, a, b), dm);
-    if (m >= 2 && m <= n - 1) tl = tl - divd(ls_face(D, G, S, d, c, m, a, b), dm);
+    if (m >= 3) tl = tl + divd(ll, dm);
+    tl = tl - divd(lh, dm);
     if (m == 1) {
-        tl = tl - divd(ls_face(D, G, S, d, c, 1, a, b), dm);
         const size_t bw = (size_t)(a - 1) + (size_t)D.plane_lead(ax) * (size_t)(b - 1);
         TR_CHECK(bw < D.plane_size(ax), "wall plane");
         const double flux = S.bc_vel[bw] * S.bc_lvs[bw] * S.dtv;
         tl = tl + divd(flux, dm);
     }
-    if (m == 2) tl = tl + divd(ls_face(D, G, S, d, c, 1, a, b), dm);
-    if (m == n) tl = tl - divd(ls_face(D, G, S, d, c, n, a, b), dm);
+    if (m == 2) tl = tl + divd(ll, dm);
     // the divergence term and the clip
-    const size_t gm = ax == 0 ? D.g(i - 1, j, k) : ax == 1 ? D.g(i, j - 1, k) : D.g(i, j, k - 1);
-    const double du = S.vel[g] - S.vel[gm];
+    const double du = ug - um;
     const double rate = divd(S.dtv, dm);
     if (S.stage == 0) {
         const double den = 1.0 - rate * du;
@@ -508,6 +594,209 @@ TR_HD void sweep_cell(const Dims &D, const Geo &G, const SweepIn &S, int i, int 
     if (tv >= 1.0 - VOFEPS) tv = 1.0;
     vf_out = tv;
     ls_out = tl;
+}
+
+// One cell of one sweep, gathered: both faces computed from the fields.
+TR_HD void sweep_cell(const Dims &D, const Geo &G, const SweepIn &S, int i, int j, int k, double &vf_out,
+                      double &ls_out)
+{
+    const int ax = S.axis, n = D.len(ax);
+    const int m = ax == 0 ? i : ax == 1 ? j : k;
+    const int a = ax == 0 ? j : i, b = ax == 2 ? j : k;
+    const double *d = ax == 0 ? G.dx : ax == 1 ? G.dy : G.dz;
+    const double *c = ax == 0 ? G.x : ax == 1 ? G.y : G.z;
+    const double vl = m >= 2 ? vof_face(D, G, S, m - 1, a, b) : 0.0;
+    const double vh = m <= n - 1 ? vof_face(D, G, S, m, a, b) : 0.0;
+    const double ll = m >= 2 ? ls_face(D, G, S, d, c, m - 1, a, b) : 0.0;
+    const double lh = ls_face(D, G, S, d, c, m, a, b);
+    sweep_update(D, G, S, i, j, k, vl, vh, ll, lh, vf_out, ls_out);
+}
+
+// ---- the sweeps with shared work -------------------------------------------
+//
+// The same update as sweep_cell, bit for bit, with fewer FP64 operations (FP64
+// issues at 2 lanes per clock per SM on GB300 and bounds the sweeps): every
+// face once, quotients by a spacing through its reciprocal and kept while the
+// spacing's bits repeat along the line, nothing computed for empty cells, and
+// comparisons, halvings and sign tests on the integer pipe.
+
+
+// x / 2, by the exponent where that stays normal.
+TR_RARE double half_rare(double x) { return x / 2.0; }
+TR_HD double half_of(double x)
+{
+    const int e = exp_of(x);
+    if (e > 1 && e < 0x7ff) return from_halves(hi32(x) - 0x100000u, lo32(x));
+    return half_rare(x);
+}
+
+// A cell's spacing along the line with what is formed from it.
+struct LineStep {
+    double d, r, r2; // r = 1/d, rounded; for a power of two exact, and r2 = 1/(2d)
+    double half;     // d/2
+    double rate;     // dtv / d
+    bool pow2;
+};
+
+// x / d, correctly rounded, r = 1/d rounded: Markstein's division (IBM J. Res.
+// Dev. 34, 1990).  One remainder step makes the quotient faithful and a second
+// one, whose remainder is exact, rounds it correctly; five operations against
+// about nine.  Outside the exponents where the remainders are exact, and for
+// zeros, the division.
+TR_RARE double div_rare(double x, double d, double r)
+{
+    const int e = exp_of(x), ed = exp_of(d);
+    if (ed > 723 && ed < 1323 && e > 423 && e < 1623) {
+        double q = x * r;
+        q = fma(fma(-d, q, x), r, q);
+        return fma(fma(-d, q, x), r, q);
+    }
+    return x / d;
+}
+// x / (2d) is half of x / d while both stay normal.
+TR_RARE double div2_rare(double x, double d, double r)
+{
+    const double q = div_rare(x, d, r);
+    const int e = exp_of(q), ed = exp_of(d);
+    if (ed > 723 && ed < 1323 && e > 1 && e < 0x7ff) return half_of(q);
+    return divd(x, 2.0 * d);
+}
+TR_HD double line_div(const LineStep &s, double x) { return s.pow2 ? x * s.r : div_rare(x, s.d, s.r); }
+TR_HD double line_div2(const LineStep &s, double x) { return s.pow2 ? x * s.r2 : div2_rare(x, s.d, s.r); }
+
+TR_RARE double recip_rare(double d) { return 1.0 / d; }
+TR_HD LineStep line_step(double d, double dtv)
+{
+    LineStep s;
+    s.d = d;
+    const uint32_t h = hi32(d), e = (h >> 20) & 0x7ffu, sign = h & 0x80000000u;
+    s.pow2 = ((h & 0xfffffu) | lo32(d)) == 0 && e >= 2 && e <= 2044;
+    s.r2 = from_halves(sign | ((2045u - e) << 20), 0u);
+    if (s.pow2) s.r = from_halves(sign | ((2046u - e) << 20), 0u);
+    else s.r = recip_rare(d);
+    s.half = half_of(d);
+    s.rate = line_div(s, dtv);
+    return s;
+}
+
+// The face between cells q and q + 1 of a line: its VOF and level-set fluxes,
+// their quotients by cell q's spacing, and that spacing.
+struct LineFace {
+    double v, l, qv, ql, d;
+};
+
+// The VOF flux of a face whose upstream cell is neither empty nor full.
+TR_RARE double vof_flux_rare(double v, double w, double dtv, const double *cut)
+{
+    return partial_cell(v) ? *cut : v * w * dtv;
+}
+TR_RARE double ls_face_rare(const Dims &D, const Geo &G, const SweepIn &S, const double *d, const double *c, int q,
+                            int a, int b)
+{
+    return ls_face(D, G, S, d, c, q, a, b);
+}
+
+// s: cell q's spacing.  flo, fhi: the fluxes k_partial_fluxes left for the
+// partial cells.
+TR_HD LineFace line_face(const Dims &D, const Geo &G, const SweepIn &S, int ax, const LineStep &s, const double *d,
+                         const double *c, const double *flo, const double *fhi, int q, int a, int b)
+{
+    const int n = D.len(ax);
+    const size_t g = line_g(D, ax, q, a, b);
+    const size_t st = ax == 0 ? 1 : ax == 1 ? (size_t)(D.I + 2) : (size_t)(D.I + 2) * (size_t)(D.J + 2);
+    const double w = S.vel[g];
+    const uint32_t wa = hi32(w) & 0x7fffffffu;
+    const bool nan = wa > 0x7ff00000u || (wa == 0x7ff00000u && lo32(w) != 0);
+    const bool wneg = (hi32(w) >> 31) != 0, wzero = (wa | lo32(w)) == 0;
+    const bool up = (!wneg || wzero) && !nan, pos = !wneg && !wzero && !nan;   // w >= 0, w > 0
+    const double wd = w * S.dtv, step = line_div(s, wd);
+    LineFace f;
+    f.d = s.d;
+    f.v = f.qv = 0.0;
+    if (q < n) {
+        const bool down = ax == 2 ? up : pos;
+        const size_t gu = down ? g : g + st;
+        const double v = S.vfl[gu];
+        if (is_one(v)) {   // 1*u*dt
+            f.v = wd;
+            f.qv = step;
+        } else if (!is_plus_zero(v) || !is_finite(w)) {   // an empty cell sends a zero
+            f.v = vof_flux_rare(v, w, S.dtv, (down ? fhi : flo) + gu);
+            f.qv = line_div(s, f.v);
+        }
+    }
+    if (q == 1 || q == n || (q == n - 1 && !up)) {
+        f.l = ls_face_rare(D, G, S, d, c, q, a, b);
+    } else {
+        // PH(q) + half*(1 - step)*(PH(q+1) - PH(q-1))/(2 d) from below,
+        // PH(q+1) - half*(1 + step)*(PH(q+2) - PH(q))/(2 d) from above
+        const size_t g0 = up ? g : g + st;
+        const double t = 1.0 - flip_if(step, !up);
+        const double e = line_div2(s, s.half * t * (S.phi[g0 + st] - S.phi[g0 - st]));
+        const double ls = S.phi[g0] + flip_if(e, !up);
+        f.l = w * ls * S.dtv;
+    }
+    f.ql = line_div(s, f.l);
+    return f;
+}
+
+// The VOF of line_update for a cell with liquid in it or in its fluxes.
+TR_RARE double line_vof_rare(LineStep s, int m, int n, double v0, double qvl, double qvh, double um, double ug,
+                             double dtv, bool later, double first, double du, double den)
+{
+    double tv = v0;
+    if (m >= 2) tv = tv + qvl;
+    if (m <= n - 1) tv = tv - qvh;
+    if (m == 1) tv = tv + line_div(s, v0 * um * dtv);
+    if (m == n) tv = tv - line_div(s, v0 * ug * dtv);
+    if (!later) tv = divd(tv, den);
+    else tv = tv + s.rate * first * du;
+    if (tv <= VOFEPS) tv = 0.0;
+    if (tv >= 1.0 - VOFEPS) tv = 1.0;
+    return tv;
+}
+TR_RARE double wall_flux_rare(LineStep s, double u, double ls, double dtv) { return line_div(s, u * ls * dtv); }
+
+// sweep_update from the faces lo (not read at m = 1) and hi; s: this cell's
+// spacing; LATER: the second or third sweep of the sub-step.  An empty cell
+// without VOF fluxes stays empty: its sum is a zero, which the clip makes +0.
+template <bool LATER>
+TR_HD void line_update(const Dims &D, const SweepIn &S, int ax, const LineStep &s, const LineFace &lo,
+                       const LineFace &hi, int m, int a, int b, double &vf_out, double &ls_out)
+{
+    const int n = D.len(ax);
+    const size_t g = line_g(D, ax, m, a, b);
+    const size_t st = ax == 0 ? 1 : ax == 1 ? (size_t)(D.I + 2) : (size_t)(D.I + 2) * (size_t)(D.J + 2);
+    const double ug = S.vel[g], um = S.vel[g - st], v0 = S.vfl[g];
+    const bool same = same_bits(lo.d, s.d);
+    const double du = ug - um;
+    const double den = LATER ? 1.0 : 1.0 - s.rate * du;
+    const double first = LATER ? S.vf_first[g] : 0.0;
+    // finite rate and du (or den neither zero nor infinite): zeros stay zeros
+    const bool tame = LATER ? is_finite(du) && is_finite(s.rate) : exp_of(den) != 0 && is_finite(den);
+    if (is_zero(v0) && is_zero(first) && is_zero(hi.qv) && (m < 2 || is_zero(lo.v)) && tame && is_finite(ug) &&
+        is_finite(um)) {
+        vf_out = 0.0;
+    } else {
+        const double qvl = m < 2 ? 0.0 : same ? lo.qv : line_div(s, lo.v);
+        vf_out = line_vof_rare(s, m, n, v0, qvl, hi.qv, um, ug, S.dtv, LATER, first, du, den);
+    }
+    // + low face - high face, in the order - high + low at m = 2; at the low
+    // wall - high + the wall's flux
+    double q1, q2;
+    if (m >= 2) {
+        const double qll = same ? lo.ql : line_div(s, lo.l), qlh = flip_if(hi.ql, true);
+        q1 = m >= 3 ? qll : qlh;
+        q2 = m >= 3 ? qlh : qll;
+    } else {
+        const size_t bw = (size_t)(a - 1) + (size_t)D.plane_lead(ax) * (size_t)(b - 1);
+        TR_CHECK(bw < D.plane_size(ax), "wall plane");
+        q1 = flip_if(hi.ql, true);
+        q2 = wall_flux_rare(s, S.bc_vel[bw], S.bc_lvs[bw], S.dtv);
+    }
+    const double tl = S.phi[g] + q1 + q2;
+    if (LATER) ls_out = tl + s.rate * S.ls_first[g] * du;
+    else ls_out = divd(tl, den);
 }
 
 // ---- redistancing (Redistance_Levelset 1689-1889) ----------------------
@@ -577,6 +866,28 @@ TR_HD void shortest_point_2d(double nx1, double ny1, double nz1, double dis1, in
     else { xs = us; ys = vs; }
 }
 
+// The third case with several axes of equal weight: the reference goes through
+// them all, each writing into the same point.
+TR_RARE double band_ties_rare(double nxx, double nyy, double nzz, double diss, int ii, int jj, int kk, double dx,
+                              double dy, double dz, double xp, double yp, double zp, double ax, double ay, double az)
+{
+    const double X = dx * (double)ii, Y = dy * (double)jj, Z = dz * (double)kk;
+    const double fc[3] = {sgn(xp) * 0.5 * dx, sgn(yp) * 0.5 * dy, sgn(zp) * 0.5 * dz};
+    const double nn[3] = {nxx, nyy, nzz};
+    double s[3] = {0.0, 0.0, 0.0};
+    const double w[3] = {ax, ay, az};
+    for (int c = 0; c < 3; ++c) {
+        const int o1 = c == 0 ? 1 : 0, o2 = c == 2 ? 1 : 2;
+        if (!(w[c] >= w[o1] && w[c] >= w[o2])) continue;
+        int cas;
+        if (cut_face(fc[c], nxx, nyy, nzz, diss, dx, dy, dz, c + 1)) cas = c;
+        else cas = w[o1] > w[o2] ? o1 : o2;
+        s[cas] = fc[cas];
+        shortest_point_2d(nxx, nyy, nzz, nn[cas] * s[cas] + diss, ii, jj, kk, cas + 1, dx, dy, dz, s[0], s[1], s[2]);
+    }
+    return sqrt((X - s[0]) * (X - s[0]) + (Y - s[1]) * (Y - s[1]) + (Z - s[2]) * (Z - s[2]));
+}
+
 // The distance Redistance_Levelset measures from the centre (ii, jj, kk)
 // cells away to an interface cell's plane n.x + diss = 0 (diss from the
 // cell centre; the interface cell's spacings): the facing boundary point
@@ -600,21 +911,217 @@ TR_HD double band_distance(double nxx, double nyy, double nzz, double diss, int 
     const double ax = fmax(fabs(xp) - 0.5 * dx, 0.0) * fabs(nxx);
     const double ay = fmax(fabs(yp) - 0.5 * dy, 0.0) * fabs(nyy);
     const double az = fmax(fabs(zp) - 0.5 * dz, 0.0) * fabs(nzz);
-    const double fc[3] = {sgn(xp) * 0.5 * dx, sgn(yp) * 0.5 * dy, sgn(zp) * 0.5 * dz};
-    const double nn[3] = {nxx, nyy, nzz};
-    double s[3] = {0.0, 0.0, 0.0};
-    const double w[3] = {ax, ay, az};
-    for (int c = 0; c < 3; ++c) {
-        const int o1 = c == 0 ? 1 : 0, o2 = c == 2 ? 1 : 2;
-        if (!(w[c] >= w[o1] && w[c] >= w[o2])) continue;
-        int cas;
-        if (cut_face(fc[c], nxx, nyy, nzz, diss, dx, dy, dz, c + 1)) cas = c;
-        else cas = w[o1] > w[o2] ? o1 : o2;
-        s[cas] = fc[cas];
-        shortest_point_2d(nxx, nyy, nzz, nn[cas] * s[cas] + diss, ii, jj, kk, cas + 1, dx, dy, dz, s[0], s[1], s[2]);
-    }
-    return sqrt((X - s[0]) * (X - s[0]) + (Y - s[1]) * (Y - s[1]) + (Z - s[2]) * (Z - s[2]));
+    // One axis outweighs the others (almost always): its face, one copy of the
+    // work for all three axes, so that a warp's lanes stay together.
+    const int c = ay > ax ? (az > ay ? 2 : 1) : (az > ax ? 2 : 0);
+    const double wc = c == 0 ? ax : c == 1 ? ay : az;
+    const double w1 = c == 0 ? ay : ax, w2 = c == 2 ? ay : az;
+    if (!(wc > w1 && wc > w2))
+        return band_ties_rare(nxx, nyy, nzz, diss, ii, jj, kk, dx, dy, dz, xp, yp, zp, ax, ay, az);
+    const double nc = c == 0 ? nxx : c == 1 ? nyy : nzz;
+    const double f = sgn(c == 0 ? xp : c == 1 ? yp : zp) * 0.5 * (c == 0 ? dx : c == 1 ? dy : dz);
+    // cut_face: the corner sums in the order x, y, z (the face's own term is the
+    // first or second addend on the x and y faces, the third on the z face)
+    const double ha = 0.5 * (c == 0 ? dy : dx) * (c == 0 ? nyy : nxx), hb = 0.5 * (c == 2 ? dy : dz) * (c == 2 ? nyy : nzz);
+    const double fn = f * nc;
+    const bool zc = c == 2;
+    const double p1 = (zc ? -ha - hb : fn - ha) + (zc ? fn : -hb) + diss;
+    const double p2 = (zc ? -ha + hb : fn - ha) + (zc ? fn : hb) + diss;
+    const double p3 = (zc ? ha + hb : fn + ha) + (zc ? fn : hb) + diss;
+    const double p4 = (zc ? ha - hb : fn + ha) + (zc ? fn : -hb) + diss;
+    int cas = c;
+    if (p1 * p2 >= 0.0 && p2 * p3 >= 0.0 && p3 * p4 >= 0.0 && p4 * p1 >= 0.0)
+        cas = w1 > w2 ? (c == 0 ? 1 : 0) : (c == 2 ? 1 : 2);
+    const double fs = cas == c ? f : sgn(cas == 0 ? xp : cas == 1 ? yp : zp) * 0.5 * (cas == 0 ? dx : cas == 1 ? dy : dz);
+    double s0 = fs, s1 = fs, s2 = fs;   // the face's coordinate; the other two are set
+    const double ns = cas == 0 ? nxx : cas == 1 ? nyy : nzz;
+    shortest_point_2d(nxx, nyy, nzz, ns * fs + diss, ii, jj, kk, cas + 1, dx, dy, dz, s0, s1, s2);
+    return sqrt((X - s0) * (X - s0) + (Y - s1) * (Y - s1) + (Z - s2) * (Z - s2));
 }
+
+// ---- FP32 bounds of a band distance ----------------------------------------
+//
+// Only the least distance of each target counts, so a pair whose FP32 lower
+// bound exceeds the target's least FP32 upper bound needs no FP64 work.  The
+// bounds come from band_distance's steps in FP32 on lengths scaled by the
+// cell's largest spacing, with every comparison required to hold by more than
+// the error of its two sides; a pair that comes too close to any of them has
+// no bounds and is computed.  Errors (in units of the scale, u = 2^-24): the
+// inputs carry a few u each, |X| <= 4 per axis, |dis| <= 2 and |n| <= 1 give
+// at most 8e-6 for dv, dij1 and the foot point; BE1 doubles that.
+
+struct BandSource {
+    float n[3], dis, d[3], h;
+    bool ok;   // inside the range the error bounds hold for
+};
+// What Iscutface and Shortest_Point_2d form of one face of the cell (index
+// 2 * axis + (1 on the high side)), whatever the target: u, v are its in-plane
+// axes.  inv_v = -1/nv and inv_u = 1/(-nu) -- on a y face over |nz| -- or 0
+// where the quotient is too steep to bound.
+struct BandFace {
+    float nu, nv, ds, e4, e5, inv_u, inv_v;
+    int cut;   // 1: the plane crosses the face, 0: it does not, -1: FP32 cannot tell
+};
+
+constexpr float BE1 = 1.6e-5f;
+
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ float band_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float band_sqrt(float a)   // within 2^-23 relative
+{
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return r;
+}
+#else
+TR_HD float band_fma(float a, float b, float c) { return a * b + c; }
+TR_HD float band_sqrt(float a) { return sqrtf(a); }
+#endif
+
+// v[q] by selects: the arrays stay in registers.
+template <typename T>
+TR_HD T pick(const T (&v)[3], int q) { return q == 0 ? v[0] : q == 1 ? v[1] : v[2]; }
+
+// From the FP32 values of an interface cell's normal, centre distance and
+// spacings.
+TR_HD BandSource band_source(float n1, float n2, float n3, float dis, float dx, float dy, float dz)
+{
+    BandSource s;
+    s.n[0] = n1; s.n[1] = n2; s.n[2] = n3;
+    const float m = dx > dy ? dx : dy;
+    s.h = m > dz ? m : dz;
+    s.d[0] = dx / s.h; s.d[1] = dy / s.h; s.d[2] = dz / s.h;
+    s.dis = dis / s.h;
+    s.ok = s.h > 1e-15f && s.h < 1e15f && s.d[0] > 1e-3f && s.d[1] > 1e-3f && s.d[2] > 1e-3f &&
+           fabsf(s.dis) <= 2.0f && n1 * n1 + n2 * n2 + n3 * n3 <= 1.001f;
+    return s;
+}
+
+TR_HD BandFace band_face(const BandSource &B, int face)
+{
+    const int c = face >> 1, u = c == 0 ? 1 : 0, v = c == 2 ? 1 : 2;
+    const float n = pick(B.n, c), pu = pick(B.n, u), pv = pick(B.n, v);
+    const float base = (face & 1 ? 0.5f : -0.5f) * pick(B.d, c) * n + B.dis;
+    BandFace f;
+    const float h1 = 0.5f * pick(B.d, u) * pu, h2 = 0.5f * pick(B.d, v) * pv;
+    const float p1 = base - h1 - h2, p2 = base - h1 + h2, p3 = base + h1 + h2, p4 = base + h1 - h2;
+    f.cut = (p1 > 0.f) == (p2 > 0.f) && (p2 > 0.f) == (p3 > 0.f) && (p3 > 0.f) == (p4 > 0.f) ? 0 : 1;
+    if (!(fabsf(p1) > BE1 && fabsf(p2) > BE1 && fabsf(p3) > BE1 && fabsf(p4) > BE1)) f.cut = -1;
+    const float t = sqrtf(pu * pu + pv * pv);
+    f.nu = f.nv = f.ds = f.e5 = f.inv_u = f.inv_v = 0.f;
+    f.e4 = 1e30f;   // no bounds: every comparison comes too close
+    if (t > 0.02f) {
+        const float r = 1.0f / t;
+        f.nu = pu * r;
+        f.nv = pv * r;
+        f.ds = base * r;
+        f.e4 = 2.4e-5f + 1.0e-5f * r;
+        f.e5 = 6.0e-6f * r + 6.0e-6f;
+        if (fabsf(f.nv) > 0.02f) f.inv_v = -1.0f / f.nv;
+        const float div = c == 1 ? fabsf(f.nv) : fabsf(f.nu);
+        if (div > 0.02f && fabsf(f.nu) > 1.0e-5f) f.inv_u = 1.0f / copysignf(div, -f.nu);
+    }
+    return f;
+}
+
+// v is certainly inside [-half, half], certainly outside, or neither (0).
+TR_HD int band_side(float v, float half, float e) { return fabsf(v) < half - e ? 1 : fabsf(v) > half + e ? -1 : 0; }
+
+// Bounds of band_distance for the offset (ii, jj, kk) and the sign of the
+// level set there; false when FP32 cannot decide.  F: the cell's six faces.
+TR_HD bool band_bounds(const BandSource &B, const BandFace *F, int ii, int jj, int kk, bool neg, float &lo, float &hi)
+{
+    if (!B.ok) return false;
+    const int o[3] = {ii, jj, kk};
+    float X[3], t[3], dv = B.dis, dij = B.dis;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int l = o[q] < -1 ? -1 : o[q] > 1 ? 1 : o[q];
+        X[q] = B.d[q] * (float)o[q];
+        t[q] = B.d[q] * (0.5f * (float)l);   // the facing boundary point
+        dv = band_fma(B.n[q], t[q], dv);
+        dij = band_fma(B.n[q], X[q], dij);
+    }
+    const float sdv = neg ? -dv : dv;
+    if (!(fabsf(sdv) > BE1)) return false;
+    float a0, a1, a2, err;   // target minus the nearest point
+    if (sdv < 0.f) {
+        a0 = X[0] - t[0]; a1 = X[1] - t[1]; a2 = X[2] - t[2];
+        err = BE1;
+    } else {
+        float xp[3], w[3];
+        int in[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            xp[q] = band_fma(-dij, B.n[q], X[q]);
+            in[q] = band_side(xp[q], 0.5f * B.d[q], BE1);
+            // a coordinate inside weighs exactly 0
+            w[q] = in[q] > 0 ? 0.f : (fabsf(xp[q]) - 0.5f * B.d[q]) * fabsf(B.n[q]);
+        }
+        if (in[0] == 0 || in[1] == 0 || in[2] == 0) return false;
+        if (in[0] > 0 && in[1] > 0 && in[2] > 0) {
+            a0 = X[0] - xp[0]; a1 = X[1] - xp[1]; a2 = X[2] - xp[2];
+            err = 2.0f * BE1;
+        } else {
+            // the face the foot point leaves through: the largest weight, which
+            // must be so beyond doubt
+            int c = w[1] > w[0] ? 1 : 0;
+            if (w[2] > pick(w, c)) c = 2;
+            const int o1 = c == 0 ? 1 : 0, o2 = c == 2 ? 1 : 2;
+            const float wc = pick(w, c) - 2.0f * BE1, w1 = pick(w, o1), w2 = pick(w, o2);
+            if (!(wc > w1) || !(wc > w2)) return false;
+            int face = 2 * c + (pick(xp, c) > 0.f ? 1 : 0);
+            const int cut = F[face].cut;
+            if (cut < 0) return false;
+            if (cut == 0) {   // the other axis that weighs more, the second if neither does
+                if (!(w1 == 0.f && w2 == 0.f) && !(fabsf(w1 - w2) > 2.0f * BE1)) return false;
+                const int cas = w1 > w2 ? o1 : o2;
+                const float x = pick(xp, cas);
+                if (!(fabsf(x) > BE1)) return false;
+                face = 2 * cas + (x > 0.f ? 1 : 0);
+            }
+            // Shortest_Point_2d on that face
+            const BandFace f = F[face];
+            const int cas = face >> 1, u = cas == 0 ? 1 : 0, v = cas == 2 ? 1 : 2;
+            const float Xu = pick(X, u), Xv = pick(X, v);
+            const float dj = band_fma(f.nu, Xu, band_fma(f.nv, Xv, f.ds));
+            const float up = band_fma(-dj, f.nu, Xu), vp = band_fma(-dj, f.nv, Xv);
+            const float hu = 0.5f * pick(B.d, u), hv = 0.5f * pick(B.d, v);
+            const int iu = band_side(up, hu, f.e4), iv = band_side(vp, hv, f.e4);
+            if (iu == 0 || iv == 0) return false;
+            float us = up, vs = vp;
+            err = 2.0f * f.e4 + BE1;
+            if (iu < 0 || iv < 0) {
+                const float wu = iu > 0 ? 0.f : (fabsf(up) - hu) * fabsf(f.nu);
+                const float wv = iv > 0 ? 0.f : (fabsf(vp) - hv) * fabsf(f.nv);
+                if (!(fabsf(wu - wv) > 2.0f * f.e4)) return false;
+                float inv, s;
+                if (wu > wv) {
+                    us = copysignf(hu, up);
+                    inv = f.inv_v;
+                    s = vs = band_fma(f.nu, us, f.ds) * inv;
+                } else {
+                    vs = copysignf(hv, vp);
+                    inv = f.inv_u;
+                    s = us = band_fma(f.nv, vs, f.ds) * inv;
+                }
+                if (inv == 0.f) return false;
+                err = f.e5 * fabsf(inv) + 2.0e-6f * fabsf(s) + f.e4 + BE1;
+            }
+            a0 = pick(X, cas) - (face & 1 ? 0.5f : -0.5f) * pick(B.d, cas);
+            a1 = Xu - us;
+            a2 = Xv - vs;
+        }
+    }
+    const float dist = band_sqrt(band_fma(a0, a0, band_fma(a1, a1, a2 * a2)));
+    err = band_fma(2.0e-6f, dist, err);
+    lo = (dist - err) * B.h;
+    hi = (dist + err) * B.h;
+    return true;
+}
+
+// An upper bound of every cell's initial key (1e4).
+constexpr float BAND_UB = 1.001e4f;
 
 TR_HD bool band_interface(double v) { return 0.0 + 1.0e-15 < v && v < 1.0 - 1.0e-15; }
 TR_HD bool band_target(double v) { return v < 0.0 + 1.0e-15 || v > 1.0 - 1.0e-15; }
@@ -683,15 +1190,24 @@ TR_HD void band_scatter(const Dims &D, const Geo &G, const double *vfl, const do
     for (int t = 0; t < BAND_CELLS; ++t) band_pair(D, G, vfl, phi, nx, ny, nz, dis, i, j, k, t, key, fix);
 }
 
+TR_RARE double band_value_rare(double v, double dx, const double *dis, bool fixed, unsigned long long key)
+{
+    if (band_interface(v)) return sgn(0.5 - v) * fabs(*dis);
+    if (fixed) return sgn(0.5 - v) * value_of(key);
+    return (double)(BAND + 1) * dx * sqrt(3.0) * sgn(0.5 - v);
+}
+
 // The level set each cell ends with (1866-1882).
 TR_HD double band_value(const Dims &D, const Geo &G, const double *vfl, const double *dis, int i, int j, int k,
                         const unsigned long long *key, const uint8_t *fix)
 {
     const size_t g = D.g(i, j, k), c = D.n(i, j, k);
     const double v = vfl[g];
-    if (band_interface(v)) return sgn(0.5 - v) * fabs(dis[g]);
-    if (fix[c]) return sgn(0.5 - v) * value_of(key[c]);
-    return (double)(BAND + 1) * G.dx[c] * sqrt(3.0) * sgn(0.5 - v);
+    if (is_plus_zero(v) || is_one(v)) {   // empty or full: only the sign depends on v
+        const double m = fix[c] ? value_of(key[c]) : (double)(BAND + 1) * G.dx[c] * sqrt(3.0);
+        return flip_if(m, hi32(v) != 0);
+    }
+    return band_value_rare(v, G.dx[c], dis + g, fix[c] != 0, key[c]);
 }
 
 // ---- boundary planes (BoundaryConditionLvsVof 2087-2221) -----------------
