@@ -24,6 +24,7 @@ UNITS = {
     "k_assemble.cu": ["-fmad=false"],
     "k_correct.cu": ["-fmad=false"],
     "k_solver.cu": [],
+    "k_coarse.cu": [],
     "scf_api.cu": [],
     "k_noalloc.cu": [],
     "k_adjoint.cu": [],

@@ -12,8 +12,10 @@
 // in a fixed order, so results are bitwise reproducible.
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
+#include "scf_cheb.cuh"
 #include "scf_kernels.h"
 #include "scf_tma.cuh"
 
@@ -23,36 +25,6 @@
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1; \
     const bool in = i <= (L).n0 && j <= (L).n1 && k <= (L).n2; \
     const int c = i + (L).sy * j + (L).sz * k;
-
-// ---------------------------------------------------------------------------
-// Jacobi scaling.  FP32 levels compute 1/diag on the fly with the hardware
-// reciprocal (one instruction, and it saves one array per pass); FP64 levels
-// read a stored inverse (FP64 division is slow on this GPU).  Inactive cells carry diag = -1 and
-// get no update and no coarse correction.
-template <typename T>
-__device__ __forceinline__ T dinv_at(const LevelView<T> &L, int c);
-template <>
-__device__ __forceinline__ float dinv_at<float>(const LevelView<float> &L, int c)
-{
-    return jacobi_inv(L.diag[c]);
-}
-template <>
-__device__ __forceinline__ double dinv_at<double>(const LevelView<double> &L, int c)
-{
-    return L.dinv[c];
-}
-template <typename T>
-__device__ __forceinline__ bool active_at(const LevelView<T> &L, int c);
-template <>
-__device__ __forceinline__ bool active_at<float>(const LevelView<float> &L, int c)
-{
-    return L.diag[c] > 0.0f;
-}
-template <>
-__device__ __forceinline__ bool active_at<double>(const LevelView<double> &L, int c)
-{
-    return __double_as_longlong(L.dinv[c]) != 0;
-}
 
 // ---------------------------------------------------------------------------
 // reductions
@@ -449,43 +421,6 @@ __global__ void __launch_bounds__(256) k_cheb_first(LevelView<T> L, const T *__r
 {
     INTERIOR_IJK(L);
     if (in) x[c] = coef * dinv_at(L, c) * b[c];
-}
-
-// Arithmetic of one Chebyshev update with every operation spelled out (no
-// contraction left to the compiler), so that the one-step kernel and the
-// fused two-step kernel give the same bits: the six neighbour products
-// summed by FMA in the order E, W, N, S, T, B; A x = diag x - s;
-// r = b - A x; the update dn = (c2 dinv) r + c1 dprev.
-__device__ __forceinline__ float fx_mul(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double fx_mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float fx_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fx_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float fx_sub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double fx_sub(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ float fx_add(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double fx_add(double a, double b) { return __dadd_rn(a, b); }
-
-// r = b - A x of one cell, the residual both the Chebyshev update and the
-// restriction use, so a fused residual gives the bits of a separate one.
-template <typename T>
-__device__ __forceinline__ T cheb_residual(T b, T dg, T x0, T xe, T xw, T xn, T xs, T xt, T xb, T ce, T cw, T cn,
-                                           T cs, T ct, T cb)
-{
-    T s = fx_mul(ce, xe);
-    s = fx_fma(cw, xw, s);
-    s = fx_fma(cn, xn, s);
-    s = fx_fma(cs, xs, s);
-    s = fx_fma(ct, xt, s);
-    s = fx_fma(cb, xb, s);
-    return fx_sub(b, fx_fma(dg, x0, -s));
-}
-
-template <typename T>
-__device__ __forceinline__ T cheb_update(T b, T dg, T dinv, T x0, T xe, T xw, T xn, T xs, T xt, T xb, T ce, T cw,
-                                         T cn, T cs, T ct, T cb, T dprev, T c1, T c2)
-{
-    const T r = cheb_residual(b, dg, x0, xe, xw, xn, xs, xt, xb, ce, cw, cn, cs, ct, cb);
-    return fx_fma(fx_mul(c2, dinv), r, fx_mul(c1, dprev));
 }
 
 template <typename T>
@@ -1028,13 +963,6 @@ bool cheb_restrict(const MgLevel<float> &F, const MgLevel<float> &C, const float
 // zero_guess: x = 0 on entry (the first pre-smoothing step); x and dprev are
 // not read.  T is a diagonally dominant M-matrix block, so its eigenvalue
 // bound for the Chebyshev interval is that of the point diagonal.
-template <typename T>
-__device__ __forceinline__ T rcp_of(T v);
-template <>
-__device__ __forceinline__ float rcp_of<float>(float v) { return __frcp_rn(v); }
-template <>
-__device__ __forceinline__ double rcp_of<double>(double v) { return 1.0 / v; }
-
 // Every operation is spelled out (as in cheb_update), so that the two halves
 // can be ordered for latency without changing a bit: first all of the
 // segment's loads and residuals, which do not depend on one another, then the
@@ -1190,11 +1118,11 @@ __global__ void __launch_bounds__(256) k_post_first(LevelView<T> F, const T *__r
         return v;
     };
     const T x0 = xc(i, j, k);
-    const T ax = F.diag[c] * x0 - (F.cE[c] * xc(i + 1, j, k) + F.cE[c - 1] * xc(i - 1, j, k) +
-                                   F.cN[c] * xc(i, j + 1, k) + F.cN[c - F.sy] * xc(i, j - 1, k) +
-                                   F.cT[c] * xc(i, j, k + 1) + F.cT[c - F.sz] * xc(i, j, k - 1));
-    const T dn = coef * dinv_at(F, c) * (b[c] - ax);
-    xout[c] = x0 + dn;
+    const T r = cheb_residual(b[c], F.diag[c], x0, xc(i + 1, j, k), xc(i - 1, j, k), xc(i, j + 1, k), xc(i, j - 1, k),
+                              xc(i, j, k + 1), xc(i, j, k - 1), F.cE[c], F.cE[c - 1], F.cN[c], F.cN[c - F.sy], F.cT[c],
+                              F.cT[c - F.sz]);
+    const T dn = fx_mul(fx_mul(coef, dinv_at(F, c)), r);
+    xout[c] = fx_add(x0, dn);
     if (dout) dout[c] = dn;
 }
 
@@ -1475,7 +1403,10 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
     T *cur[32];
     bool first_written[32] = {};    // level l's first step already written by the restriction into it
     const int last = nlev - 1;
-    for (int l = 0; l < last; ++l) {
+    // the levels from `small` down run in one launch (k_coarse.cu)
+    int small = coarse_first_level<T>(L, nlev, cc.lines != 0);
+    if (kt && small == 0) small = 1;   // the timers look at the fine level's own launches
+    for (int l = 0; l < std::min(small, last); ++l) {
         MgLevel<T> &F = L[l];
         LevelView<T> v = F.view();
         Launch3 lf = launch_interior(F.n0, F.n1, F.n2);
@@ -1568,14 +1499,19 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
         kt_end(kt, id, st);
         *launches += 1;
     }
-    {
+    if (small < last) {
+        if (coarse_ready) cudaStreamWaitEvent(st, coarse_ready, 0);
+        cur[small] = launch_coarse_cycle<T>(L + small, nlev - small, cc, ainv, map, ncoarse, singular,
+                                            small == 0 ? first_done : first_written[small], st);
+        *launches += 1;
+    } else {
         MgLevel<T> &Cst = L[last];
         if (coarse_ready) cudaStreamWaitEvent(st, coarse_ready, 0);
         k_coarse_solve<T><<<1, 128, 0, st>>>(Cst.b, Cst.x, Cst.active, ainv, map, ncoarse, singular ? 1 : 0);
         *launches += 1;
         cur[last] = Cst.x;
     }
-    for (int l = last - 1; l >= 0; --l) {
+    for (int l = std::min(small, last) - 1; l >= 0; --l) {
         MgLevel<T> &F = L[l];
         MgLevel<T> &C = L[l + 1];
         LevelView<T> v = F.view();

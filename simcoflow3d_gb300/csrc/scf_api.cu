@@ -255,6 +255,7 @@ int ensure_mg(scf_ctx *ctx)
         // the two-step smoother's shared memory (set here, outside any capture)
         CK(pair_smem_attr());
     }
+    CK(coarse_cycle_attr());
     // coarsest dense map
     const int last = ctx->nlev - 1;
     const int c0 = dims[last][0], c1 = dims[last][1], c2 = dims[last][2];

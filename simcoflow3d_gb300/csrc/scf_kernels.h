@@ -155,6 +155,16 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
              bool singular, bool first_done, cudaStream_t st, int *launches, KTimer *kt = nullptr,
              cudaEvent_t coarse_ready = nullptr);
 
+// The small levels of a V-cycle in one launch (k_coarse.cu).  The first level
+// that runs there (nlev - 1: none does), and the launch itself: levels L[0] ..
+// L[nlev - 1], the rhs in L[0].b; the result's buffer is returned.
+template <typename T>
+int coarse_first_level(const MgLevel<T> *L, int nlev, bool lines);
+template <typename T>
+T *launch_coarse_cycle(const MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, const int *map,
+                       int ncoarse, bool singular, bool first_done, cudaStream_t st);
+cudaError_t coarse_cycle_attr();   // its launch attributes (called outside any capture)
+
 // Single launches of the fine-level kernels, for timing.
 template <typename T>
 void probe_smooth(MgLevel<T> &F, const ChebCoef &cc, cudaStream_t st);
