@@ -1267,77 +1267,127 @@ void mg_coarsen(const MgLevel<T> &F, MgLevel<T> &C, cudaStream_t st, int *launch
 // Dense inverse of the coarsest operator by in-place Gauss-Jordan (SPD, no
 // pivoting); all-Neumann systems get the rank-one term s*1*1^T on the active
 // cells so that the inverse maps zero-mean vectors to the zero-mean solution.
-template <typename T>
-__global__ void __launch_bounds__(256) k_coarse_inverse(MgLevel<T> L, double *__restrict__ Aout,
-                                                        const int *__restrict__ map, int n, int singular)
+//
+// One cluster of 8 blocks, each with W columns; a thread keeps its row of them
+// in registers.  Per pivot, the block that owns the next pivot's column brings
+// it up to date first and writes it into every block's shared memory, and the
+// cluster barrier's latency runs under the other columns' updates.
+// Bound: 64 pivots' serial chain of barrier, one FP64 division and an update;
+// 128 x 128 unknowns are 2 M FMAs, 0.5 ms of one SM's FP64 pipe, which one
+// block had to itself (and every warp of it formed the division).
+constexpr int INV_BLOCKS = 8;
+
+template <typename T, int W>
+__global__ void __cluster_dims__(INV_BLOCKS) __launch_bounds__(128) k_coarse_inverse(MgLevel<T> L, double *__restrict__ Aout,
+                                                                                     const int *__restrict__ map, int n,
+                                                                                     int singular)
 {
-    extern __shared__ double A[];      // n*n, in shared memory
-    __shared__ double fcol[128];
-    __shared__ double red[2];
+    // Column buffers in a ring of three, pivot rows of two: a block runs ahead
+    // of another by less than one pivot past the barrier both have reached.
+    __shared__ double fcol[3][128], row[2][W], shift;
     __shared__ int smap[128];
-    const int t = threadIdx.x;
-    const int nt = blockDim.x;
-    for (int e = t; e < n * n; e += nt) A[e] = 0.0;
-    for (int a = t; a < n; a += nt) smap[a] = map[a];
+    __shared__ unsigned char sact[128];
+    const int a = threadIdx.x, b0 = blockIdx.x * W;   // the grid is one cluster
+    const int c = a < n ? map[a] : -1;
+    smap[a] = c;
+    sact[a] = c >= 0 && L.active[c];
     __syncthreads();
-    double dsum = 0.0, cnt = 0.0;
-    for (int a = t; a < n; a += nt) {
-        const int c = smap[a];
-        A[a * n + a] = (double)L.diag[c];
-        if (L.active[c]) { dsum += (double)L.diag[c]; cnt += 1.0; }
+    double r[W], diag = 0.0;
+#pragma unroll
+    for (int q = 0; q < W; ++q) r[q] = 0.0;
+    if (c >= 0) {
+        diag = (double)L.diag[c];
         const int nb[6] = {c + 1, c - 1, c + L.sy, c - L.sy, c + L.sz, c - L.sz};
         const T w[6] = {L.cE[c], L.cE[c - 1], L.cN[c], L.cN[c - L.sy], L.cT[c], L.cT[c - L.sz]};
-        for (int q = 0; q < 6; ++q) {
-            if (w[q] == T(0)) continue;
-            for (int b = 0; b < n; ++b)
-                if (smap[b] == nb[q]) { A[a * n + b] -= (double)w[q]; break; }
+#pragma unroll
+        for (int q = 0; q < W; ++q) {
+            const int b = b0 + q;
+            if (b >= n) continue;
+            if (b == a) r[q] = diag;
+            const int cb = smap[b];
+#pragma unroll
+            for (int p = 0; p < 6; ++p)
+                if (cb == nb[p] && w[p] != T(0)) r[q] -= (double)w[p];
         }
     }
-    dsum = block_sum(dsum);
-    __syncthreads();
-    cnt = block_sum(cnt);
-    if (t == 0) { red[0] = dsum; red[1] = cnt; }
-    __syncthreads();
-    if (singular && red[1] > 0.0) {
-        const double s = red[0] / red[1] / red[1];
-        for (int e = t; e < n * n; e += nt) {
-            const int a = e / n, b = e % n;
-            if (L.active[smap[a]] && L.active[smap[b]]) A[e] += s;
+    if (singular) {
+        const double dsum = block_sum(sact[a] ? diag : 0.0);
+        __syncthreads();
+        const double cnt = block_sum(sact[a] ? 1.0 : 0.0);
+        if (a == 0) shift = cnt > 0.0 ? dsum / cnt / cnt : 0.0;
+        __syncthreads();
+        if (sact[a]) {
+            const double s = shift;
+#pragma unroll
+            for (int q = 0; q < W; ++q)
+                if (b0 + q < n && sact[b0 + q]) r[q] += s;
         }
     }
-    __syncthreads();
+    // column b, which this block owns, into every block's ring slot
+    auto publish = [&](int b) {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < W; ++q)
+            if (b0 + q == b) v = r[q];
+        if (a >= n) return;
+        const unsigned at = (unsigned)__cvta_generic_to_shared(&fcol[b % 3][a]);
+        for (int o = 0; o < INV_BLOCKS; ++o) {
+            unsigned dst;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(at), "r"(o));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(dst), "d"(v) : "memory");
+        }
+    };
+    // no block writes into another before all have started
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (b0 == 0) publish(0);
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     for (int kk = 0; kk < n; ++kk) {
-        const double piv = A[kk * n + kk];
-        const double pinv = piv > 0.0 ? 1.0 / piv : 0.0;
-        __syncthreads();
-        for (int a = t; a < n; a += nt) fcol[a] = A[a * n + kk];
-        __syncthreads();
-        for (int b = t; b < n; b += nt) A[kk * n + b] = (b == kk) ? pinv : A[kk * n + b] * pinv;
-        __syncthreads();
-        for (int e = t; e < n * n; e += nt) {
-            const int a = e / n, b = e % n;
-            if (a == kk) continue;
-            if (b == kk)
-                A[e] = -fcol[a] * pinv;
-            else
-                A[e] -= fcol[a] * A[kk * n + b];
+        const double f = fcol[kk % 3][a < n ? a : 0];
+        double *pr = row[kk & 1];
+        if (a == kk) {
+            const double pinv = f > 0.0 ? 1.0 / f : 0.0;
+#pragma unroll
+            for (int q = 0; q < W; ++q) pr[q] = r[q] = b0 + q == kk ? pinv : r[q] * pinv;
         }
         __syncthreads();
+        const bool mine = a < n && a != kk;
+        auto update = [&](int q) {
+            const double p = pr[q];
+            r[q] = b0 + q == kk ? -f * p : __fma_rn(-f, p, r[q]);
+        };
+        const int next = kk + 1;
+        const bool owner = next < n && next >= b0 && next < b0 + W;
+        if (owner) {
+            if (mine)
+#pragma unroll
+                for (int q = 0; q < W; ++q)
+                    if (b0 + q == next) update(q);
+            publish(next);
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (mine)
+#pragma unroll
+            for (int q = 0; q < W; ++q)
+                if (!owner || b0 + q != next) update(q);
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
-    for (int e = t; e < n * n; e += nt) Aout[e] = A[e];
+    if (a < n)
+#pragma unroll
+        for (int q = 0; q < W; ++q)
+            if (b0 + q < n) Aout[a * n + b0 + q] = r[q];
 }
 
 template <typename T>
 void mg_coarse_inverse(const MgLevel<T> &L, double *ainv, int *map, int n, bool singular, cudaStream_t st,
                        int *launches)
 {
-    const size_t smem = (size_t)n * n * sizeof(double);
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_coarse_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 8);
-        attr_set = true;
-    }
-    k_coarse_inverse<T><<<1, 256, smem, st>>>(L, ainv, map, n, singular ? 1 : 0);
+    const int sg = singular ? 1 : 0;
+    if (n <= 4 * INV_BLOCKS) k_coarse_inverse<T, 4><<<INV_BLOCKS, 128, 0, st>>>(L, ainv, map, n, sg);
+    else if (n <= 8 * INV_BLOCKS) k_coarse_inverse<T, 8><<<INV_BLOCKS, 128, 0, st>>>(L, ainv, map, n, sg);
+    else k_coarse_inverse<T, 16><<<INV_BLOCKS, 128, 0, st>>>(L, ainv, map, n, sg);
     *launches += 1;
 }
 
