@@ -1270,11 +1270,12 @@ void mg_coarsen(const MgLevel<T> &F, MgLevel<T> &C, cudaStream_t st, int *launch
 //
 // One cluster of 8 blocks, each with W columns; a thread keeps its row of them
 // in registers.  Per pivot, the block that owns the next pivot's column brings
-// it up to date first and writes it into every block's shared memory, and the
-// cluster barrier's latency runs under the other columns' updates.
-// Bound: 64 pivots' serial chain of barrier, one FP64 division and an update;
-// 128 x 128 unknowns are 2 M FMAs, 0.5 ms of one SM's FP64 pipe, which one
-// block had to itself (and every warp of it formed the division).
+// it up to date first and writes it, with the pivot's inverse, into every
+// block's shared memory; the other columns' updates run under that.
+// Bound: the pivots' serial chain of one FP64 division (about 1000 cycles), an
+// update, the remote stores and the cluster barrier.  One block alone also had
+// 64 x 64 updates a pivot on one FP64 pipe and a division in every warp.
+// Measured at 27 / 64 unknowns: 56 / 270 us in one block, 28 / 77 in eight.
 constexpr int INV_BLOCKS = 8;
 
 template <typename T, int W>
@@ -1282,15 +1283,18 @@ __global__ void __cluster_dims__(INV_BLOCKS) __launch_bounds__(128) k_coarse_inv
                                                                                      const int *__restrict__ map, int n,
                                                                                      int singular)
 {
-    // Column buffers in a ring of three, pivot rows of two: a block runs ahead
-    // of another by less than one pivot past the barrier both have reached.
-    __shared__ double fcol[3][128], row[2][W], shift;
-    __shared__ int smap[128];
+    // Columns and pivots in a ring of three, pivot rows of two: a block runs
+    // ahead of another by less than one pivot past the barrier both reached.
+    __shared__ double fcol[3][128], piv[3], raw[W], row[2][W], shift;
+    __shared__ int smap[128], wcnt[4];
     __shared__ unsigned char sact[128];
-    const int a = threadIdx.x, b0 = blockIdx.x * W;   // the grid is one cluster
+    const int a = threadIdx.x, lane = a & 31, b0 = blockIdx.x * W;   // the grid is one cluster
     const int c = a < n ? map[a] : -1;
+    const bool act = c >= 0 && L.active[c];
     smap[a] = c;
-    sact[a] = c >= 0 && L.active[c];
+    sact[a] = act;
+    const unsigned vote = __ballot_sync(0xffffffffu, act);
+    if (lane == 0) wcnt[a >> 5] = __popc(vote);
     __syncthreads();
     double r[W], diag = 0.0;
 #pragma unroll
@@ -1301,41 +1305,42 @@ __global__ void __cluster_dims__(INV_BLOCKS) __launch_bounds__(128) k_coarse_inv
         const T w[6] = {L.cE[c], L.cE[c - 1], L.cN[c], L.cN[c - L.sy], L.cT[c], L.cT[c - L.sz]};
 #pragma unroll
         for (int q = 0; q < W; ++q) {
-            const int b = b0 + q;
-            if (b >= n) continue;
-            if (b == a) r[q] = diag;
-            const int cb = smap[b];
+            const int cb = b0 + q < n ? smap[b0 + q] : -1;
+            T v = T(0);
 #pragma unroll
             for (int p = 0; p < 6; ++p)
-                if (cb == nb[p] && w[p] != T(0)) r[q] -= (double)w[p];
+                if (cb == nb[p]) v = w[p];
+            r[q] = cb == c ? diag : 0.0 - (double)v;
         }
     }
     if (singular) {
-        const double dsum = block_sum(sact[a] ? diag : 0.0);
+        const double dsum = block_sum(act ? diag : 0.0);
+        const int cnt = wcnt[0] + wcnt[1] + wcnt[2] + wcnt[3];
+        if (a == 0) shift = cnt ? dsum / (double)cnt / (double)cnt : 0.0;
         __syncthreads();
-        const double cnt = block_sum(sact[a] ? 1.0 : 0.0);
-        if (a == 0) shift = cnt > 0.0 ? dsum / cnt / cnt : 0.0;
-        __syncthreads();
-        if (sact[a]) {
+        if (act) {
             const double s = shift;
 #pragma unroll
             for (int q = 0; q < W; ++q)
                 if (b0 + q < n && sact[b0 + q]) r[q] += s;
         }
     }
-    // column b, which this block owns, into every block's ring slot
-    auto publish = [&](int b) {
-        double v = 0.0;
+    auto send = [](const double *slot, double v) {   // into the slot of every block
+        const unsigned at = (unsigned)__cvta_generic_to_shared(slot);
 #pragma unroll
-        for (int q = 0; q < W; ++q)
-            if (b0 + q == b) v = r[q];
-        if (a >= n) return;
-        const unsigned at = (unsigned)__cvta_generic_to_shared(&fcol[b % 3][a]);
         for (int o = 0; o < INV_BLOCKS; ++o) {
             unsigned dst;
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(at), "r"(o));
             asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(dst), "d"(v) : "memory");
         }
+    };
+    auto publish = [&](int b) {   // column b, which this block owns, and the inverse of its pivot
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < W; ++q)
+            if (b0 + q == b) v = r[q];
+        if (a < n) send(&fcol[b % 3][a], v);
+        if (a == b) send(&piv[b % 3], v > 0.0 ? 1.0 / v : 0.0);
     };
     // no block writes into another before all have started
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
@@ -1343,31 +1348,32 @@ __global__ void __cluster_dims__(INV_BLOCKS) __launch_bounds__(128) k_coarse_inv
     __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     for (int kk = 0; kk < n; ++kk) {
-        const double f = fcol[kk % 3][a < n ? a : 0];
         double *pr = row[kk & 1];
-        if (a == kk) {
-            const double pinv = f > 0.0 ? 1.0 / f : 0.0;
+        if ((kk ^ a) < 32) {   // the pivot row's warp scales it, a lane per column
+            if (a == kk)
 #pragma unroll
-            for (int q = 0; q < W; ++q) pr[q] = r[q] = b0 + q == kk ? pinv : r[q] * pinv;
+                for (int q = 0; q < W; ++q) raw[q] = r[q];
+            __syncwarp();
+            const double pinv = piv[kk % 3];
+            if (lane < W) pr[lane] = b0 + lane == kk ? pinv : raw[lane] * pinv;
         }
+        const double f = fcol[kk % 3][a < n ? a : 0];
         __syncthreads();
-        const bool mine = a < n && a != kk;
+        // A -= f row; in the pivot's own column -f / pivot (-0.0 keeps the product's sign)
         auto update = [&](int q) {
-            const double p = pr[q];
-            r[q] = b0 + q == kk ? -f * p : __fma_rn(-f, p, r[q]);
+            r[q] = a == kk ? pr[q] : __fma_rn(-f, pr[q], b0 + q == kk ? -0.0 : r[q]);
         };
         const int next = kk + 1;
         const bool owner = next < n && next >= b0 && next < b0 + W;
         if (owner) {
-            if (mine)
 #pragma unroll
-                for (int q = 0; q < W; ++q)
-                    if (b0 + q == next) update(q);
+            for (int q = 0; q < W; ++q)
+                if (b0 + q == next && a < n) update(q);
             publish(next);
         }
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        if (mine)
+        if (a < n)
 #pragma unroll
             for (int q = 0; q < W; ++q)
                 if (!owner || b0 + q != next) update(q);
