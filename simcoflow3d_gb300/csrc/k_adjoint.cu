@@ -222,7 +222,7 @@ void launch_adj_divergence(const AdjArgs &A, Reducer &R, cudaStream_t st, int *l
     Launch3 l = launch_interior(A.d.I, A.d.J, A.d.K);
     k_adj_divergence<<<l.grid, l.block, 0, st>>>(A, R.partials, R.max_blocks);
     *launches += 1;
-    reduce2_to(R, (int)nblocks(l), 2, st, launches);
+    reduce2_to(R, (int)nblocks(l), S_JP, S_JD, st, launches);   // the loss terms
 }
 
 void launch_adj_rhs(const AdjArgs &A, const double *scal, double *b, cudaStream_t st, int *launches)

@@ -19,7 +19,7 @@
 // hide.  The solution is converted back to FP64 at the end of a CG round and
 // its residual is recomputed in FP64, so the stopping test on the true
 // residual is unchanged.
-#include "scf_kernels.h"
+#include "scf_reduce.cuh"
 
 namespace {
 
@@ -89,11 +89,12 @@ __device__ __forceinline__ float2 cf(const float *hi, const float *lo, int c) { 
 
 }  // namespace
 
-// q = A p, and the block partials of (p, q) (FP64 products and sums) and of
-// the sum of q (for the mean of A p in all-Neumann systems, which is zero in
-// exact arithmetic: double-float per thread, FP64 across threads)
+// q = A p; alpha from (p, q) (FP64 products and sums), and in all-Neumann
+// systems the mean of A p, which is zero in exact arithmetic (double-float
+// per thread, FP64 across threads)
+template <bool LAST>
 __global__ void __launch_bounds__(128, 8) k_spmv_df(DfOp A, const float2 *__restrict__ p, float2 *__restrict__ q,
-                                                 double *__restrict__ part, int n0, int kz)
+                                                 RedOut red, int kz)
 {
     DF_ZCHUNK(A);
     double v = 0.0;
@@ -121,19 +122,17 @@ __global__ void __launch_bounds__(128, 8) k_spmv_df(DfOp A, const float2 *__rest
             xm = x0; x0 = xp; tb = tt;
         }
     }
-    double dv = block_sum(v);
+    const double dv = block_sum(v);
     __syncthreads();
-    double ds = block_sum(dto(sq));
-    if (thread_linear() == 0) {
-        part[block_linear()] = dv;
-        part[n0 + block_linear()] = ds;
-    }
+    double v2[2] = {dv, block_sum(dto(sq))};
+    red_end<RK_ALPHA, LAST>(red, v2);
 }
 
 // (r, z) for beta: r double-float, z the FP32 preconditioned residual; FP64
 // products and sums
+template <bool LAST>
 __global__ void __launch_bounds__(128) k_dot_rz_df(DfOp A, const float2 *__restrict__ r, const float *__restrict__ z,
-                                                   double *__restrict__ part, int kz)
+                                                   RedOut red, int kz)
 {
     DF_ZCHUNK(A);
     double v = 0.0;
@@ -142,22 +141,22 @@ __global__ void __launch_bounds__(128) k_dot_rz_df(DfOp A, const float2 *__restr
         int c = i + sy * j + sz * k0;
         for (int k = k0; k <= k1; ++k, c += sz) v = fma(dwide(ld(r, c)), widen(z[c]), v);
     }
-    v = block_sum(v);
-    if (thread_linear() == 0) part[block_linear()] = v;
+    red_end<RK_BETA, LAST>(red, block_sum(v));
 }
 
 // x += alpha p, r -= alpha (q - mean q), (r, r) in FP64; also the FP32 copy
 // of r (its hi part) for the V-cycle and, when x0 is given, the first
 // point-Jacobi smoothing step from a zero guess, x0 = first D^-1 r.
+template <bool LAST>
 __global__ void __launch_bounds__(128) k_cg_update_df(DfOp A, float2 *__restrict__ x, float2 *__restrict__ r,
                                                       const float2 *__restrict__ p, const float2 *__restrict__ q,
                                                       float *__restrict__ rlow, float *__restrict__ x0, float first,
-                                                      const double *__restrict__ scal, double *__restrict__ part, int kz)
+                                                      RedOut red, int kz)
 {
     DF_ZCHUNK(A);
     double v = 0.0;
     if (in) {
-        const float2 al = dfrom(scal[S_ALPHA]), mal = dneg(al), qm = dfrom(scal[S_QMEAN]);
+        const float2 al = dfrom(red.scal[S_ALPHA]), mal = dneg(al), qm = dfrom(red.scal[S_QMEAN]);
         const int sy = A.hi.sy, sz = A.hi.sz;
         int c = i + sy * j + sz * k0;
         for (int k = k0; k <= k1; ++k, c += sz) {
@@ -173,8 +172,7 @@ __global__ void __launch_bounds__(128) k_cg_update_df(DfOp A, float2 *__restrict
             v = fma(rd, rd, v);
         }
     }
-    v = block_sum(v);
-    if (thread_linear() == 0) part[block_linear()] = v;
+    red_end<RK_RR, LAST>(red, block_sum(v));
 }
 
 // p = z + beta p (p = z on the first call)
@@ -223,18 +221,20 @@ void df_spmv_dot(const DfOp &A, const float2 *p, float2 *q, Reducer &R, bool sin
 {
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     const int id = kt_begin(kt, KC_SPMV, st);
-    k_spmv_df<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_spmv_df<true> : k_spmv_df<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, p, q, red_out(R, singular), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
-    reduce_alpha(R, (int)nblocks(l), singular, st, launches);
+    red_finish<RK_ALPHA>(R, nblocks(l), singular, st, launches);
 }
 
 void df_dot_rz(const DfOp &A, const float2 *r, const float *z, Reducer &R, cudaStream_t st, int *launches)
 {
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
-    k_dot_rz_df<<<l.grid, l.block, 0, st>>>(A, r, z, R.partials, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_dot_rz_df<true> : k_dot_rz_df<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, r, z, red_out(R), l.kz);
     *launches += 1;
-    reduce_beta(R, (int)nblocks(l), st, launches);
+    red_finish<RK_BETA>(R, nblocks(l), false, st, launches);
 }
 
 void df_cg_update(const DfOp &A, float2 *x, float2 *r, const float2 *p, const float2 *q, float *rlow, float *x0,
@@ -242,10 +242,11 @@ void df_cg_update(const DfOp &A, float2 *x, float2 *r, const float2 *p, const fl
 {
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     const int id = kt_begin(kt, KC_CGUPDATE, st);
-    k_cg_update_df<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, x0, (float)first, R.scal, R.partials, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_cg_update_df<true> : k_cg_update_df<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, x0, (float)first, red_out(R), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
-    reduce_to(R, (int)nblocks(l), S_RR, st, launches);
+    red_finish<RK_RR>(R, nblocks(l), false, st, launches);
 }
 
 void df_pupdate(const DfOp &A, const float *z, float2 *p, const double *scal, bool first, cudaStream_t st,

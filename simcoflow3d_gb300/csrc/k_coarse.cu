@@ -17,8 +17,8 @@
 // Bound: the latency of a step -- six remote shared-memory reads per cell
 // (some 10 cycles per warp and read at an SM's port) and the cluster barrier
 // (480 cycles at 512 threads), 1200 to 1800 cycles together.  Measured, a
-// whole projection with a launch per step -> with this kernel: 20^3 FP32
-// V-cycle 1245 -> 1036 us, 64^3 FP64 2612 -> 2435, 74x47x61 3997 -> 3833,
+// whole projection with a launch per step -> with this kernel: 40^3 FP32
+// V-cycle 1245 -> 1036 us, 64^3 FP64 2612 -> 2435, 147x93x121 3997 -> 3833,
 // 256x128x128 with lines 8677 -> 7465 (the kernel itself 22 us, 27, 21, 119).
 // Four cells per thread (32^3 levels) lose: 4000 to 6000 cycles a step where
 // the chip-wide kernel takes 2.5 us.  Nor does a cheaper exchange help: with

@@ -17,6 +17,7 @@
 
 #include "scf_cheb.cuh"
 #include "scf_kernels.h"
+#include "scf_reduce.cuh"
 #include "scf_tma.cuh"
 
 #define INTERIOR_IJK(L)                                       \
@@ -25,37 +26,6 @@
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1; \
     const bool in = i <= (L).n0 && j <= (L).n1 && k <= (L).n2; \
     const int c = i + (L).sy * j + (L).sz * k;
-
-// ---------------------------------------------------------------------------
-// reductions
-
-enum ReduceMode { RM_STORE = 0, RM_BETA = 2, RM_MEAN = 3 };
-
-__global__ void __launch_bounds__(1024) k_reduce(const double *__restrict__ part, int n, double *scal, int slot,
-                                                 int mode)
-{
-    double s = 0.0;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) s += part[t];
-    s = block_sum(s);
-    if (threadIdx.x == 0) {
-        if (mode == RM_BETA) {
-            const double old = scal[S_RZ];
-            scal[S_BETA] = old != 0.0 ? s / old : 0.0;
-            scal[S_RZ] = s;
-        } else if (mode == RM_MEAN) {
-            scal[S_SUM] = s;
-            scal[S_MEAN] = scal[S_COUNT] > 0.0 ? s / scal[S_COUNT] : 0.0;
-        } else {
-            scal[slot] = s;
-        }
-    }
-}
-
-void reduce_to(Reducer &R, int nblocks, int slot, cudaStream_t st, int *launches)
-{
-    k_reduce<<<1, 1024, 0, st>>>(R.partials, nblocks, R.scal, slot, RM_STORE);
-    *launches += 1;
-}
 
 // ---------------------------------------------------------------------------
 // FP64 CG kernels on the fine level
@@ -70,10 +40,11 @@ void reduce_to(Reducer &R, int nblocks, int slot, cudaStream_t st, int *launches
     const int k1 = min(k0 + kz - 1, (L).n2);                          \
     const bool in = i <= (L).n0 && j <= (L).n1;
 
-// q = A p and the block partials of (p, q) and of the sum of q (q is zero on
-// inactive cells, whose p is zero and which couple to nothing).
+// q = A p, alpha from (p, q), and the mean of q (q is zero on inactive cells,
+// whose p is zero and which couple to nothing).
+template <bool LAST>
 __global__ void __launch_bounds__(128) k_spmv_dot(LevelView<double> A, const double *__restrict__ p,
-                                                  double *__restrict__ q, double *__restrict__ part, int n0, int kz)
+                                                  double *__restrict__ q, RedOut red, int kz)
 {
     ZCHUNK_IJK(A);
     double v = 0.0, sq = 0.0;
@@ -92,41 +63,8 @@ __global__ void __launch_bounds__(128) k_spmv_dot(LevelView<double> A, const dou
     }
     v = block_sum(v);
     __syncthreads();
-    sq = block_sum(sq);
-    if (thread_linear() == 0) {
-        part[block_linear()] = v;
-        part[n0 + block_linear()] = sq;
-    }
-}
-
-// alpha = (r, z) / (p, q); for an all-Neumann system also the mean of q over
-// the active cells.  That mean is zero in exact arithmetic (the constant is
-// the null vector of the symmetric operator); the CG update subtracts the
-// rounding that it carries, so that the recursive residual stays in the
-// range of the operator instead of collecting a component that no iterate
-// can remove.
-__global__ void __launch_bounds__(1024) k_reduce_alpha(const double *__restrict__ part, int n, int n0,
-                                                       double *scal, int singular)
-{
-    double s = 0.0, t = 0.0;
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-        s += part[q];
-        t += part[n0 + q];
-    }
-    s = block_sum(s);
-    __syncthreads();
-    t = block_sum(t);
-    if (threadIdx.x == 0) {
-        scal[S_PQ] = s;
-        scal[S_ALPHA] = s != 0.0 ? scal[S_RZ] / s : 0.0;
-        scal[S_QMEAN] = (singular && scal[S_COUNT] > 0.0) ? t / scal[S_COUNT] : 0.0;
-    }
-}
-
-void reduce_alpha(Reducer &R, int nblocks, bool singular, cudaStream_t st, int *launches)
-{
-    k_reduce_alpha<<<1, 1024, 0, st>>>(R.partials, nblocks, R.max_blocks, R.scal, singular ? 1 : 0);
-    *launches += 1;
+    double v2[2] = {v, block_sum(sq)};
+    red_end<RK_ALPHA, LAST>(red, v2);
 }
 
 void cg_spmv_dot(const LevelView<double> &A, const double *p, double *q, Reducer &R, bool singular,
@@ -134,27 +72,28 @@ void cg_spmv_dot(const LevelView<double> &A, const double *p, double *q, Reducer
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
     const int id = kt_begin(kt, KC_SPMV, st);
-    k_spmv_dot<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_spmv_dot<true> : k_spmv_dot<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, p, q, red_out(R, singular), l.kz);
     kt_end(kt, id, st);
-    k_reduce_alpha<<<1, 1024, 0, st>>>(R.partials, (int)nblocks(l), R.max_blocks, R.scal, singular ? 1 : 0);
-    *launches += 2;
+    *launches += 1;
+    red_finish<RK_ALPHA>(R, nblocks(l), singular, st, launches);
 }
 
 // x += alpha p, r -= alpha (q - mean q), (r, r); also writes the preconditioner's
 // level-0 rhs (FP32 copy of r in mixed mode) and the first Chebyshev step
 // of the V-cycle from a zero guess, x0 = dinv * r / theta, which saves that
 // pass in the V-cycle.
-template <typename T>
+template <typename T, bool LAST>
 __global__ void __launch_bounds__(128) k_cg_update(LevelView<double> A, double *__restrict__ x,
                                                    double *__restrict__ r, const double *__restrict__ p,
                                                    const double *__restrict__ q, T *__restrict__ rlow,
                                                    LevelView<T> L0, T *__restrict__ x0, T first,
-                                                   const double *__restrict__ scal, double *__restrict__ part, int kz)
+                                                   RedOut red, int kz)
 {
     ZCHUNK_IJK(A);
     double v = 0.0;
     if (in) {
-        const double alpha = scal[S_ALPHA], qm = scal[S_QMEAN];
+        const double alpha = red.scal[S_ALPHA], qm = red.scal[S_QMEAN];
         int c = i + A.sy * j + A.sz * k0;
         for (int k = k0; k <= k1; ++k, c += A.sz) {
             x[c] = x[c] + alpha * p[c];
@@ -166,8 +105,7 @@ __global__ void __launch_bounds__(128) k_cg_update(LevelView<double> A, double *
             v += rn * rn;
         }
     }
-    v = block_sum(v);
-    if (thread_linear() == 0) part[block_linear()] = v;
+    red_end<RK_RR, LAST>(red, block_sum(v));
 }
 
 template <typename T>
@@ -177,20 +115,21 @@ void cg_update(const LevelView<double> &A, double *x, double *r, const double *p
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
     const int id = kt_begin(kt, KC_CGUPDATE, st);
-    k_cg_update<T><<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, L0, x0, (T)first, R.scal, R.partials, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_cg_update<T, true> : k_cg_update<T, false>;
+    k<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, L0, x0, (T)first, red_out(R), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
-    reduce_to(R, (int)nblocks(l), S_RR, st, launches);
+    red_finish<RK_RR>(R, nblocks(l), false, st, launches);
 }
 
 // (r, z): in mixed mode r is taken from its FP32 copy (the V-cycle's rhs) and
 // the products are formed in FP32, accumulated per thread in FP32 over kz
 // cells and across threads in FP64; z is an FP32 preconditioner output, so
 // this loses nothing that matters for beta.  FP64 mode: FP64 throughout.
-template <typename T>
+template <typename T, bool LAST>
 __global__ void __launch_bounds__(128) k_dot_rz(LevelView<double> A, const double *__restrict__ r,
                                                 const T *__restrict__ rlow, const T *__restrict__ z,
-                                                double *__restrict__ part, int kz)
+                                                RedOut red, int kz)
 {
     ZCHUNK_IJK(A);
     double v = 0.0;
@@ -204,8 +143,7 @@ __global__ void __launch_bounds__(128) k_dot_rz(LevelView<double> A, const doubl
             for (int k = k0; k <= k1; ++k, c += A.sz) v += r[c] * (double)z[c];
         }
     }
-    v = block_sum(v);
-    if (thread_linear() == 0) part[block_linear()] = v;
+    red_end<RK_BETA, LAST>(red, block_sum(v));
 }
 
 template <typename T>
@@ -213,15 +151,10 @@ void cg_dot_rz(const LevelView<double> &A, const double *r, const T *rlow, const
                int *launches)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    k_dot_rz<T><<<l.grid, l.block, 0, st>>>(A, r, rlow, z, R.partials, l.kz);
-    k_reduce<<<1, 1024, 0, st>>>(R.partials, (int)nblocks(l), R.scal, 0, RM_BETA);
-    *launches += 2;
-}
-
-void reduce_beta(Reducer &R, int nblocks, cudaStream_t st, int *launches)
-{
-    k_reduce<<<1, 1024, 0, st>>>(R.partials, nblocks, R.scal, 0, RM_BETA);
+    auto *k = red_last(nblocks(l)) ? k_dot_rz<T, true> : k_dot_rz<T, false>;
+    k<<<l.grid, l.block, 0, st>>>(A, r, rlow, z, red_out(R), l.kz);
     *launches += 1;
+    red_finish<RK_BETA>(R, nblocks(l), false, st, launches);
 }
 
 template <typename T>
@@ -250,7 +183,7 @@ void cg_pupdate(const LevelView<double> &A, const T *z, double *p, const double 
 
 // two-slot reduction: sums of part[0..n) and part[n0..n0+n)
 __global__ void __launch_bounds__(1024) k_reduce2(const double *__restrict__ part, int n, int n0,
-                                                  double *scal, int mode)
+                                                  double *scal, int slot0, int slot1)
 {
     double s = 0.0, t = 0.0;
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
@@ -261,23 +194,14 @@ __global__ void __launch_bounds__(1024) k_reduce2(const double *__restrict__ par
     __syncthreads();
     t = block_sum(t);
     if (threadIdx.x == 0) {
-        if (mode == 0) {           // sum of b, count
-            scal[S_SUM] = s;
-            scal[S_COUNT] = t;
-            scal[S_MEAN] = t > 0.0 ? s / t : 0.0;
-        } else if (mode == 1) {    // (r, r), sum of x
-            scal[S_RR] = s;
-            scal[S_MEANX] = scal[S_COUNT] > 0.0 ? t / scal[S_COUNT] : 0.0;
-        } else {                   // loss terms
-            scal[S_JP] = s;
-            scal[S_JD] = t;
-        }
+        scal[slot0] = s;
+        scal[slot1] = t;
     }
 }
 
+template <bool LAST>
 __global__ void __launch_bounds__(128) k_sum_count(LevelView<double> A, const unsigned char *__restrict__ act,
-                                                   const double *__restrict__ v, double *__restrict__ part, int n0,
-                                                   int kz)
+                                                   const double *__restrict__ v, RedOut red, int kz)
 {
     ZCHUNK_IJK(A);
     double s = 0.0, cnt = 0.0;
@@ -288,21 +212,19 @@ __global__ void __launch_bounds__(128) k_sum_count(LevelView<double> A, const un
     }
     s = block_sum(s);
     __syncthreads();
-    cnt = block_sum(cnt);
-    if (thread_linear() == 0) {
-        part[block_linear()] = s;
-        part[n0 + block_linear()] = cnt;
-    }
+    double v2[2] = {s, block_sum(cnt)};
+    red_end<RK_COUNT, LAST>(red, v2);
 }
 
+template <bool LAST>
 __global__ void __launch_bounds__(128) k_center_norm(LevelView<double> A, const unsigned char *__restrict__ act,
-                                                     double *__restrict__ b, const double *__restrict__ scal,
-                                                     int singular, double *__restrict__ part, int kz)
+                                                     double *__restrict__ b, RedOut red, int kz)
 {
     ZCHUNK_IJK(A);
     double s = 0.0;
     if (in) {
-        const double mu = singular ? scal[S_MEAN] : 0.0;
+        const bool singular = red.singular;
+        const double mu = singular ? red.scal[S_MEAN] : 0.0;
         int c = i + A.sy * j + A.sz * k0;
         for (int k = k0; k <= k1; ++k, c += A.sz) {
             double v = b[c];
@@ -310,13 +232,12 @@ __global__ void __launch_bounds__(128) k_center_norm(LevelView<double> A, const 
             s += v * v;
         }
     }
-    s = block_sum(s);
-    if (thread_linear() == 0) part[block_linear()] = s;
+    red_end<RK_BB, LAST>(red, block_sum(s));
 }
 
-void reduce2_to(Reducer &R, int nblocks, int mode, cudaStream_t st, int *launches)
+void reduce2_to(Reducer &R, int nblocks, int slot0, int slot1, cudaStream_t st, int *launches)
 {
-    k_reduce2<<<1, 1024, 0, st>>>(R.partials, nblocks, R.max_blocks, R.scal, mode);
+    k_reduce2<<<1, 1024, 0, st>>>(R.partials, nblocks, R.max_blocks, R.scal, slot0, slot1);
     *launches += 1;
 }
 
@@ -324,30 +245,33 @@ void active_mean(const LevelView<double> &A, const unsigned char *active, const 
                  cudaStream_t st, int *launches)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    k_sum_count<<<l.grid, l.block, 0, st>>>(A, active, v, R.partials, R.max_blocks, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_sum_count<true> : k_sum_count<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, active, v, red_out(R), l.kz);
     *launches += 1;
-    reduce2_to(R, (int)nblocks(l), 0, st, launches);
+    red_finish<RK_COUNT>(R, nblocks(l), false, st, launches);
 }
 
 void rhs_prologue(const LevelView<double> &A, const unsigned char *active, double *b, bool singular, Reducer &R,
                   cudaStream_t st, int *launches)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    const int nb = (int)nblocks(l);
     if (singular) {
-        k_sum_count<<<l.grid, l.block, 0, st>>>(A, active, b, R.partials, R.max_blocks, l.kz);
-        k_reduce2<<<1, 1024, 0, st>>>(R.partials, nb, R.max_blocks, R.scal, 0);
-        *launches += 2;
+        auto *k = red_last(nblocks(l)) ? k_sum_count<true> : k_sum_count<false>;
+        k<<<l.grid, l.block, 0, st>>>(A, active, b, red_out(R), l.kz);
+        *launches += 1;
+        red_finish<RK_COUNT>(R, nblocks(l), false, st, launches);
     }
-    k_center_norm<<<l.grid, l.block, 0, st>>>(A, active, b, R.scal, singular ? 1 : 0, R.partials, l.kz);
-    k_reduce<<<1, 1024, 0, st>>>(R.partials, nb, R.scal, S_BB, RM_STORE);
-    *launches += 2;
+    auto *k = red_last(nblocks(l)) ? k_center_norm<true> : k_center_norm<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, active, b, red_out(R, singular), l.kz);
+    *launches += 1;
+    red_finish<RK_BB>(R, nblocks(l), singular, st, launches);
 }
 
+template <bool LAST>
 __global__ void __launch_bounds__(128) k_final_residual(LevelView<double> A, const unsigned char *__restrict__ act,
                                                         const double *__restrict__ b, const double *__restrict__ x,
-                                                        double *__restrict__ r, int singular,
-                                                        double *__restrict__ part, int n0, int kz)
+                                                        double *__restrict__ r, int singular, RedOut red,
+                                                        int kz)
 {
     ZCHUNK_IJK(A);
     double s = 0.0, sx = 0.0;
@@ -362,21 +286,18 @@ __global__ void __launch_bounds__(128) k_final_residual(LevelView<double> A, con
     }
     s = block_sum(s);
     __syncthreads();
-    sx = block_sum(sx);
-    if (thread_linear() == 0) {
-        part[block_linear()] = s;
-        part[n0 + block_linear()] = sx;
-    }
+    double v[2] = {s, block_sum(sx)};
+    red_end<RK_RESIDUAL, LAST>(red, v);
 }
 
 void final_residual(const LevelView<double> &A, const unsigned char *active, const double *b, const double *x,
                     double *r, bool singular, Reducer &R, cudaStream_t st, int *launches)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    const int nb = (int)nblocks(l);
-    k_final_residual<<<l.grid, l.block, 0, st>>>(A, active, b, x, r, singular ? 1 : 0, R.partials, R.max_blocks, l.kz);
-    k_reduce2<<<1, 1024, 0, st>>>(R.partials, nb, R.max_blocks, R.scal, 1);
-    *launches += 2;
+    auto *k = red_last(nblocks(l)) ? k_final_residual<true> : k_final_residual<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, active, b, x, r, singular ? 1 : 0, red_out(R), l.kz);
+    *launches += 1;
+    red_finish<RK_RESIDUAL>(R, nblocks(l), false, st, launches);
 }
 
 __global__ void __launch_bounds__(128) k_shift(LevelView<double> A, const unsigned char *__restrict__ act,
@@ -1684,7 +1605,8 @@ void probe_prolong(MgLevel<T> &F, MgLevel<T> &C, const ChebCoef &cc, cudaStream_
 void probe_spmv(const LevelView<double> &A, const double *p, double *q, Reducer &R, cudaStream_t st)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    k_spmv_dot<<<l.grid, l.block, 0, st>>>(A, p, q, R.partials, R.max_blocks, l.kz);
+    auto *k = red_last(nblocks(l)) ? k_spmv_dot<true> : k_spmv_dot<false>;
+    k<<<l.grid, l.block, 0, st>>>(A, p, q, red_out(R), l.kz);
 }
 
 template void probe_smooth<float>(MgLevel<float> &, const ChebCoef &, cudaStream_t);

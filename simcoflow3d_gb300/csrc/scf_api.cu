@@ -1019,6 +1019,7 @@ int scf_ctx_create(scf_ctx **out, int32_t imax, int32_t jmax, int32_t kmax, cons
     ctx->R.max_blocks = (int)nblocks(l);
     A(ctx->R.partials, 2 * ctx->R.max_blocks + 1024);
     A(ctx->R.scal, S_NUM);
+    A(ctx->R.done, 1);
 #undef A
     if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) return fail(SCF_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&ctx->cst, cudaStreamNonBlocking) != cudaSuccess) return fail(SCF_ERR_CUDA);

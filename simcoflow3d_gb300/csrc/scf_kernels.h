@@ -85,6 +85,7 @@ struct Reducer {
     double *partials;    // >= max blocks of any reducing launch
     double *scal;        // ScfScalar slots
     int max_blocks;
+    unsigned *done;      // blocks of the running launch that have finished (0 between launches)
 };
 
 // Coarsening and the coarsest dense inverse.
@@ -203,10 +204,6 @@ void df_from_double(const double *src, float2 *dst, int n, cudaStream_t st, int 
 // its FP32 hi part written to rlow
 void df_round_start(double *r, float *rlow, int n, cudaStream_t st, int *launches);
 void df_to_double(const float2 *src, double *dst, int n, cudaStream_t st, int *launches);
-// alpha and the mean of A p from the two-lane partials of an SpMV
-void reduce_alpha(Reducer &R, int nblocks, bool singular, cudaStream_t st, int *launches);
-// beta = (r, z) / (previous (r, z)) from one-lane partials; (r, z) kept
-void reduce_beta(Reducer &R, int nblocks, cudaStream_t st, int *launches);
 
 // CG building blocks on the fine level (FP64 vectors, ghosted layout).
 void cg_spmv_dot(const LevelView<double> &A, const double *p, double *q, Reducer &R, bool singular,
@@ -221,7 +218,6 @@ void cg_dot_rz(const LevelView<double> &A, const double *r, const T *rlow, const
 template <typename T>
 void cg_pupdate(const LevelView<double> &A, const T *z, double *p, const double *scal, bool first, cudaStream_t st,
                 int *launches);
-void reduce_to(Reducer &R, int nblocks, int slot, cudaStream_t st, int *launches);
 // Right-hand side prologue: for an all-Neumann system the mean of b over the
 // active cells is removed (S_COUNT, S_MEAN); then S_BB = (b, b).
 void rhs_prologue(const LevelView<double> &A, const unsigned char *active, double *b, bool singular, Reducer &R,
@@ -235,9 +231,8 @@ void shift_solution(const LevelView<double> &A, const unsigned char *active, dou
                     cudaStream_t st, int *launches);
 void copy_to_low(const LevelView<double> &A, const double *src, float *dst, cudaStream_t st, int *launches);
 
-// sums of two partial arrays: mode 0 sum+count (S_SUM, S_COUNT, S_MEAN),
-// 1 (S_RR, S_MEANX), 2 loss terms (S_JP, S_JD)
-void reduce2_to(Reducer &R, int nblocks, int mode, cudaStream_t st, int *launches);
+// sums of two partial arrays into two scalar slots
+void reduce2_to(Reducer &R, int nblocks, int slot0, int slot1, cudaStream_t st, int *launches);
 // S_MEAN = mean of v over the active cells
 void active_mean(const LevelView<double> &A, const unsigned char *active, const double *v, Reducer &R,
                  cudaStream_t st, int *launches);
