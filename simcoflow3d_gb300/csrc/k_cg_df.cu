@@ -19,6 +19,7 @@
 // hide.  The solution is converted back to FP64 at the end of a CG round and
 // its residual is recomputed in FP64, so the stopping test on the true
 // residual is unchanged.
+#include "scf_df.cuh"
 #include "scf_reduce.cuh"
 
 namespace {
@@ -59,22 +60,6 @@ __device__ __forceinline__ float2 dfrom(double d)
 }
 __device__ __forceinline__ double dto(float2 x) { return (double)x.x + (double)x.y; }
 
-// FP32 -> FP64 widening on the integer pipe (exact: the exponent is rebiased
-// and the significand shifted into place).  Zeros keep their sign; the rare
-// subnormal inputs, Inf and NaN take the hardware conversion.
-__device__ __forceinline__ double widen(float f)
-{
-    const unsigned u = __float_as_uint(f);
-    const unsigned e = (u >> 23) & 0xffu;
-    if (e - 1u < 254u) {   // normal numbers
-        const unsigned hi = (u & 0x80000000u) | ((e + 896u) << 20) | ((u & 0x7fffffu) >> 3);
-        return __hiloint2double((int)hi, (int)(u << 29));
-    }
-    if ((u & 0x7fffffffu) == 0u) return __hiloint2double((int)(u & 0x80000000u), 0);
-    return (double)f;
-}
-// the FP64 value of a double-float: one FP64 addition
-__device__ __forceinline__ double dwide(float2 x) { return widen(x.x) + widen(x.y); }
 __device__ __forceinline__ float2 ld(const float2 *__restrict__ v, int c) { return v[c]; }
 
 #define DF_ZCHUNK(A)                                                   \
@@ -139,7 +124,20 @@ __global__ void __launch_bounds__(128) k_dot_rz_df(DfOp A, const float2 *__restr
     if (in) {
         const int sy = A.hi.sy, sz = A.hi.sz;
         int c = i + sy * j + sz * k0;
-        for (int k = k0; k <= k1; ++k, c += sz) v = fma(dwide(ld(r, c)), widen(z[c]), v);
+        // four cells' loads in flight at a time
+        for (int k = k0; k <= k1; k += 4) {
+            float2 rr[4];
+            float zz[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const bool on = k + u <= k1;
+                rr[u] = on ? ld(r, c + u * sz) : make_float2(0.f, 0.f);
+                zz[u] = on ? z[c + u * sz] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v = fma(dwide(rr[u]), widen(zz[u]), v);
+            c += 4 * sz;
+        }
     }
     red_end<RK_BETA, LAST>(red, block_sum(v));
 }
