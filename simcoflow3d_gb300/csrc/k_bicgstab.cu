@@ -11,14 +11,16 @@
 //      and the stopping test
 // s is never stored.  Each thread marches d.kz cells of one (i, j) column and
 // keeps its share of the dot products in registers, so a block writes one
-// partial sum per dot for 128 x kz cells; after each of P, S and X one
-// block of 1024 threads sums the partials in a fixed order (so every run is
-// bitwise reproducible) and updates the scalars, which stay in device
-// memory.  (Summing them in the last block of the pass instead was slower:
-// 128 threads on one SM add 8192 partials.)  The reduction after X sets
-// `done` when ||r||^2 <= target or on a breakdown, and every kernel after
-// that returns at once, so the host enqueues several iterations and reads
-// the scalars once per batch.
+// partial sum per dot for 128 x kz cells; after each of P, S and X the
+// partials are summed in a fixed order (so every run is bitwise
+// reproducible) and the scalars updated, which stay in device memory: by the
+// block that finishes last on grids up to LAST_MAX, else by a launch of one
+// block.  (The launches were 4 to 5 us each, three per iteration: a predictor
+// step at 67x53x75 in FP64 2570 us with them, 2280 without; at 128x112x96
+// mixed 4457 and 4205.)  The reduction after X sets `done` when
+// ||r||^2 <= target or on a breakdown, and every kernel after that returns at
+// once, so the host enqueues several iterations and reads the scalars once
+// per batch.
 #include "pred_kernels.h"
 
 namespace pred {
@@ -26,16 +28,124 @@ namespace {
 
 constexpr int NT = 128;
 
-// Sum of up to 4 values over the block; thread 0 writes them to
-// partials[4 * block + q].  The products and the warp sums are formed in A
-// (FP32 for the FP32 iteration: this GPU runs FP64 at 1/64 of the FP32
-// rate), the sums over the block's warps and over the blocks in FP64.
-template <int Q, typename A>
-__device__ __forceinline__ void block_partials(A (&v)[Q], double *partials)
+__device__ __forceinline__ bool finite_nonzero(double a) { return a != 0.0 && isfinite(a); }
+
+// What a pass sums: r0.v; t.s and t.t; r0.r and r.r; ||r||^2, ||r_T||^2 and ||b||^2.
+enum RedKind { BR_ALPHA, BR_OMEGA, BR_RHO, BR_RESID };
+constexpr int red_sums(int kind) { return kind == BR_ALPHA ? 1 : kind == BR_RESID ? 3 : 2; }
+
+struct Red {
+    double *partials;   // 4 per block
+    unsigned *finished; // blocks of the running pass that have; 0 between passes
+    BcgScalars *sc;
+    int want_bb;
+};
+// Blocks up to which the last one sums a pass: one resident wave of P and S
+// (16 blocks per SM), half of that of X and the residual, where a block's
+// fence waits for more stores.  Beyond, the fences cost more than a launch.
+constexpr int LAST_MAX = 152 * 16, LAST_MAX_X = 152 * 8;
+
+// The scalars from a pass's sums, by one warp (which divides in one go).
+template <int KIND>
+__device__ __forceinline__ void scalars(BcgScalars *sc, const double (&s)[red_sums(KIND)], int want_bb)
 {
+    const int lane = threadIdx.x & 31;   // blocks are 32 wide
+    if constexpr (KIND == BR_ALPHA) {    // alpha = rho / (r0.v)
+        if (lane) return;
+        const double a = sc->rho / s[0];
+        if (finite_nonzero(s[0]) && isfinite(a)) sc->alpha = a;
+        else { sc->alpha = 0.0; sc->breakdown = 1; sc->done = 1; }
+    } else if constexpr (KIND == BR_OMEGA) {
+        // omega = (t.s) / (t.t); t.t = 0 means s = 0 (omega = 0 finishes)
+        if (lane) return;
+        const double w = s[1] > 0.0 ? s[0] / s[1] : 0.0;
+        sc->omega = isfinite(w) ? w : 0.0;
+    } else if constexpr (KIND == BR_RHO) {
+        // beta = (rho_new / rho) (alpha / omega), rho = rho_new, rr, and the stopping test
+        const double omega = sc->omega, num = lane == 1 ? sc->alpha : s[0], den = lane == 1 ? omega : sc->rho;
+        const double quot = num / den, other = __shfl_sync(0xffffffffu, quot, 1);
+        if (lane) return;
+        sc->rr = s[1];
+        sc->iters += 1;
+        const double b = quot * other;
+        if (finite_nonzero(s[0]) && omega != 0.0 && isfinite(b)) sc->beta = b;
+        else { sc->beta = 0.0; sc->breakdown = 1; sc->done = 1; }
+        sc->rho = s[0];
+        if (!(s[1] > sc->target)) sc->done = 1;   // converged (or NaN: the host checks)
+    } else {   // a fresh start (p = r on the next P)
+        if (lane) return;
+        sc->rr = s[0];
+        sc->rho = s[1];
+        if (want_bb) sc->bb = s[2];
+        sc->alpha = 1.0;
+        sc->omega = 1.0;
+        sc->beta = 0.0;
+        sc->breakdown = 0;
+        sc->done = 0;
+        sc->iters = 0;
+    }
+}
+
+// Sums the partials of nb blocks with 128 threads: 1024 strided sums, eight
+// per thread, then a tree over their index (512, 256, ... 1 apart), whose
+// first three levels are the thread's own.
+template <int KIND>
+__device__ __forceinline__ void red_tail(const Red &R, int nb)
+{
+    constexpr int Q = red_sums(KIND);
+    __shared__ double sh[Q][NT];
+    const int t = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    double a[Q][8];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[q][j] = 0.0;
+    for (int m = 0; m < nb; m += 8 * NT) {
+        double p[Q][8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = m + t + NT * j;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) p[q][j] = e < nb ? __ldcg(R.partials + 4 * (long long)e + q) : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (m + NT * j < nb)   // (an FP64 addition of nothing would still hold the pipe)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) a[q][j] += p[q][j];
+    }
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1)
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int j = 0; j < d; ++j) a[q][j] += a[q][j + d];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) sh[q][t] = a[q][0];
+    __syncthreads();
+    if (t >= 32) return;
+    double s[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        s[q] = (sh[q][t] + sh[q][t + 64]) + (sh[q][t + 32] + sh[q][t + 96]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
+    }
+    scalars<KIND>(R.sc, s, R.want_bb);   // (s is the sums in lane 0)
+}
+
+// The end of a pass: the block's sums to its partials, and with LAST the
+// grid's in the block that finishes last.  The products and the warp sums are
+// formed in A (FP32 for the FP32 iteration: this GPU runs FP64 at 1/64 of the
+// FP32 rate), the sums over the block's warps and over the blocks in FP64.
+template <int KIND, bool LAST, typename A>
+__device__ __forceinline__ void pass_end(A (&v)[red_sums(KIND)], const Red &R)
+{
+    constexpr int Q = red_sums(KIND);
     __shared__ double sh[NT / 32][4];
+    __shared__ int last;
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-    const int lane = tid & 31, warp = tid >> 5;
+    const int lane = tid & 31, warp = tid >> 5, nb = (int)(gridDim.x * gridDim.y * gridDim.z);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         A a = v[q];
@@ -50,12 +160,28 @@ __device__ __forceinline__ void block_partials(A (&v)[Q], double *partials)
         for (int q = 0; q < Q; ++q) {
             double a = 0.0;
             for (int w = 0; w < NT / 32; ++w) a += sh[w][q];
-            partials[4 * blk + q] = a;
+            R.partials[4 * blk + q] = a;
         }
+        if (LAST) {
+            __threadfence();
+            last = atomicAdd(R.finished, 1u) == (unsigned)nb - 1u;
+        }
+    }
+    if constexpr (LAST) {
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        if (tid == 0) *R.finished = 0;
+        red_tail<KIND>(R, nb);
     }
 }
 
-__device__ __forceinline__ bool finite_nonzero(double a) { return a != 0.0 && isfinite(a); }
+template <int KIND>
+__global__ void __launch_bounds__(NT) k_red(Red R, int nb)
+{
+    if (KIND != BR_RESID && R.sc->done) return;
+    red_tail<KIND>(R, nb);
+}
 
 template <typename T>
 struct M6 {
@@ -94,11 +220,11 @@ __global__ void __launch_bounds__(NT) k_bcg_u(Dims d, const T *__restrict__ r, T
         for (int k = k0; k <= k1; ++k, c += d.sz) p[c] = r[c] + beta * (p[c] - omega * v[c]);
 }
 
-template <typename T>
+template <typename T, bool LAST>
 __global__ void __launch_bounds__(NT) k_bcg_p(Dims d, M6<T> m, const T *__restrict__ p, const T *__restrict__ r0,
-                                              T *__restrict__ v, const BcgScalars *sc, double *partials)
+                                              T *__restrict__ v, Red R)
 {
-    if (sc->done) return;
+    if (R.sc->done) return;
     COLUMN
     T acc[1] = {T(0)};
     if (in) {
@@ -110,18 +236,18 @@ __global__ void __launch_bounds__(NT) k_bcg_p(Dims d, M6<T> m, const T *__restri
             acc[0] += r0[c] * y;
         }
     }
-    block_partials<1, T>(acc, partials);
+    pass_end<BR_ALPHA, LAST>(acc, R);
 }
 
-template <typename T>
+template <typename T, bool LAST>
 __global__ void __launch_bounds__(NT) k_bcg_s(Dims d, M6<T> m, const T *__restrict__ r, const T *__restrict__ v,
-                                              T *__restrict__ t, const BcgScalars *sc, double *partials)
+                                              T *__restrict__ t, Red R)
 {
-    if (sc->done) return;
+    if (R.sc->done) return;
     COLUMN
     T acc[2] = {T(0), T(0)};
     if (in) {
-        const T alpha = (T)sc->alpha;
+        const T alpha = (T)R.sc->alpha;
         auto S = [&](long long q) { return r[q] - alpha * v[q]; };
         long long c = c0;
         for (int k = k0; k <= k1; ++k, c += d.sz) {
@@ -131,20 +257,19 @@ __global__ void __launch_bounds__(NT) k_bcg_s(Dims d, M6<T> m, const T *__restri
             acc[1] += y * y;
         }
     }
-    block_partials<2, T>(acc, partials);
+    pass_end<BR_OMEGA, LAST>(acc, R);
 }
 
-template <typename T>
+template <typename T, bool LAST>
 __global__ void __launch_bounds__(NT) k_bcg_x(Dims d, T *__restrict__ x, T *__restrict__ r,
                                               const T *__restrict__ r0, const T *__restrict__ p,
-                                              const T *__restrict__ v, const T *__restrict__ t, const BcgScalars *sc,
-                                              double *partials)
+                                              const T *__restrict__ v, const T *__restrict__ t, Red R)
 {
-    if (sc->done) return;
+    if (R.sc->done) return;
     COLUMN
     T acc[2] = {T(0), T(0)};
     if (in) {
-        const T alpha = (T)sc->alpha, omega = (T)sc->omega;
+        const T alpha = (T)R.sc->alpha, omega = (T)R.sc->omega;
         long long c = c0;
         for (int k = k0; k <= k1; ++k, c += d.sz) {
             const T s = r[c] - alpha * v[c];
@@ -155,7 +280,7 @@ __global__ void __launch_bounds__(NT) k_bcg_x(Dims d, T *__restrict__ x, T *__re
             acc[1] += rn * rn;
         }
     }
-    block_partials<2, T>(acc, partials);
+    pass_end<BR_RHO, LAST>(acc, R);
 }
 
 // x += e (the FP32 correction of a refinement round), pointwise.
@@ -170,9 +295,10 @@ __global__ void __launch_bounds__(NT) k_xadd(Dims d, double *__restrict__ x, con
 // r = b - A x in FP64 (x = NULL stands for x = 0: r = b without the stencil
 // pass); ||r||^2, ||r_T||^2 of the stored vector (r32 when given, summed in
 // FP32) and, with want_bb, ||b||^2.
+template <bool LAST>
 __global__ void __launch_bounds__(NT) k_resid64(Dims d, M6<double> m, const double *__restrict__ b,
                                                 const double *__restrict__ x, double *__restrict__ r64,
-                                                float *__restrict__ r32, int want_bb, double *partials)
+                                                float *__restrict__ r32, Red R)
 {
     COLUMN
     double acc[3] = {0.0, 0.0, 0.0};
@@ -189,96 +315,11 @@ __global__ void __launch_bounds__(NT) k_resid64(Dims d, M6<double> m, const doub
                 rt2 += f * f;
             }
             acc[0] += r * r;
-            if (want_bb) acc[2] += b[c] * b[c];
+            if (R.want_bb) acc[2] += b[c] * b[c];
         }
         acc[1] = r32 ? (double)rt2 : acc[0];
     }
-    block_partials<3, double>(acc, partials);
-}
-
-// Sums q columns of the partials (fixed order: thread-strided, then a tree).
-template <int Q>
-__device__ __forceinline__ void sum_partials(const double *partials, int nb, double (&out)[Q])
-{
-    __shared__ double sh[1024][Q];
-    double a[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) a[q] = 0.0;
-    for (int blk = threadIdx.x; blk < nb; blk += blockDim.x)
-#pragma unroll
-        for (int q = 0; q < Q; ++q) a[q] += partials[4 * (long long)blk + q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) sh[threadIdx.x][q] = a[q];
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-#pragma unroll
-            for (int q = 0; q < Q; ++q) sh[threadIdx.x][q] += sh[threadIdx.x + s][q];
-        __syncthreads();
-    }
-#pragma unroll
-    for (int q = 0; q < Q; ++q) out[q] = sh[0][q];
-}
-
-// after P: alpha = rho / (r0.v)
-__global__ void __launch_bounds__(1024) k_red_alpha(const double *partials, int nb, BcgScalars *sc)
-{
-    if (sc->done) return;
-    double s[1];
-    sum_partials<1>(partials, nb, s);
-    if (threadIdx.x == 0) {
-        const double a = sc->rho / s[0];
-        if (finite_nonzero(s[0]) && isfinite(a)) sc->alpha = a;
-        else { sc->alpha = 0.0; sc->breakdown = 1; sc->done = 1; }
-    }
-}
-
-// after S: omega = (t.s) / (t.t); t.t = 0 means s = 0 (omega = 0 finishes)
-__global__ void __launch_bounds__(1024) k_red_omega(const double *partials, int nb, BcgScalars *sc)
-{
-    if (sc->done) return;
-    double s[2];
-    sum_partials<2>(partials, nb, s);
-    if (threadIdx.x == 0) {
-        const double w = s[1] > 0.0 ? s[0] / s[1] : 0.0;
-        sc->omega = isfinite(w) ? w : 0.0;
-    }
-}
-
-// after X: beta = (rho_new / rho) (alpha / omega), rho = rho_new, rr, and
-// the stopping test
-__global__ void __launch_bounds__(1024) k_red_rho(const double *partials, int nb, BcgScalars *sc)
-{
-    if (sc->done) return;
-    double s[2];
-    sum_partials<2>(partials, nb, s);
-    if (threadIdx.x == 0) {
-        sc->rr = s[1];
-        sc->iters += 1;
-        const double b = (s[0] / sc->rho) * (sc->alpha / sc->omega);
-        if (finite_nonzero(s[0]) && sc->omega != 0.0 && isfinite(b)) sc->beta = b;
-        else { sc->beta = 0.0; sc->breakdown = 1; sc->done = 1; }
-        sc->rho = s[0];
-        if (!(s[1] > sc->target)) sc->done = 1;   // converged (or NaN: the host checks)
-    }
-}
-
-// after a residual: a fresh start (p = r on the next P)
-__global__ void __launch_bounds__(1024) k_red_resid(const double *partials, int nb, BcgScalars *sc, int want_bb)
-{
-    double s[3];
-    sum_partials<3>(partials, nb, s);
-    if (threadIdx.x == 0) {
-        sc->rr = s[0];
-        sc->rho = s[1];
-        if (want_bb) sc->bb = s[2];
-        sc->alpha = 1.0;
-        sc->omega = 1.0;
-        sc->beta = 0.0;
-        sc->breakdown = 0;
-        sc->done = 0;
-        sc->iters = 0;
-    }
+    pass_end<BR_RESID, LAST>(acc, R);
 }
 
 __global__ void k_set_target(BcgScalars *sc, double target)
@@ -308,7 +349,7 @@ dim3 solver_block() { return dim3(32, 4, 1); }
 dim3 solver_grid(const Dims &d) { return dim3((d.I + 31) / 32, (d.J + 3) / 4, (d.K + d.kz - 1) / d.kz); }
 
 template <typename T>
-void bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first, Reduce &R,
+int bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first, Reduce &R,
                    BcgScalars *sc, cudaStream_t st, cudaEvent_t *ev)
 {
     const dim3 g = solver_grid(d), b = solver_block();
@@ -316,25 +357,35 @@ void bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first
     T *p = V.p, *v = V.v;
     if (ev) cudaEventRecord(ev[0], st);
     k_bcg_u<T><<<g, b, 0, st>>>(d, V.r, p, v, sc, first ? 1 : 0);
+    const Red red{R.partials, R.finished, sc, 0};
+    const bool last = R.nblocks <= LAST_MAX, last_x = R.nblocks <= LAST_MAX_X;
+    auto *kp = last ? k_bcg_p<T, true> : k_bcg_p<T, false>;
+    auto *ks = last ? k_bcg_s<T, true> : k_bcg_s<T, false>;
+    auto *kx = last_x ? k_bcg_x<T, true> : k_bcg_x<T, false>;
     if (ev) cudaEventRecord(ev[1], st);
-    k_bcg_p<T><<<g, b, 0, st>>>(d, M, p, V.r0, v, sc, R.partials);
+    kp<<<g, b, 0, st>>>(d, M, p, V.r0, v, red);
     if (ev) cudaEventRecord(ev[2], st);
-    k_red_alpha<<<1, 1024, 0, st>>>(R.partials, R.nblocks, sc);
+    if (!last) k_red<BR_ALPHA><<<1, NT, 0, st>>>(red, R.nblocks);
     if (ev) cudaEventRecord(ev[3], st);
-    k_bcg_s<T><<<g, b, 0, st>>>(d, M, V.r, v, V.t, sc, R.partials);
+    ks<<<g, b, 0, st>>>(d, M, V.r, v, V.t, red);
     if (ev) cudaEventRecord(ev[4], st);
-    k_red_omega<<<1, 1024, 0, st>>>(R.partials, R.nblocks, sc);
+    if (!last) k_red<BR_OMEGA><<<1, NT, 0, st>>>(red, R.nblocks);
     if (ev) cudaEventRecord(ev[5], st);
-    k_bcg_x<T><<<g, b, 0, st>>>(d, V.x, V.r, V.r0, p, v, V.t, sc, R.partials);
+    kx<<<g, b, 0, st>>>(d, V.x, V.r, V.r0, p, v, V.t, red);
     if (ev) cudaEventRecord(ev[6], st);
-    k_red_rho<<<1, 1024, 0, st>>>(R.partials, R.nblocks, sc);
+    if (!last_x) k_red<BR_RHO><<<1, NT, 0, st>>>(red, R.nblocks);
+    return 4 + (last ? 0 : 2) + (last_x ? 0 : 1);
 }
 
-void resid64(const Dims &d, const double *const m[6], const double *b, const double *x, double *r64, float *r32,
-             bool want_bb, Reduce &R, BcgScalars *sc, cudaStream_t st)
+int resid64(const Dims &d, const double *const m[6], const double *b, const double *x, double *r64, float *r32,
+            bool want_bb, Reduce &R, BcgScalars *sc, cudaStream_t st)
 {
-    k_resid64<<<solver_grid(d), solver_block(), 0, st>>>(d, m6(m), b, x, r64, r32, want_bb ? 1 : 0, R.partials);
-    k_red_resid<<<1, 1024, 0, st>>>(R.partials, R.nblocks, sc, want_bb ? 1 : 0);
+    const Red red{R.partials, R.finished, sc, want_bb ? 1 : 0};
+    const bool last = R.nblocks <= LAST_MAX_X;
+    auto *k = last ? k_resid64<true> : k_resid64<false>;
+    k<<<solver_grid(d), solver_block(), 0, st>>>(d, m6(m), b, x, r64, r32, red);
+    if (!last) k_red<BR_RESID><<<1, NT, 0, st>>>(red, R.nblocks);
+    return last ? 1 : 2;
 }
 
 void set_target(BcgScalars *sc, double target, cudaStream_t st)
@@ -347,9 +398,9 @@ void xadd(const Dims &d, double *x, const float *e, cudaStream_t st)
     k_xadd<<<solver_grid(d), solver_block(), 0, st>>>(d, x, e);
 }
 
-template void bcg_iteration<double>(const Dims &, const double *const[6], BcgVecs<double> &, bool, Reduce &,
+template int bcg_iteration<double>(const Dims &, const double *const[6], BcgVecs<double> &, bool, Reduce &,
                                     BcgScalars *, cudaStream_t, cudaEvent_t *);
-template void bcg_iteration<float>(const Dims &, const float *const[6], BcgVecs<float> &, bool, Reduce &,
+template int bcg_iteration<float>(const Dims &, const float *const[6], BcgVecs<float> &, bool, Reduce &,
                                    BcgScalars *, cudaStream_t, cudaEvent_t *);
 
 }  // namespace pred

@@ -182,10 +182,9 @@ int run_batches(scf_mom_ctx *ctx, const scf_mom_opts &o, const T *const m[6], Bc
     while (done_its < cap) {
         const int nb = std::min(batch, cap - done_its);
         for (int q = 0; q < nb; ++q)
-            bcg_iteration<T>(d, m, V, first && q == 0, ctx->R, ctx->sc, ctx->st,
-                             o.kernel_timing ? ctx->kev : nullptr);
+            out.launches += bcg_iteration<T>(d, m, V, first && q == 0, ctx->R, ctx->sc, ctx->st,
+                                             o.kernel_timing ? ctx->kev : nullptr);
         first = false;
-        out.launches += 7 * nb;
         if ((rc = read_scalars(ctx)) != SCF_OK) return done_its;
         done_its = ctx->sc_host->iters;
         if (o.kernel_timing) add_kernel_times(ctx, out);
@@ -209,9 +208,8 @@ int solve_fp64(scf_mom_ctx *ctx, const scf_mom_opts &o, SolveOut &out)
     const double *const *m = ctx->m;
     const size_t bytes = (size_t)d.ng * sizeof(double);
     MK(cudaMemsetAsync(V.x, 0, bytes, ctx->st));
-    resid64(d, m, ctx->b, nullptr, V.r, nullptr, true, ctx->R, ctx->sc, ctx->st);
+    out.launches += resid64(d, m, ctx->b, nullptr, V.r, nullptr, true, ctx->R, ctx->sc, ctx->st);
     MK(cudaMemcpyAsync(V.r0, V.r, bytes, cudaMemcpyDeviceToDevice, ctx->st));
-    out.launches += 2;
     RS();
     const double bb = ctx->sc_host->bb, target = o.rel_tol * o.rel_tol * bb;
     out.x = V.x;
@@ -231,8 +229,7 @@ int solve_fp64(scf_mom_ctx *ctx, const scf_mom_opts &o, SolveOut &out)
         if (!ctx->sc_host->done) break;   // iteration cap
         // converged by the recursive residual, or broken down: check the
         // true residual and restart from it if needed
-        resid64(d, m, ctx->b, V.x, V.r, nullptr, false, ctx->R, ctx->sc, ctx->st);
-        out.launches += 2;
+        out.launches += resid64(d, m, ctx->b, V.x, V.r, nullptr, false, ctx->R, ctx->sc, ctx->st);
         RS();
         rr = ctx->sc_host->rr;
         if (!std::isfinite(rr)) {
@@ -263,8 +260,7 @@ int solve_mixed(scf_mom_ctx *ctx, const scf_mom_opts &o, SolveOut &out)
     double *xa = ctx->V64.x;
     const size_t bytes32 = (size_t)d.ng * sizeof(float);
     MK(cudaMemsetAsync(xa, 0, (size_t)d.ng * sizeof(double), ctx->st));
-    resid64(d, m, ctx->b, nullptr, nullptr, V.r, true, ctx->R, ctx->sc, ctx->st);
-    out.launches += 2;
+    out.launches += resid64(d, m, ctx->b, nullptr, nullptr, V.r, true, ctx->R, ctx->sc, ctx->st);
     RS();
     const double bb = ctx->sc_host->bb, target = o.rel_tol * o.rel_tol * bb;
     double rr = ctx->sc_host->rr;
@@ -286,8 +282,7 @@ int solve_mixed(scf_mom_ctx *ctx, const scf_mom_opts &o, SolveOut &out)
         if (rc != SCF_OK) return rc;
         if (its == 0) break;   // breakdown at the round's first iteration: x unchanged, no progress possible
         xadd(d, xa, V.x, ctx->st);
-        resid64(d, m, ctx->b, xa, nullptr, V.r, false, ctx->R, ctx->sc, ctx->st);
-        out.launches += 3;
+        out.launches += 1 + resid64(d, m, ctx->b, xa, nullptr, V.r, false, ctx->R, ctx->sc, ctx->st);
         ++out.rounds;
         RS();
         rr = ctx->sc_host->rr;
@@ -373,6 +368,7 @@ extern "C" int scf_mom_create(scf_mom_ctx **out, int32_t imax, int32_t jmax, int
     TRY(ctx->V32.p, ng) TRY(ctx->V32.v, ng)
     ctx->R.nblocks = (int)(solver_grid(d).x * solver_grid(d).y * solver_grid(d).z);
     TRY(ctx->R.partials, 4 * (size_t)ctx->R.nblocks)
+    TRY(ctx->R.finished, 1)
     TRY(ctx->sc, 1)
     TRY(ctx->counts, 2)
 #undef TRY

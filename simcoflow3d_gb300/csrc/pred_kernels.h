@@ -77,17 +77,19 @@ struct BcgVecs {
 };
 struct Reduce {
     double *partials;     // 4 per block
+    unsigned *finished;   // blocks of the running pass that have (0 between passes)
     int nblocks;
 };
 // ev (optional, 7 events): recorded around the four passes U, P, S, X.
+// Returns the launches, as resid64 does.
 template <typename T>
-void bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first, Reduce &R, BcgScalars *sc,
+int bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first, Reduce &R, BcgScalars *sc,
                    cudaStream_t st, cudaEvent_t *ev = nullptr);
 // r = b - A x with the FP64 couplings (x = NULL: x = 0, r = b) into r64
 // and/or r32 (rounded); ||r||^2 into sc->rr, the stored vector's norm^2 into
 // sc->rho, and with want_bb ||b||^2 into sc->bb; resets alpha, omega, beta.
-void resid64(const Dims &d, const double *const m[6], const double *b, const double *x, double *r64, float *r32,
-             bool want_bb, Reduce &R, BcgScalars *sc, cudaStream_t st);
+int resid64(const Dims &d, const double *const m[6], const double *b, const double *x, double *r64, float *r32,
+            bool want_bb, Reduce &R, BcgScalars *sc, cudaStream_t st);
 // x += e (FP32 correction), pointwise.
 void xadd(const Dims &d, double *x, const float *e, cudaStream_t st);
 // sc->target = target; clears done and iters.

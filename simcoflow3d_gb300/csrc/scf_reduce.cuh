@@ -61,8 +61,9 @@ __device__ __forceinline__ void red_tail(const RedOut &o, int nb)
             }
 #pragma unroll
         for (int q = 0; q < Q; ++q)
+            if (m + 256 * (t >> 5) < nb)   // (an FP64 addition of nothing would still hold the pipe)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) a[q][j] += p[q][j];
+                for (int j = 0; j < 8; ++j) a[q][j] += p[q][j];
     }
 #pragma unroll
     for (int d = 4; d > 0; d >>= 1)
