@@ -4,6 +4,7 @@
 // order, so Dp is bit-identical to the Fortran and the rows differ from
 // HYPRE's only by the Jacobi scaling.
 #include "pred_kernels.h"
+#include "scf_common.cuh"
 
 namespace pred {
 
@@ -26,9 +27,69 @@ enum { KDFE, KDFW, KDFN, KDFS, KDFT, KDFB, KEE, KEW, KEN, KES, KET, KEB, KETAE, 
 enum { MW, MS, MB, ME, MN, MT, MINV, MDP, MG, MCW, MCE, MCS, MCN, MCB, MCT, NMEMO };
 constexpr int ASM_NT = 128;   // threads of an assembly block; the stride of the shared-memory slots
 
+__device__ __forceinline__ int exp_bits(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+__device__ __forceinline__ bool zero_bits(double x) { return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0; }
+// sign of x xor y's, on 0
+__device__ __forceinline__ double signed_zero(int sign_hi) { return __hiloint2double(sign_hi & (int)0x80000000u, 0); }
+
+// Divisions and the like that few rows need stay out of line: inline, they
+// would be executed under a predicate, and an FP64 warp instruction holds its
+// pipe for 16 cycles either way.
+__device__ __noinline__ double div_full(double x, double d) { return x / d; }
+
+// x / d, correctly rounded, r = 1/d rounded: Markstein's division (IBM J. Res.
+// Dev. 34, 1990).  One remainder step makes the quotient faithful and a second
+// one, whose remainder is exact, rounds it correctly; five operations against
+// about ten.  Outside the exponents where the remainders are exact, the division.
+__device__ __forceinline__ double quotient(double x, double d, double r)
+{
+    const int e = exp_bits(x), ed = exp_bits(d);
+    if (ed > 723 && ed < 1323 && e > 423 && e < 1623) {
+        double q = __dmul_rn(x, r);
+        q = __fma_rn(__fma_rn(-d, q, x), r, q);
+        return __fma_rn(__fma_rn(-d, q, x), r, q);
+    }
+    if (zero_bits(x) && ed > 0 && ed < 0x7ff) return signed_zero(__double2hiint(x) ^ __double2hiint(d));
+    return div_full(x, d);
+}
+
+// rfr2 vof dx dy dz G3 / g; with G3 = 0 (gravity normal to the component) and
+// moderate factors a zero whose sign is theirs.
+__device__ __noinline__ double gravity_full(double vof, double dx, double dy, double dz, const MomParams &o)
+{
+    return o.rfr2 * vof * dx * dy * dz * o.g3 / o.g;
+}
+__device__ __forceinline__ double gravity(double vof, double dx, double dy, double dz, const MomParams &o)
+{
+    auto mid = [](double x) { const int e = exp_bits(x); return e > 823 && e < 1223; };
+    if (zero_bits(o.g3) && mid(dx) && mid(dy) && mid(dz) && mid(o.rfr2) && mid(o.g) && exp_bits(vof) < 1223)
+        return signed_zero(__double2hiint(vof) ^ __double2hiint(dx) ^ __double2hiint(dy) ^ __double2hiint(dz) ^
+                           __double2hiint(o.rfr2) ^ __double2hiint(o.g3) ^ __double2hiint(o.g));
+    return gravity_full(vof, dx, dy, dz, o);
+}
+
+// U dv dx dy dz / dt (no division of a zero dv's product, as the reference's
+// quotient is that zero).  Away from the interface and moving solids dv is 0.
+__device__ __noinline__ double unsteady_full(double U, double dv, double dx, double dy, double dz, double dt, double rdt)
+{
+    return dv == 0.0 ? U * dv * dx * dy * dz : quotient(U * dv * dx * dy * dz, dt, rdt);
+}
+__device__ __forceinline__ double unsteady(double U, double dv, double dx, double dy, double dz, double dt, double rdt)
+{
+    auto mid = [](double x) { const int e = exp_bits(x); return e > 823 && e < 1223; };
+    if (zero_bits(dv) && mid(dx) && mid(dy) && mid(dz) && exp_bits(U) < 0x7ff)
+        return signed_zero(__double2hiint(U) ^ __double2hiint(dv) ^ __double2hiint(dx) ^ __double2hiint(dy) ^
+                           __double2hiint(dz));
+    return unsteady_full(U, dv, dx, dy, dz, dt, rdt);
+}
+
 // SetMatrix for one row (PredictUVW.f90:904-1040) with the reference's
 // operations in its order; called only when the key differs from the
-// previous row's (never inlined, so none of it runs speculatively).
+// previous row's (never inlined, so none of it runs speculatively).  PLAIN:
+// the six cut-face terms are +0 and the weights in [0, 1], so with rho > 0 every
+// convective term is +0 (most rows: only cut cells and their neighbours have
+// others), which leaves about 75 of 150 FP64 operations.
+template <bool PLAIN>
 __device__ __noinline__ void mom_row(const double *k, const MomParams &o, int comp, int ib, double *mo)
 {
     const int iu = comp == 1, iv = comp == 2, iw = comp == 3;
@@ -39,75 +100,78 @@ __device__ __noinline__ void mom_row(const double *k, const MomParams &o, int co
     const double omb = 1.0 - o.beta_vis;
     const double vof = K(KVOF), vofl = K(KVOFL);
     const double rho = vofl * o.rho_w + (vof - vofl) * o.rho_a;
-    // x / rho without a division where that is exact: rho a power of two
-    // (the liquid's 1.0 with the water reference density) gives the same
-    // rounding as x * (1/rho) (the two real quotients are equal), and
-    // x = +-0 over a finite non-zero rho gives the signed zero.
-    const long long rb = __double_as_longlong(rho);
-    const int rexp = (int)((rb >> 52) & 0x7ff);
-    const bool pow2 = (rb & 0xfffffffffffffLL) == 0 && rexp > 0 && rexp < 0x7fe;
-    const bool finite_nz = rexp > 0 && rexp < 0x7ff;
-    const double rinv = pow2 ? 1.0 / rho : 0.0;
-    auto q = [&](double x) {
-        if (pow2) return x * rinv;
-        if (x == 0.0 && finite_nz) return rho > 0.0 ? x : -x;
-        return x / rho;
-    };
+    // x / rho: for rho a power of two (the liquid's 1.0 with the water
+    // reference density) x * (1/rho) is the same quotient, rounded the same,
+    // and 1/rho is rho with its exponent reflected; otherwise one division
+    // and quotient().
+    const int rexp = exp_bits(rho);
+    if constexpr (PLAIN)
+        if (__double2hiint(rho) < 0x100000 || rexp == 0x7ff) {
+            mom_row<false>(k, o, comp, ib, mo);
+            return;
+        }
+    const bool pow2 = ((__double2hiint(rho) & 0xfffff) | __double2loint(rho)) == 0 && rexp > 0 && rexp < 0x7fe;
+    const double rinv = pow2 ? __hiloint2double((__double2hiint(rho) & (int)0x80000000u) | (0x7fe - rexp) << 20, 0)
+                             : div_full(1.0, rho);
+    auto q = [&](double x) { return pow2 ? x * rinv : quotient(x, rho, rinv); };
     double Dfe = q(omb * K(KDFE)), Dfw = q(omb * K(KDFW));
     double Dfn = q(omb * K(KDFN)), Dfs = q(omb * K(KDFS));
     double Dft = q(omb * K(KDFT)), Dfb = q(omb * K(KDFB));
-    const double ee = K(KEE), ew = K(KEW), en = K(KEN), es = K(KES), et = K(KET), eb = K(KEB);
-    const double etaE = K(KETAE), etaW = K(KETAW), etaN = K(KETAN), etaS = K(KETAS), etaT = K(KETAT),
-                 etaB = K(KETAB);
-    double Fep = q(ee * (1.0 - etaE)), Fem = q(ee * etaE);
-    double Fwp = q(ew * etaW), Fwm = q(ew * (1.0 - etaW));
-    double Fnp = q(en * (1.0 - etaN)), Fnm = q(en * etaN);
-    double Fsp = q(es * etaS), Fsm = q(es * (1.0 - etaS));
-    double Ftp = q(et * (1.0 - etaT)), Ftm = q(et * etaT);
-    double Fbp = q(eb * etaB), Fbm = q(eb * (1.0 - etaB));
+    double Fep = 0.0, Fem = 0.0, Fwp = 0.0, Fwm = 0.0, Fnp = 0.0, Fnm = 0.0, Fsp = 0.0, Fsm = 0.0, Ftp = 0.0, Ftm = 0.0,
+           Fbp = 0.0, Fbm = 0.0;
+    if (!PLAIN) {
+        const double ee = K(KEE), ew = K(KEW), en = K(KEN), es = K(KES), et = K(KET), eb = K(KEB);
+        const double etaE = K(KETAE), etaW = K(KETAW), etaN = K(KETAN), etaS = K(KETAS), etaT = K(KETAT),
+                     etaB = K(KETAB);
+        Fep = q(ee * (1.0 - etaE)); Fem = q(ee * etaE);
+        Fwp = q(ew * etaW); Fwm = q(ew * (1.0 - etaW));
+        Fnp = q(en * (1.0 - etaN)); Fnm = q(en * etaN);
+        Fsp = q(es * etaS); Fsm = q(es * (1.0 - etaS));
+        Ftp = q(et * (1.0 - etaT)); Ftm = q(et * etaT);
+        Fbp = q(eb * etaB); Fbm = q(eb * (1.0 - etaB));
+    }
     // boundary faces (939-1009); ib bits: i = 1, i = ie, j = 1, j = je,
     // k = 1, k = ke; flags 1 = Neumann
     const int *fl = o.flags;
     if (ib & 1) {
         if (fl[0] == 1) { Dfw = 0.0; Fwp = 0.0; Fwm = 0.0; }
-        else { Dfw = Dfw * CoefEW; Fwp = Fwp * CoefEW; Fwm = Fwm * CoefEW; }
+        else { Dfw = Dfw * CoefEW; if (!PLAIN) { Fwp = Fwp * CoefEW; Fwm = Fwm * CoefEW; } }
     }
     if (ib & 2) {
         if (fl[1] == 1) { Dfe = 0.0; Fep = 0.0; Fem = 0.0; }
-        else { Dfe = Dfe * CoefEW; Fep = Fep * CoefEW; Fem = Fem * CoefEW; }
+        else { Dfe = Dfe * CoefEW; if (!PLAIN) { Fep = Fep * CoefEW; Fem = Fem * CoefEW; } }
     }
     if (ib & 4) {
         if (fl[2] == 1) { Dfs = 0.0; Fsp = 0.0; Fsm = 0.0; }
-        else { Dfs = Dfs * CoefNS; Fsp = Fsp * CoefNS; Fsm = Fsm * CoefNS; }
+        else { Dfs = Dfs * CoefNS; if (!PLAIN) { Fsp = Fsp * CoefNS; Fsm = Fsm * CoefNS; } }
     }
     if (ib & 8) {
         if (fl[3] == 1) { Dfn = 0.0; Fnp = 0.0; Fnm = 0.0; }
-        else { Dfn = Dfn * CoefNS; Fnp = Fnp * CoefNS; Fnm = Fnm * CoefNS; }
+        else { Dfn = Dfn * CoefNS; if (!PLAIN) { Fnp = Fnp * CoefNS; Fnm = Fnm * CoefNS; } }
     }
     if (ib & 16) {
         if (fl[4] == 1) { Dfb = 0.0; Fbp = 0.0; Fbm = 0.0; }
-        else { Dfb = Dfb * CoefTB; Fbp = Fbp * CoefTB; Fbm = Fbm * CoefTB; }
+        else { Dfb = Dfb * CoefTB; if (!PLAIN) { Fbp = Fbp * CoefTB; Fbm = Fbm * CoefTB; } }
     }
     if (ib & 32) {
         if (fl[5] == 1) { Dft = 0.0; Ftp = 0.0; Ftm = 0.0; }
-        else { Dft = Dft * CoefTB; Ftp = Ftp * CoefTB; Ftm = Ftm * CoefTB; }
+        else { Dft = Dft * CoefTB; if (!PLAIN) { Ftp = Ftp * CoefTB; Ftm = Ftm * CoefTB; } }
     }
     double aE = Dfe, aW = Dfw, aN = Dfn, aS = Dfs, aT = Dft, aB = Dfb;
     auto M = [&](int r, double val) { mo[r * ASM_NT] = val; };
     M(MCW, aW); M(MCE, aE); M(MCS, aS); M(MCN, aN); M(MCB, aB); M(MCT, aT);   // CWE/CSN/CBT
     const double dx = K(KDX), dy = K(KDY), dz = K(KDZ);
-    double aP = vof * dx * dy * dz / o.dt + aE + aW + aN + aS + aT + aB + K(KFRIC);
-    aP = aP + Fep - Fwp + Fnp - Fsp + Ftp - Fbp;
-    aE = aE - Fem;
+    const double dV = vof * dx * dy * dz;
+    double aP = quotient(dV, o.dt, o.rdt) + aE + aW + aN + aS + aT + aB + K(KFRIC);
+    // (+0 changes nothing but a zero's sign, and -0 not even that)
+    aP = PLAIN ? aP + 0.0 : aP + Fep - Fwp + Fnp - Fsp + Ftp - Fbp;
+    if (!PLAIN) { aE = aE - Fem; aN = aN - Fnm; aT = aT - Ftm; }
     aW = aW + Fwm;
-    aN = aN - Fnm;
     aS = aS + Fsm;
-    aT = aT - Ftm;
     aB = aB + Fbm;
     const double dp0 = 1.0 / (aP - aE - aW - aN - aS - aT - aB);
-    M(MDP, vof * dx * dy * dz * dp0);
-    const double G3 = o.gx * (double)iu + o.gy * (double)iv + o.gz * (double)iw;
-    M(MG, o.rfr2 * vof * dx * dy * dz * G3 / o.g);   // rfr2 = 1.d0/Fr**2.d0, formed once
+    M(MDP, dV * dp0);
+    M(MG, gravity(vof, dx, dy, dz, o));   // rfr2 = 1.d0/Fr**2.d0, formed once
     const double inv = 1.0 / aP;
     M(MINV, inv);
     M(MW, aW * inv); M(MS, aS * inv); M(MB, aB * inv);
@@ -123,7 +187,11 @@ __device__ __noinline__ void mom_row(const double *k, const MomParams &o, int co
 // rows away from the interface and the solid) reuse the previous row's
 // memo, so the FP64 divisions run only where the inputs change.  The key
 // being compared is in registers; the previous key and the memo live in the
-// thread's shared-memory slots, which a miss hands to mom_row.
+// thread's shared-memory slots, which a miss hands to mom_row.  On grids whose
+// spacings differ in their last bits most rows miss, and the FP64 pipe bounds
+// the kernel (77% busy): 128 x 112 x 96, per component, 305 us with a division
+// per quotient and every row's convective terms formed, 220 without
+// (67 x 53 x 75: 127 and 92).
 __global__ void __launch_bounds__(ASM_NT, 4) k_mom_assemble(MomDev in, MomParams o, int comp, Dims d, MomSys S,
                                                          int want32, int kz)
 {
@@ -179,12 +247,20 @@ __global__ void __launch_bounds__(ASM_NT, 4) k_mom_assemble(MomDev in, MomParams
 #pragma unroll
                     for (int q = 0; q < NKEY; ++q) sprev[q][tid] = v[q];
                     skb[tid] = kb;
-                    mom_row(&sprev[0][tid], o, comp, kb, &smemo[0][tid]);
+                    unsigned cut = 0, weights = 0;
+#pragma unroll
+                    for (int q = KEE; q <= KEB; ++q) cut |= __double2hiint(v[q]) | __double2loint(v[q]);
+#pragma unroll
+                    for (int q = KETAE; q <= KETAB; ++q)   // +0 <= eta <= 1 by its bits
+                        weights |= (unsigned long long)__double_as_longlong(v[q]) > 0x3ff0000000000000ull;
+                    if ((cut | weights) == 0u)
+                        mom_row<true>(&sprev[0][tid], o, comp, kb, &smemo[0][tid]);
+                    else mom_row<false>(&sprev[0][tid], o, comp, kb, &smemo[0][tid]);
 #pragma unroll
                     for (int q = 0; q < 6; ++q) {
                         mm[q] = smemo[MW + q][tid];
                         mcb[q] = smemo[MCW + q][tid];
-                        mf[q] = (float)mm[q];
+                        mf[q] = scf_to_f32(mm[q]);
                     }
                     minv = smemo[MINV][tid]; mdp = smemo[MDP][tid]; mg = smemo[MG][tid];
                     have = true;
@@ -195,8 +271,8 @@ __global__ void __launch_bounds__(ASM_NT, 4) k_mom_assemble(MomDev in, MomParams
                 const double vof = v[KVOF], dx = v[KDX], dy = v[KDY], dz = v[KDZ];
                 const double U = in.tvar[c] + 0.0;
                 const double dv = vof - in.vof_old[c];
-                const double t1 = U * vof * dx * dy * dz / o.dt;
-                const double t2 = dv == 0.0 ? U * dv * dx * dy * dz : U * dv * dx * dy * dz / o.dt;
+                const double t1 = quotient(U * vof * dx * dy * dz, o.dt, o.rdt);
+                const double t2 = unsteady(U, dv, dx, dy, dz, o.dt, o.rdt);
                 double rhs = t1 - t2 + mg;
                 rhs = rhs - in.flux_div[n];
                 if (kb & 1) rhs = rhs + mcb[0] * in.bc[0][(j - 1) + (long long)d.J * (k - 1)];

@@ -27,6 +27,8 @@ struct MomDev {
 struct MomParams {
     double dt, rho_a, rho_w, fr, gx, gy, gz, g, beta_vis;
     double rfr2;    // 1 / (fr * fr), the same IEEE quotient the rows would form
+    double rdt;     // 1 / dt, for quotient()
+    double g3;      // the component's gx (u), gy (v), gz (w) sum as the rows form it
     int flags[6];   // the component's BC%flag (1 = Neumann)
 };
 
