@@ -86,7 +86,11 @@ struct Reducer {
     double *scal;        // ScfScalar slots
     int max_blocks;
     unsigned *done;      // blocks of the running launch that have finished (0 between launches)
+    double *mail;        // pinned host memory: the sums that the host waits for, MAIL_STRIDE apart
 };
+// (r, r) of the CG update, of a residual, and (b, b).
+enum Mail { MAIL_RR, MAIL_RESIDUAL, MAIL_BB, MAIL_NUM };
+constexpr int MAIL_STRIDE = 16;   // a cache line each
 
 // Coarsening and the coarsest dense inverse.
 template <typename T>

@@ -17,14 +17,14 @@
 #include "scf_kernels.h"
 
 struct RedOut {
-    double *part, *scal;
+    double *part, *scal, *mail;
     unsigned *done;   // blocks that have finished; 0 between launches
     int n0;           // offset of the second sum's partials
     int singular;
 };
 inline RedOut red_out(const Reducer &R, bool singular = false)
 {
-    return RedOut{R.partials, R.scal, R.done, R.max_blocks, singular ? 1 : 0};
+    return RedOut{R.partials, R.scal, R.mail, R.done, R.max_blocks, singular ? 1 : 0};
 }
 inline bool red_last(unsigned blocks) { return blocks <= MARCH_WAVE; }
 
@@ -88,6 +88,12 @@ __device__ __forceinline__ void red_tail(const RedOut &o, int nb)
 #pragma unroll
     for (int q = 0; q < Q; ++q) v[q] = __shfl_sync(0xffffffffu, v[q], 0);
     if (t > 1) return;
+    // to the waiting host without a copy of its own (scf_api.cu, await_mail)
+    constexpr int mail = KIND == RK_RR ? MAIL_RR : KIND == RK_RESIDUAL ? MAIL_RESIDUAL : KIND == RK_BB ? MAIL_BB : -1;
+    if (mail >= 0 && t == 0) {
+        *(volatile double *)(o.mail + (mail >= 0 ? mail : 0) * MAIL_STRIDE) = v[0];
+        __threadfence_system();
+    }
     // lanes 0 and 1 form the two quotients of a kind in one division
     if constexpr (KIND == RK_ALPHA) {
         // alpha = (r, z) / (p, q); for an all-Neumann system also the mean of
