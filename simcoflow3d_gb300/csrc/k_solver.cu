@@ -344,20 +344,61 @@ __global__ void __launch_bounds__(256) k_cheb_first(LevelView<T> L, const T *__r
     if (in) x[c] = coef * dinv_at(L, c) * b[c];
 }
 
-template <typename T>
+// M cells of one (i, j) column per thread, all loads first.
+template <typename T, int M>
 __global__ void __launch_bounds__(256) k_cheb_step(LevelView<T> L, const T *__restrict__ b,
                                                    const T *__restrict__ xin, const T *dprev,
                                                    T *__restrict__ xout, T *dout, T c1, T c2)
 {
-    INTERIOR_IJK(L);
-    if (!in) return;
-    const int sy = L.sy, sz = L.sz;
-    const T x0 = xin[c];
-    const T dn = cheb_update(b[c], L.diag[c], dinv_at(L, c), x0, xin[c + 1], xin[c - 1], xin[c + sy], xin[c - sy],
-                             xin[c + sz], xin[c - sz], L.cE[c], L.cE[c - 1], L.cN[c], L.cN[c - sy], L.cT[c],
-                             L.cT[c - sz], dprev[c], c1, c2);
-    xout[c] = fx_add(x0, dn);
-    if (dout) dout[c] = dn;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+    const int k = (blockIdx.z * blockDim.z + threadIdx.z) * M + 1;
+    if (i > L.n0 || j > L.n1 || k > L.n2) return;
+    const int sy = L.sy, sz = L.sz, c = i + sy * j + sz * k;
+    T x[M + 2], ct[M + 1], xe[M], xw[M], xn[M], xs[M], ce[M], cw[M], cn[M], cs[M], bb[M], dg[M], di[M], dp[M];
+    x[0] = xin[c - sz];
+    x[1] = xin[c];
+    ct[0] = L.cT[c - sz];
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const int q = c + sz * (M == 1 ? 0 : min(m, L.n2 - k));
+        x[m + 2] = xin[q + sz];
+        ct[m + 1] = L.cT[q];
+        xe[m] = xin[q + 1]; xw[m] = xin[q - 1]; xn[m] = xin[q + sy]; xs[m] = xin[q - sy];
+        ce[m] = L.cE[q]; cw[m] = L.cE[q - 1]; cn[m] = L.cN[q]; cs[m] = L.cN[q - sy];
+        bb[m] = b[q]; dg[m] = L.diag[q]; dp[m] = dprev[q];
+        di[m] = sizeof(T) == 8 ? L.dinv[q] : T(0);
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        if (M > 1 && k + m > L.n2) break;
+        const T inv = sizeof(T) == 8 ? di[m] : (T)jacobi_inv((float)dg[m]);
+        const T dn = cheb_update(bb[m], dg[m], inv, x[m + 1], xe[m], xw[m], xn[m], xs[m], x[m + 2], x[m], ce[m], cw[m],
+                                 cn[m], cs[m], ct[m + 1], ct[m], dp[m], c1, c2);
+        xout[c + sz * m] = fx_add(x[m + 1], dn);
+        if (dout) dout[c + sz * m] = dn;
+    }
+}
+
+// Cells per thread: FP32 levels of at least 2^18 cells are bound by the
+// latency and the number of their loads (18 per cell one at a time; the cells
+// of a column share five of them), us per step with 1 / 2 / 4 cells per
+// thread: 147x93x121 10.4 / 9.4 / 9.2, 128^3 11.9 / 10.9 / 10.6, 64^3
+// 3.72 / 3.64 / 3.62.  Smaller levels lack blocks (32^3 2.69 / 2.77 / 2.97), and
+// FP64 levels are bound by the FP64 pipe (128^3 48.6 / 49.0 / 53.7).
+template <typename T>
+void cheb_step(const LevelView<T> &L, const T *b, const T *xin, const T *dprev, T *xout, T *dout, T c1, T c2,
+               cudaStream_t st)
+{
+    Launch3 l = launch_interior(L.n0, L.n1, L.n2);
+    if constexpr (sizeof(T) == 4) {
+        if ((long long)L.n0 * L.n1 * L.n2 >= 1ll << 18) {
+            l.grid.z = (L.n2 + 7) / 8;
+            k_cheb_step<T, 4><<<l.grid, l.block, 0, st>>>(L, b, xin, dprev, xout, dout, c1, c2);
+            return;
+        }
+    }
+    k_cheb_step<T, 1><<<l.grid, l.block, 0, st>>>(L, b, xin, dprev, xout, dout, c1, c2);
 }
 
 // ---------------------------------------------------------------------------
@@ -824,11 +865,9 @@ cudaError_t cheb_pair(const MgLevel<float> &F, const float *xin, const float *dp
     if (ok) ok = pair_smem_attr() == cudaSuccess;
     if (!ok) {
         g_pair_fallback.fetch_add(1);
-        Launch3 lf = launch_interior(F.n0, F.n1, F.n2);
         float *x1 = xout, *x2 = const_cast<float *>(xin);
-        k_cheb_step<float><<<lf.grid, lf.block, 0, st>>>(v, F.b, xin, dprev ? dprev : xin, x1, F.d, (float)c1a,
-                                                         (float)c2a);
-        k_cheb_step<float><<<lf.grid, lf.block, 0, st>>>(v, F.b, x1, F.d, x2, dout, (float)c1b, (float)c2b);
+        cheb_step<float>(v, F.b, xin, dprev ? dprev : xin, x1, F.d, (float)c1a, (float)c2a, st);
+        cheb_step<float>(v, F.b, x1, F.d, x2, dout, (float)c1b, (float)c2b, st);
         return cudaMemcpyAsync(xout, x2, sizeof(float) * (size_t)F.tot, cudaMemcpyDeviceToDevice, st);
     }
     g_pair_tma.fetch_add(1);
@@ -1460,7 +1499,7 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
             const T *dprev = (s == 1) ? xa : F.d;
             T *dout = (s == cc.degree - 1) ? nullptr : F.d;
             const int id = l == 0 ? kt_begin(kt, KC_SMOOTH, st, smooth_bytes<T>(F, s == 1, dout != nullptr)) : -1;
-            k_cheb_step<T><<<lf.grid, lf.block, 0, st>>>(v, F.b, xa, dprev, xb, dout, (T)cc.c1[s], (T)cc.c2[s]);
+            cheb_step<T>(v, F.b, xa, dprev, xb, dout, (T)cc.c1[s], (T)cc.c2[s], st);
             kt_end(kt, id, st);
             *launches += 1;
             T *tmp = xa; xa = xb; xb = tmp;
@@ -1546,8 +1585,7 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
             const int idp = l == 0 ? kt_begin(kt, KC_PROLONG, st, prolong_bytes<T>(F, more)) : -1;
             launch_prolong<T>(F, C, xa, cur[l + 1], st);
             // first post-smoothing step from x: the previous update term is 0
-            k_cheb_step<T><<<lf.grid, lf.block, 0, st>>>(v, F.b, xa, xa, xb, more ? F.d : nullptr, T(0),
-                                                         (T)cc.first);
+            cheb_step<T>(v, F.b, xa, xa, xb, more ? F.d : nullptr, T(0), (T)cc.first, st);
             kt_end(kt, idp, st);
             *launches += 2;
         } else {
@@ -1561,8 +1599,7 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
         for (; s < cc.degree; ++s) {
             const bool last_step = s == cc.degree - 1;
             const int id = l == 0 ? kt_begin(kt, KC_SMOOTH, st, smooth_bytes<T>(F, false, !last_step)) : -1;
-            k_cheb_step<T><<<lf.grid, lf.block, 0, st>>>(v, F.b, xa, F.d, xb, last_step ? nullptr : F.d,
-                                                         (T)cc.c1[s], (T)cc.c2[s]);
+            cheb_step<T>(v, F.b, xa, F.d, xb, last_step ? nullptr : F.d, (T)cc.c1[s], (T)cc.c2[s], st);
             kt_end(kt, id, st);
             *launches += 1;
             T *tmp = xa; xa = xb; xb = tmp;
@@ -1577,9 +1614,8 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
 template <typename T>
 void probe_smooth(MgLevel<T> &F, const ChebCoef &cc, cudaStream_t st)
 {
-    Launch3 lf = launch_interior(F.n0, F.n1, F.n2);
     const int s = cc.degree > 1 ? 1 : 0;
-    k_cheb_step<T><<<lf.grid, lf.block, 0, st>>>(F.view(), F.b, F.x, F.d, F.xb, F.d, (T)cc.c1[s], (T)cc.c2[s]);
+    cheb_step<T>(F.view(), F.b, F.x, F.d, F.xb, F.d, (T)cc.c1[s], (T)cc.c2[s], st);
 }
 
 cudaError_t probe_smooth2(MgLevel<float> &F, const ChebCoef &cc, cudaStream_t st)
