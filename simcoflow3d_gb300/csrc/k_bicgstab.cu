@@ -22,6 +22,7 @@
 // once, so the host enqueues several iterations and reads the scalars once
 // per batch.
 #include "pred_kernels.h"
+#include "scf_launch.cuh"
 
 namespace pred {
 namespace {
@@ -179,6 +180,7 @@ __device__ __forceinline__ void pass_end(A (&v)[red_sums(KIND)], const Red &R)
 template <int KIND>
 __global__ void __launch_bounds__(NT) k_red(Red R, int nb)
 {
+    after_previous();
     if (KIND != BR_RESID && R.sc->done) return;
     red_tail<KIND>(R, nb);
 }
@@ -209,6 +211,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) k_bcg_u(Dims d, const T *__restrict__ r, T *__restrict__ p,
                                               const T *__restrict__ v, const BcgScalars *sc, int first)
 {
+    after_previous();
     if (sc->done) return;
     COLUMN
     if (!in) return;
@@ -224,6 +227,7 @@ template <typename T, bool LAST>
 __global__ void __launch_bounds__(NT) k_bcg_p(Dims d, M6<T> m, const T *__restrict__ p, const T *__restrict__ r0,
                                               T *__restrict__ v, Red R)
 {
+    after_previous();
     if (R.sc->done) return;
     COLUMN
     T acc[1] = {T(0)};
@@ -243,6 +247,7 @@ template <typename T, bool LAST>
 __global__ void __launch_bounds__(NT) k_bcg_s(Dims d, M6<T> m, const T *__restrict__ r, const T *__restrict__ v,
                                               T *__restrict__ t, Red R)
 {
+    after_previous();
     if (R.sc->done) return;
     COLUMN
     T acc[2] = {T(0), T(0)};
@@ -265,6 +270,7 @@ __global__ void __launch_bounds__(NT) k_bcg_x(Dims d, T *__restrict__ x, T *__re
                                               const T *__restrict__ r0, const T *__restrict__ p,
                                               const T *__restrict__ v, const T *__restrict__ t, Red R)
 {
+    after_previous();
     if (R.sc->done) return;
     COLUMN
     T acc[2] = {T(0), T(0)};
@@ -286,6 +292,7 @@ __global__ void __launch_bounds__(NT) k_bcg_x(Dims d, T *__restrict__ x, T *__re
 // x += e (the FP32 correction of a refinement round), pointwise.
 __global__ void __launch_bounds__(NT) k_xadd(Dims d, double *__restrict__ x, const float *__restrict__ e)
 {
+    after_previous();
     COLUMN
     if (!in) return;
     long long c = c0;
@@ -300,6 +307,7 @@ __global__ void __launch_bounds__(NT) k_resid64(Dims d, M6<double> m, const doub
                                                 const double *__restrict__ x, double *__restrict__ r64,
                                                 float *__restrict__ r32, Red R)
 {
+    after_previous();
     COLUMN
     double acc[3] = {0.0, 0.0, 0.0};
     if (in) {
@@ -324,6 +332,7 @@ __global__ void __launch_bounds__(NT) k_resid64(Dims d, M6<double> m, const doub
 
 __global__ void k_set_target(BcgScalars *sc, double target)
 {
+    after_previous();
     sc->target = target;
     sc->done = 0;
     sc->iters = 0;
@@ -356,24 +365,24 @@ int bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first,
     const M6<T> M = m6(m);
     T *p = V.p, *v = V.v;
     if (ev) cudaEventRecord(ev[0], st);
-    k_bcg_u<T><<<g, b, 0, st>>>(d, V.r, p, v, sc, first ? 1 : 0);
+    launch_after(k_bcg_u<T>, g, b, 0, st, d, V.r, p, v, sc, first ? 1 : 0);
     const Red red{R.partials, R.finished, sc, 0};
     const bool last = R.nblocks <= LAST_MAX, last_x = R.nblocks <= LAST_MAX_X;
     auto *kp = last ? k_bcg_p<T, true> : k_bcg_p<T, false>;
     auto *ks = last ? k_bcg_s<T, true> : k_bcg_s<T, false>;
     auto *kx = last_x ? k_bcg_x<T, true> : k_bcg_x<T, false>;
     if (ev) cudaEventRecord(ev[1], st);
-    kp<<<g, b, 0, st>>>(d, M, p, V.r0, v, red);
+    launch_after(kp, g, b, 0, st, d, M, p, V.r0, v, red);
     if (ev) cudaEventRecord(ev[2], st);
-    if (!last) k_red<BR_ALPHA><<<1, NT, 0, st>>>(red, R.nblocks);
+    if (!last) launch_after(k_red<BR_ALPHA>, 1, NT, 0, st, red, R.nblocks);
     if (ev) cudaEventRecord(ev[3], st);
-    ks<<<g, b, 0, st>>>(d, M, V.r, v, V.t, red);
+    launch_after(ks, g, b, 0, st, d, M, V.r, v, V.t, red);
     if (ev) cudaEventRecord(ev[4], st);
-    if (!last) k_red<BR_OMEGA><<<1, NT, 0, st>>>(red, R.nblocks);
+    if (!last) launch_after(k_red<BR_OMEGA>, 1, NT, 0, st, red, R.nblocks);
     if (ev) cudaEventRecord(ev[5], st);
-    kx<<<g, b, 0, st>>>(d, V.x, V.r, V.r0, p, v, V.t, red);
+    launch_after(kx, g, b, 0, st, d, V.x, V.r, V.r0, p, v, V.t, red);
     if (ev) cudaEventRecord(ev[6], st);
-    if (!last_x) k_red<BR_RHO><<<1, NT, 0, st>>>(red, R.nblocks);
+    if (!last_x) launch_after(k_red<BR_RHO>, 1, NT, 0, st, red, R.nblocks);
     return 4 + (last ? 0 : 2) + (last_x ? 0 : 1);
 }
 
@@ -383,8 +392,8 @@ int resid64(const Dims &d, const double *const m[6], const double *b, const doub
     const Red red{R.partials, R.finished, sc, want_bb ? 1 : 0};
     const bool last = R.nblocks <= LAST_MAX_X;
     auto *k = last ? k_resid64<true> : k_resid64<false>;
-    k<<<solver_grid(d), solver_block(), 0, st>>>(d, m6(m), b, x, r64, r32, red);
-    if (!last) k_red<BR_RESID><<<1, NT, 0, st>>>(red, R.nblocks);
+    launch_after(k, solver_grid(d), solver_block(), 0, st, d, m6(m), b, x, r64, r32, red);
+    if (!last) launch_after(k_red<BR_RESID>, 1, NT, 0, st, red, R.nblocks);
     return last ? 1 : 2;
 }
 
@@ -395,7 +404,7 @@ void set_target(BcgScalars *sc, double target, cudaStream_t st)
 
 void xadd(const Dims &d, double *x, const float *e, cudaStream_t st)
 {
-    k_xadd<<<solver_grid(d), solver_block(), 0, st>>>(d, x, e);
+    launch_after(k_xadd, solver_grid(d), solver_block(), 0, st, d, x, e);
 }
 
 template int bcg_iteration<double>(const Dims &, const double *const[6], BcgVecs<double> &, bool, Reduce &,

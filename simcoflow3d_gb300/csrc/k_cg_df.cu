@@ -20,6 +20,7 @@
 // its residual is recomputed in FP64, so the stopping test on the true
 // residual is unchanged.
 #include "scf_df.cuh"
+#include "scf_launch.cuh"
 #include "scf_reduce.cuh"
 
 namespace {
@@ -81,6 +82,7 @@ template <bool LAST>
 __global__ void __launch_bounds__(128, 8) k_spmv_df(DfOp A, const float2 *__restrict__ p, float2 *__restrict__ q,
                                                  RedOut red, int kz)
 {
+    after_previous();
     DF_ZCHUNK(A);
     double v = 0.0;
     float2 sq = make_float2(0.f, 0.f);
@@ -119,6 +121,7 @@ template <bool LAST>
 __global__ void __launch_bounds__(128) k_dot_rz_df(DfOp A, const float2 *__restrict__ r, const float *__restrict__ z,
                                                    RedOut red, int kz)
 {
+    after_previous();
     DF_ZCHUNK(A);
     double v = 0.0;
     if (in) {
@@ -151,6 +154,7 @@ __global__ void __launch_bounds__(128) k_cg_update_df(DfOp A, float2 *__restrict
                                                       float *__restrict__ rlow, float *__restrict__ x0, float first,
                                                       RedOut red, int kz)
 {
+    after_previous();
     DF_ZCHUNK(A);
     double v = 0.0;
     if (in) {
@@ -177,6 +181,7 @@ __global__ void __launch_bounds__(128) k_cg_update_df(DfOp A, float2 *__restrict
 __global__ void __launch_bounds__(128) k_pupdate_df(DfOp A, const float *__restrict__ z, float2 *__restrict__ p,
                                                     const double *__restrict__ scal, int first, int kz)
 {
+    after_previous();
     DF_ZCHUNK(A);
     if (!in) return;
     const float2 be = dfrom(first ? 0.0 : scal[S_BETA]);
@@ -220,7 +225,7 @@ void df_spmv_dot(const DfOp &A, const float2 *p, float2 *q, Reducer &R, bool sin
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     const int id = kt_begin(kt, KC_SPMV, st);
     auto *k = red_last(nblocks(l)) ? k_spmv_df<true> : k_spmv_df<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, p, q, red_out(R, singular), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, p, q, red_out(R, singular), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     red_finish<RK_ALPHA>(R, nblocks(l), singular, st, launches);
@@ -230,7 +235,7 @@ void df_dot_rz(const DfOp &A, const float2 *r, const float *z, Reducer &R, cudaS
 {
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     auto *k = red_last(nblocks(l)) ? k_dot_rz_df<true> : k_dot_rz_df<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, r, z, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, r, z, red_out(R), l.kz);
     *launches += 1;
     red_finish<RK_BETA>(R, nblocks(l), false, st, launches);
 }
@@ -241,7 +246,7 @@ void df_cg_update(const DfOp &A, float2 *x, float2 *r, const float2 *p, const fl
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
     const int id = kt_begin(kt, KC_CGUPDATE, st);
     auto *k = red_last(nblocks(l)) ? k_cg_update_df<true> : k_cg_update_df<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, x0, (float)first, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, x, r, p, q, rlow, x0, (float)first, red_out(R), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     red_finish<RK_RR>(R, nblocks(l), false, st, launches);
@@ -251,7 +256,7 @@ void df_pupdate(const DfOp &A, const float *z, float2 *p, const double *scal, bo
                 int *launches)
 {
     const March l = launch_march(A.hi.n0, A.hi.n1, A.hi.n2);
-    k_pupdate_df<<<l.grid, l.block, 0, st>>>(A, z, p, scal, first ? 1 : 0, l.kz);
+    launch_after(k_pupdate_df, l.grid, l.block, 0, st, A, z, p, scal, first ? 1 : 0, l.kz);
     *launches += 1;
 }
 

@@ -26,6 +26,7 @@
 // the block's own cells by plain loads cost more in branches than it saved.
 #include "scf_cheb.cuh"
 #include "scf_kernels.h"
+#include "scf_launch.cuh"
 
 namespace {
 
@@ -565,6 +566,7 @@ __device__ void coarsest(const CcArgs<T> &a, const Ctx<T> &S, const CcLevel<T> &
 template <typename T, bool LINES>
 __global__ void __launch_bounds__(CC_THREADS, 1) k_coarse_cycle(const __grid_constant__ CcArgs<T> a)
 {
+    after_previous();
     extern __shared__ __align__(16) unsigned char cc_smem[];
     __shared__ double sb[128], red[5];
     __shared__ unsigned char sact[128];
@@ -728,7 +730,7 @@ int coarse_first_level(const MgLevel<T> *L, int nlev, bool lines)
 
 template <typename T>
 T *launch_coarse_cycle(const MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, const int *map,
-                       int ncoarse, bool singular, bool first_done, cudaStream_t st)
+                       int ncoarse, bool singular, bool first_done, bool after_event, cudaStream_t st)
 {
     CcArgs<T> a;
     cudaLaunchConfig_t cfg = {};
@@ -747,12 +749,14 @@ T *launch_coarse_cycle(const MgLevel<T> *L, int nlev, const ChebCoef &cc, const 
     cfg.gridDim = dim3(cluster_blocks());
     cfg.blockDim = dim3(CC_THREADS);
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = cfg.gridDim.x;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = after_event ? 1 : 2;   // (a kernel that also waits for an event is launched plainly)
     if constexpr (sizeof(T) == 4) {
         if (cc.lines) cudaLaunchKernelEx(&cfg, k_coarse_cycle<T, true>, a);
         else cudaLaunchKernelEx(&cfg, k_coarse_cycle<T, false>, a);
@@ -765,6 +769,6 @@ T *launch_coarse_cycle(const MgLevel<T> *L, int nlev, const ChebCoef &cc, const 
 template int coarse_first_level<float>(const MgLevel<float> *, int, bool);
 template int coarse_first_level<double>(const MgLevel<double> *, int, bool);
 template float *launch_coarse_cycle<float>(const MgLevel<float> *, int, const ChebCoef &, const double *, const int *,
-                                           int, bool, bool, cudaStream_t);
+                                           int, bool, bool, bool, cudaStream_t);
 template double *launch_coarse_cycle<double>(const MgLevel<double> *, int, const ChebCoef &, const double *, const int *,
-                                             int, bool, bool, cudaStream_t);
+                                             int, bool, bool, bool, cudaStream_t);

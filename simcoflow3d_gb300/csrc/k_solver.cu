@@ -17,6 +17,7 @@
 
 #include "scf_cheb.cuh"
 #include "scf_kernels.h"
+#include "scf_launch.cuh"
 #include "scf_reduce.cuh"
 #include "scf_tma.cuh"
 
@@ -46,6 +47,7 @@ template <bool LAST>
 __global__ void __launch_bounds__(128) k_spmv_dot(LevelView<double> A, const double *__restrict__ p,
                                                   double *__restrict__ q, RedOut red, int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     double v = 0.0, sq = 0.0;
     if (in) {
@@ -73,7 +75,7 @@ void cg_spmv_dot(const LevelView<double> &A, const double *p, double *q, Reducer
     const March l = launch_march(A.n0, A.n1, A.n2);
     const int id = kt_begin(kt, KC_SPMV, st);
     auto *k = red_last(nblocks(l)) ? k_spmv_dot<true> : k_spmv_dot<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, p, q, red_out(R, singular), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, p, q, red_out(R, singular), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     red_finish<RK_ALPHA>(R, nblocks(l), singular, st, launches);
@@ -90,6 +92,7 @@ __global__ void __launch_bounds__(128) k_cg_update(LevelView<double> A, double *
                                                    LevelView<T> L0, T *__restrict__ x0, T first,
                                                    RedOut red, int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     double v = 0.0;
     if (in) {
@@ -116,7 +119,7 @@ void cg_update(const LevelView<double> &A, double *x, double *r, const double *p
     const March l = launch_march(A.n0, A.n1, A.n2);
     const int id = kt_begin(kt, KC_CGUPDATE, st);
     auto *k = red_last(nblocks(l)) ? k_cg_update<T, true> : k_cg_update<T, false>;
-    k<<<l.grid, l.block, 0, st>>>(A, x, r, p, q, rlow, L0, x0, (T)first, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, x, r, p, q, rlow, L0, x0, (T)first, red_out(R), l.kz);
     kt_end(kt, id, st);
     *launches += 1;
     red_finish<RK_RR>(R, nblocks(l), false, st, launches);
@@ -131,6 +134,7 @@ __global__ void __launch_bounds__(128) k_dot_rz(LevelView<double> A, const doubl
                                                 const T *__restrict__ rlow, const T *__restrict__ z,
                                                 RedOut red, int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     double v = 0.0;
     if (in) {
@@ -152,7 +156,7 @@ void cg_dot_rz(const LevelView<double> &A, const double *r, const T *rlow, const
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
     auto *k = red_last(nblocks(l)) ? k_dot_rz<T, true> : k_dot_rz<T, false>;
-    k<<<l.grid, l.block, 0, st>>>(A, r, rlow, z, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, r, rlow, z, red_out(R), l.kz);
     *launches += 1;
     red_finish<RK_BETA>(R, nblocks(l), false, st, launches);
 }
@@ -162,6 +166,7 @@ __global__ void __launch_bounds__(128) k_pupdate(LevelView<double> A, const T *_
                                                  double *__restrict__ p, const double *__restrict__ scal, int first,
                                                  int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     if (!in) return;
     const double beta = first ? 0.0 : scal[S_BETA];
@@ -177,7 +182,7 @@ void cg_pupdate(const LevelView<double> &A, const T *z, double *p, const double 
                 int *launches)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    k_pupdate<T><<<l.grid, l.block, 0, st>>>(A, z, p, scal, first ? 1 : 0, l.kz);
+    launch_after(k_pupdate<T>, l.grid, l.block, 0, st, A, z, p, scal, first ? 1 : 0, l.kz);
     *launches += 1;
 }
 
@@ -340,6 +345,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_cheb_first(LevelView<T> L, const T *__restrict__ b, T *__restrict__ x,
                                                     T coef)
 {
+    after_previous();
     INTERIOR_IJK(L);
     if (in) x[c] = coef * dinv_at(L, c) * b[c];
 }
@@ -350,6 +356,7 @@ __global__ void __launch_bounds__(256) k_cheb_step(LevelView<T> L, const T *__re
                                                    const T *__restrict__ xin, const T *dprev,
                                                    T *__restrict__ xout, T *dout, T c1, T c2)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = (blockIdx.z * blockDim.z + threadIdx.z) * M + 1;
@@ -394,11 +401,11 @@ void cheb_step(const LevelView<T> &L, const T *b, const T *xin, const T *dprev, 
     if constexpr (sizeof(T) == 4) {
         if ((long long)L.n0 * L.n1 * L.n2 >= 1ll << 18) {
             l.grid.z = (L.n2 + 7) / 8;
-            k_cheb_step<T, 4><<<l.grid, l.block, 0, st>>>(L, b, xin, dprev, xout, dout, c1, c2);
+            launch_after(k_cheb_step<T, 4>, l.grid, l.block, 0, st, L, b, xin, dprev, xout, dout, c1, c2);
             return;
         }
     }
-    k_cheb_step<T, 1><<<l.grid, l.block, 0, st>>>(L, b, xin, dprev, xout, dout, c1, c2);
+    launch_after(k_cheb_step<T, 1>, l.grid, l.block, 0, st, L, b, xin, dprev, xout, dout, c1, c2);
 }
 
 // ---------------------------------------------------------------------------
@@ -557,6 +564,7 @@ template <bool DP, bool DO, bool RS>
 __global__ void __launch_bounds__(C2_THREADS, C2_BLOCKS_PER_SM) k_cheb_pair(const __grid_constant__ PairMaps tm,
                                                                           PairArgs a)
 {
+    after_previous();
     extern __shared__ __align__(128) float c2_raw[];
     const unsigned raw = (unsigned)__cvta_generic_to_shared(c2_raw);
     const unsigned sb = (raw + 127u) & ~127u;            // 128-byte aligned start of the rings
@@ -873,10 +881,10 @@ cudaError_t cheb_pair(const MgLevel<float> &F, const float *xin, const float *dp
     g_pair_tma.fetch_add(1);
     const dim3 blk(C2_TX, C2_TY, 1);
     const dim3 grd((F.n0 + C2_TX - 1) / C2_TX, (F.n1 + C2_TY - 1) / C2_TY, (F.n2 + a.planes - 1) / a.planes);
-    if (dprev && dout) k_cheb_pair<true, true, false><<<grd, blk, C2_SMEM, st>>>(tm, a);
-    else if (dprev) k_cheb_pair<true, false, false><<<grd, blk, C2_SMEM, st>>>(tm, a);
-    else if (dout) k_cheb_pair<false, true, false><<<grd, blk, C2_SMEM, st>>>(tm, a);
-    else k_cheb_pair<false, false, false><<<grd, blk, C2_SMEM, st>>>(tm, a);
+    if (dprev && dout) launch_after(k_cheb_pair<true, true, false>, grd, blk, C2_SMEM, st, tm, a);
+    else if (dprev) launch_after(k_cheb_pair<true, false, false>, grd, blk, C2_SMEM, st, tm, a);
+    else if (dout) launch_after(k_cheb_pair<false, true, false>, grd, blk, C2_SMEM, st, tm, a);
+    else launch_after(k_cheb_pair<false, false, false>, grd, blk, C2_SMEM, st, tm, a);
     return cudaSuccess;
 }
 
@@ -908,7 +916,7 @@ bool cheb_restrict(const MgLevel<float> &F, const MgLevel<float> &C, const float
     g_pair_tma.fetch_add(1);
     const dim3 blk(C2_TX, C2_TY, 1);
     const dim3 grd((F.n0 + C2_TX - 1) / C2_TX, (F.n1 + C2_TY - 1) / C2_TY, (F.n2 + a.planes - 1) / a.planes);
-    k_cheb_pair<true, false, true><<<grd, blk, C2_SMEM, st>>>(tm, a);
+    launch_after(k_cheb_pair<true, false, true>, grd, blk, C2_SMEM, st, tm, a);
     return true;
 }
 
@@ -935,6 +943,7 @@ __global__ void __launch_bounds__(128) k_cheb_line(LevelView<T> L, const T *__re
                                                    const T *dprev, T *__restrict__ xout, T *__restrict__ dout, T c1,
                                                    T c2, int zero_guess)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k0 = blockIdx.z * LINE_SEG + 1;
@@ -1010,7 +1019,7 @@ void launch_cheb_line(const MgLevel<T> &F, const T *x, const T *dprev, T *xout, 
 {
     dim3 blk(32, 4, 1);
     dim3 grd((F.n0 + 31) / 32, (F.n1 + 3) / 4, (F.n2 + LINE_SEG - 1) / LINE_SEG);
-    k_cheb_line<T><<<grd, blk, 0, st>>>(F.view(), F.b, x, dprev, xout, dout, (T)c1, (T)c2, zero_guess ? 1 : 0);
+    launch_after(k_cheb_line<T>, grd, blk, 0, st, F.view(), F.b, x, dprev, xout, dout, (T)c1, (T)c2, zero_guess ? 1 : 0);
 }
 
 // Residual of the fine level summed over each coarse cell's children (and,
@@ -1026,6 +1035,7 @@ __global__ void __launch_bounds__(128) k_restrict(LevelView<T> F, const T *__res
                                                   const T *__restrict__ x, LevelView<T> C, T *__restrict__ bc,
                                                   int f0, int f1, int f2, T *__restrict__ xc, T first)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int J = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int K = blockIdx.z + 1;
@@ -1065,6 +1075,7 @@ __global__ void __launch_bounds__(256) k_post_first(LevelView<T> F, const T *__r
                                                     const T *__restrict__ e, T *__restrict__ xout,
                                                     T *__restrict__ dout, int f0, int f1, int f2, T coef)
 {
+    after_previous();
     INTERIOR_IJK(F);
     if (!in) return;
     const int s0 = f0 - 1, s1 = f1 - 1, s2 = f2 - 1;   // factors are 1 or 2
@@ -1100,6 +1111,7 @@ __global__ void __launch_bounds__(256) k_prolong(LevelView<T> F, const unsigned 
                                                  T *__restrict__ x, LevelView<T> C, const T *__restrict__ e, int s0,
                                                  int s1, int s2)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int kb = blockIdx.z * PR_KZ + 1;
@@ -1129,7 +1141,7 @@ void launch_prolong(const MgLevel<T> &F, const MgLevel<T> &C, T *x, const T *e, 
 {
     const dim3 blk(32, 8, 1);
     const dim3 grd((F.n0 + 31) / 32, (F.n1 + 7) / 8, (F.n2 + PR_KZ - 1) / PR_KZ);
-    k_prolong<T><<<grd, blk, 0, st>>>(F.view(), F.active, x, C.view(), e, F.f0 - 1, F.f1 - 1, F.f2 - 1);
+    launch_after(k_prolong<T>, grd, blk, 0, st, F.view(), F.active, x, C.view(), e, F.f0 - 1, F.f1 - 1, F.f2 - 1);
 }
 
 // coarsest level: y = Ainv (b - mean) on the active cells (one block)
@@ -1445,13 +1457,13 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
             MgLevel<T> &C = L[l + 1];
             dim3 rg((F.n0 + 31) / 32, (C.n1 + 3) / 4, C.n2), rb(32, 4, 1);
             const int id = l == 0 ? kt_begin(kt, KC_RESTRICT, st) : -1;
-            k_restrict<T><<<rg, rb, 0, st>>>(v, F.b, xa, C.view(), C.b, F.f0, F.f1, F.f2, nullptr, T(0));
+            launch_after(k_restrict<T>, rg, rb, 0, st, v, F.b, xa, C.view(), C.b, F.f0, F.f1, F.f2, nullptr, T(0));
             kt_end(kt, id, st);
             *launches += 1;
             continue;
         }
         if (!(l == 0 ? first_done : first_written[l])) {
-            k_cheb_first<T><<<lf.grid, lf.block, 0, st>>>(v, F.b, xa, (T)cc.first);
+            launch_after(k_cheb_first<T>, lf.grid, lf.block, 0, st, v, F.b, xa, (T)cc.first);
             *launches += 1;
         }
         int s = 1;
@@ -1509,7 +1521,7 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
         dim3 rg((F.n0 + 31) / 32, (C.n1 + 3) / 4, C.n2), rb(32, 4, 1);
         const int id = l == 0 ? kt_begin(kt, KC_RESTRICT, st) : -1;
         const bool wx = l + 1 < last;
-        k_restrict<T><<<rg, rb, 0, st>>>(v, F.b, xa, C.view(), C.b, F.f0, F.f1, F.f2, wx ? C.x : nullptr,
+        launch_after(k_restrict<T>, rg, rb, 0, st, v, F.b, xa, C.view(), C.b, F.f0, F.f1, F.f2, wx ? C.x : nullptr,
                                          (T)cc.first);
         first_written[l + 1] = wx;
         kt_end(kt, id, st);
@@ -1518,7 +1530,7 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
     if (small < last) {
         if (coarse_ready) cudaStreamWaitEvent(st, coarse_ready, 0);
         cur[small] = launch_coarse_cycle<T>(L + small, nlev - small, cc, ainv, map, ncoarse, singular,
-                                            small == 0 ? first_done : first_written[small], st);
+                                            small == 0 ? first_done : first_written[small], coarse_ready != nullptr, st);
         *launches += 1;
     } else {
         MgLevel<T> &Cst = L[last];
@@ -1590,7 +1602,7 @@ T *mg_vcycle(MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, co
             *launches += 2;
         } else {
             const int idp = l == 0 ? kt_begin(kt, KC_PROLONG, st) : -1;
-            k_post_first<T><<<lf.grid, lf.block, 0, st>>>(v, F.b, xa, C.view(), cur[l + 1], xb, more ? F.d : nullptr,
+            launch_after(k_post_first<T>, lf.grid, lf.block, 0, st, v, F.b, xa, C.view(), cur[l + 1], xb, more ? F.d : nullptr,
                                                           F.f0, F.f1, F.f2, (T)cc.first);
             kt_end(kt, idp, st);
             *launches += 1;
@@ -1627,14 +1639,14 @@ template <typename T>
 void probe_restrict(MgLevel<T> &F, MgLevel<T> &C, cudaStream_t st)
 {
     dim3 rg((F.n0 + 31) / 32, (C.n1 + 3) / 4, C.n2), rb(32, 4, 1);
-    k_restrict<T><<<rg, rb, 0, st>>>(F.view(), F.b, F.x, C.view(), C.b, F.f0, F.f1, F.f2, nullptr, T(0));
+    launch_after(k_restrict<T>, rg, rb, 0, st, F.view(), F.b, F.x, C.view(), C.b, F.f0, F.f1, F.f2, nullptr, T(0));
 }
 
 template <typename T>
 void probe_prolong(MgLevel<T> &F, MgLevel<T> &C, const ChebCoef &cc, cudaStream_t st)
 {
     Launch3 lf = launch_interior(F.n0, F.n1, F.n2);
-    k_post_first<T><<<lf.grid, lf.block, 0, st>>>(F.view(), F.b, F.x, C.view(), C.x, F.xb, F.d, F.f0, F.f1, F.f2,
+    launch_after(k_post_first<T>, lf.grid, lf.block, 0, st, F.view(), F.b, F.x, C.view(), C.x, F.xb, F.d, F.f0, F.f1, F.f2,
                                                    (T)cc.first);
 }
 
@@ -1642,7 +1654,7 @@ void probe_spmv(const LevelView<double> &A, const double *p, double *q, Reducer 
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
     auto *k = red_last(nblocks(l)) ? k_spmv_dot<true> : k_spmv_dot<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, p, q, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, p, q, red_out(R), l.kz);
 }
 
 template void probe_smooth<float>(MgLevel<float> &, const ChebCoef &, cudaStream_t);

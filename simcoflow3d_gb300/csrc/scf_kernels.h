@@ -167,7 +167,7 @@ template <typename T>
 int coarse_first_level(const MgLevel<T> *L, int nlev, bool lines);
 template <typename T>
 T *launch_coarse_cycle(const MgLevel<T> *L, int nlev, const ChebCoef &cc, const double *ainv, const int *map,
-                       int ncoarse, bool singular, bool first_done, cudaStream_t st);
+                       int ncoarse, bool singular, bool first_done, bool after_event, cudaStream_t st);
 cudaError_t coarse_cycle_attr();   // its launch attributes (called outside any capture)
 
 // Single launches of the fine-level kernels, for timing.

@@ -15,6 +15,7 @@
 // where a shuffle tree in 1024 threads has 160.
 #pragma once
 #include "scf_kernels.h"
+#include "scf_launch.cuh"
 
 struct RedOut {
     double *part, *scal, *mail;
@@ -159,6 +160,7 @@ __device__ __forceinline__ void red_end(const RedOut &o, double s)
 template <int KIND>
 __global__ void __launch_bounds__(128) k_reduce(RedOut o, int nb)
 {
+    after_previous();
     red_tail<KIND>(o, nb);
 }
 
@@ -167,6 +169,6 @@ template <int KIND>
 void red_finish(const Reducer &R, unsigned blocks, bool singular, cudaStream_t st, int *launches)
 {
     if (red_last(blocks)) return;
-    k_reduce<KIND><<<1, 128, 0, st>>>(red_out(R, singular), (int)blocks);
+    launch_after(k_reduce<KIND>, 1, 128, 0, st, red_out(R, singular), (int)blocks);
     *launches += 1;
 }
