@@ -6,6 +6,7 @@
 #include <cuda_pipeline.h>
 
 #include "scf_kernels.h"
+#include "scf_launch.cuh"
 
 namespace {
 
@@ -178,6 +179,7 @@ __device__ __forceinline__ void load_face_in(const AsmArgs &a, int i, int j, int
 // below.
 __global__ void __launch_bounds__(128) k_pocoef(AsmArgs a)
 {
+    after_previous();
     const Dims &d = a.d;
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -269,6 +271,7 @@ __global__ void __launch_bounds__(128) k_pocoef(AsmArgs a)
 // chain of dependent loads: 52 us at 147x93x121.)
 __global__ void __launch_bounds__(128) k_pocoef_groups(AsmArgs a, int ncol, int ngrp)
 {
+    after_previous();
     const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (g >= ngrp) return;
     const int c0 = g * 64;
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(128) k_pocoef_groups(AsmArgs a, int ncol, int 
 // within the cell's group, then whole groups) that assigned the stream.
 __global__ void k_pocoef_heads(AsmArgs a, unsigned count)
 {
+    after_previous();
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= count) return;
     const Dims &d = a.d;
@@ -318,6 +322,7 @@ __global__ void k_pocoef_heads(AsmArgs a, unsigned count)
 // Boundary planes take the neighbouring plane (ProjectionP.f90:256-264).
 __global__ void k_pocoef_boundary(AsmArgs a)
 {
+    after_previous();
     const Dims &d = a.d;
     const int f = blockIdx.z;  // 0..5
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -463,6 +468,7 @@ __device__ __forceinline__ void op_issue(const AsmArgs &a, double *sd, int *si, 
 template <bool MIXED>
 __global__ void __launch_bounds__(OP_THREADS, 3) k_operator(AsmArgs a, OpArgs o)
 {
+    after_previous();
     extern __shared__ __align__(16) unsigned char op_smem[];
     double *sd0 = (double *)op_smem;
     int *si0 = (int *)(sd0 + 2 * V_COUNT * OP_THREADS);
@@ -626,7 +632,7 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
     } else {
         dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + a.kseg - 1) / a.kseg);
         k_phase<<<2 * 152 * 8, 256, 0, st>>>(a);
-        k_pocoef<<<g, b, 0, st>>>(a);
+        launch_after(k_pocoef, g, b, 0, st, a);
         *launches += 2;
         cudaMemcpyAsync(stale_count_host, a.stale_count, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
         cudaStreamSynchronize(st);
@@ -635,8 +641,8 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
     if (cnt > a.stale_cap) cnt = a.stale_cap;
     if (cnt) {
         const int ncol = d.I * d.J * ((d.K + a.kseg - 1) / a.kseg), ngrp = (ncol + 63) / 64;
-        k_pocoef_groups<<<(ngrp + 3) / 4, 128, 0, st>>>(a, ncol, ngrp);
-        k_pocoef_heads<<<(cnt + 127) / 128, 128, 0, st>>>(a, cnt);
+        launch_after(k_pocoef_groups, (ngrp + 3) / 4, 128, 0, st, a, ncol, ngrp);
+        launch_after(k_pocoef_heads, (cnt + 127) / 128, 128, 0, st, a, cnt);
         *launches += 2;
     }
     {
@@ -644,7 +650,7 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
         if (d.I * d.K > m) m = d.I * d.K;
         if (d.I * d.J > m) m = d.I * d.J;
         dim3 g((m + 255) / 256, 1, 6);
-        k_pocoef_boundary<<<g, 256, 0, st>>>(a);
+        launch_after(k_pocoef_boundary, g, 256, 0, st, a);
         *launches += 1;
     }
     dim3 ob(32, 4), og((d.I + 31) / 32, (d.J + 3) / 4, (d.K + a.kseg - 1) / a.kseg);
@@ -653,9 +659,9 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
     cudaFuncSetAttribute(k_operator<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OP_SMEM);
     cudaFuncSetAttribute(k_operator<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OP_SMEM);
     if (mixed)
-        k_operator<true><<<og, ob, OP_SMEM, st>>>(a, o);
+        launch_after(k_operator<true>, og, ob, OP_SMEM, st, a, o);
     else
-        k_operator<false><<<og, ob, OP_SMEM, st>>>(a, o);
+        launch_after(k_operator<false>, og, ob, OP_SMEM, st, a, o);
     *launches += 1;
     return (int)cudaGetLastError();
 }

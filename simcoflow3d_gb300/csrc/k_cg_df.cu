@@ -196,6 +196,7 @@ __global__ void __launch_bounds__(128) k_pupdate_df(DfOp A, const float *__restr
 // element-wise conversions over the whole padded array (in place allowed)
 __global__ void k_df_from_double(const double *src, float2 *dst, int n)
 {
+    after_previous();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const double d = src[e];
         dst[e] = dfrom(d);
@@ -205,6 +206,7 @@ __global__ void k_df_from_double(const double *src, float2 *dst, int n)
 // and its FP32 copy (the hi part) for the V-cycle, in one pass
 __global__ void k_df_round_start(double *r, float *rlow, int n)
 {
+    after_previous();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const float2 v = dfrom(r[e]);
         ((float2 *)r)[e] = v;
@@ -213,6 +215,7 @@ __global__ void k_df_round_start(double *r, float *rlow, int n)
 }
 __global__ void k_df_to_double(const float2 *src, double *dst, int n)
 {
+    after_previous();
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
         const float2 v = src[e];
         dst[e] = dwide(v);
@@ -262,18 +265,18 @@ void df_pupdate(const DfOp &A, const float *z, float2 *p, const double *scal, bo
 
 void df_from_double(const double *src, float2 *dst, int n, cudaStream_t st, int *launches)
 {
-    k_df_from_double<<<152 * 8, 256, 0, st>>>(src, dst, n);
+    launch_after(k_df_from_double, 152 * 8, 256, 0, st, src, dst, n);
     *launches += 1;
 }
 
 void df_round_start(double *r, float *rlow, int n, cudaStream_t st, int *launches)
 {
-    k_df_round_start<<<152 * 8, 256, 0, st>>>(r, rlow, n);
+    launch_after(k_df_round_start, 152 * 8, 256, 0, st, r, rlow, n);
     *launches += 1;
 }
 
 void df_to_double(const float2 *src, double *dst, int n, cudaStream_t st, int *launches)
 {
-    k_df_to_double<<<152 * 8, 256, 0, st>>>(src, dst, n);
+    launch_after(k_df_to_double, 152 * 8, 256, 0, st, src, dst, n);
     *launches += 1;
 }

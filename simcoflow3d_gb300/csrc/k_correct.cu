@@ -3,6 +3,7 @@
 // Compiled with -fmad=false so that each expression rounds exactly as the
 // reference's Fortran statement does.
 #include "scf_kernels.h"
+#include "scf_launch.cuh"
 
 // ---------------------------------------------------------------------------
 // DeltaPressureGetValues + DeltaPressureBoundaryCondition (ProjectionP.f90:
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(256) k_scatter(CorrArgs a)
 
 __global__ void k_pp_ghost(CorrArgs a)
 {
+    after_previous();
     const Dims &d = a.d;
     const int f = blockIdx.z;  // 0..5 = W,E,S,N,B,T
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -57,7 +59,7 @@ void launch_scatter(const CorrArgs &a, cudaStream_t st, int *launches)
     Launch3 l = launch_interior(d.I, d.J, d.K);
     k_scatter<<<l.grid, l.block, 0, st>>>(a);
     dim3 g((max_plane(d) + 255) / 256, 1, 6);
-    k_pp_ghost<<<g, 256, 0, st>>>(a);
+    launch_after(k_pp_ghost, g, 256, 0, st, a);
     *launches += 2;
 }
 
@@ -148,6 +150,7 @@ __device__ __forceinline__ double spacing(const CorrArgs &c, int axis, int face,
 // phase 1 (top face only): apply the writes from the saved Var.
 __global__ void k_bc_face(CorrArgs c, int face, int phase)
 {
+    after_previous();
     const Dims &d = c.d;
     const int axis = face >> 1;
     const int na = axis == 0 ? d.J : d.I;
@@ -184,6 +187,7 @@ __global__ void k_bc_face(CorrArgs c, int face, int phase)
 // Dirichlet pressure face in the order W,E,S,N,B,T is corrected.
 __global__ void k_mass_fix(CorrArgs c, int face)
 {
+    after_previous();
     const Dims &d = c.d;
     const int axis = face >> 1;
     const int na = axis == 0 ? d.J : d.I;
@@ -239,10 +243,10 @@ void launch_correct(const CorrArgs &a, cudaStream_t st, int *launches)
         const int na = axis == 0 ? d.J : d.I;
         const int nb = axis == 2 ? d.J : d.K;
         dim3 g((na * nb + 255) / 256, 4);
-        k_bc_face<<<g, 256, 0, st>>>(a, face, 0);
+        launch_after(k_bc_face, g, 256, 0, st, a, face, 0);
         *launches += 1;
         if (face == 5) {
-            k_bc_face<<<g, 256, 0, st>>>(a, face, 1);
+            launch_after(k_bc_face, g, 256, 0, st, a, face, 1);
             *launches += 1;
         }
     }
@@ -253,7 +257,7 @@ void launch_correct(const CorrArgs &a, cudaStream_t st, int *launches)
         const int axis = first >> 1;
         const int na = axis == 0 ? d.J : d.I;
         const int nb = axis == 2 ? d.J : d.K;
-        k_mass_fix<<<(na * nb + 255) / 256, 256, 0, st>>>(a, first);
+        launch_after(k_mass_fix, (na * nb + 255) / 256, 256, 0, st, a, first);
         *launches += 1;
     }
 }

@@ -5,6 +5,7 @@
 // HYPRE's only by the Jacobi scaling.
 #include "pred_kernels.h"
 #include "scf_common.cuh"
+#include "scf_launch.cuh"
 
 namespace pred {
 
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(256) k_mom_numbering(MomDev in, int comp, Dims
 // phase 0: lines along i over (j, k) in [0,J+1]x[0,K+1]; 1: along j; 2: along k.
 __global__ void k_dp_phase(double *dp, Dims d, int comp, int phase)
 {
+    after_previous();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     long long base, s;
@@ -361,6 +363,7 @@ __global__ void k_dp_phase(double *dp, Dims d, int comp, int phase)
 // loop-range cells of solid type already hold 0.
 __global__ void k_pred_bc(double *pred, MomDev in, Dims d, int comp)
 {
+    after_previous();
     const int a = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int b = blockIdx.y + 1;
     long long base, s;
@@ -417,12 +420,12 @@ void mom_check_numbering(const MomDev &in, int comp, const Dims &d, unsigned lon
 void mom_tail_comp(const MomDev &in, const Dims &d, int c, double *pred, double *dp, cudaStream_t st,
                    int *launches)
 {
-    k_dp_phase<<<dim3((d.J + 2 + 127) / 128, d.K + 2), 128, 0, st>>>(dp, d, c + 1, 0);
-    k_dp_phase<<<dim3((d.I + 2 + 127) / 128, d.K + 2), 128, 0, st>>>(dp, d, c + 1, 1);
-    k_dp_phase<<<dim3((d.I + 2 + 127) / 128, d.J + 2), 128, 0, st>>>(dp, d, c + 1, 2);
-    if (c == 0) k_pred_bc<<<dim3((d.J + 127) / 128, d.K), 128, 0, st>>>(pred, in, d, 1);
-    else if (c == 1) k_pred_bc<<<dim3((d.I + 127) / 128, d.K), 128, 0, st>>>(pred, in, d, 2);
-    else k_pred_bc<<<dim3((d.I + 127) / 128, d.J), 128, 0, st>>>(pred, in, d, 3);
+    launch_after(k_dp_phase, dim3((d.J + 2 + 127) / 128, d.K + 2), 128, 0, st, dp, d, c + 1, 0);
+    launch_after(k_dp_phase, dim3((d.I + 2 + 127) / 128, d.K + 2), 128, 0, st, dp, d, c + 1, 1);
+    launch_after(k_dp_phase, dim3((d.I + 2 + 127) / 128, d.J + 2), 128, 0, st, dp, d, c + 1, 2);
+    if (c == 0) launch_after(k_pred_bc, dim3((d.J + 127) / 128, d.K), 128, 0, st, pred, in, d, 1);
+    else if (c == 1) launch_after(k_pred_bc, dim3((d.I + 127) / 128, d.K), 128, 0, st, pred, in, d, 2);
+    else launch_after(k_pred_bc, dim3((d.I + 127) / 128, d.J), 128, 0, st, pred, in, d, 3);
     *launches += 4;
 }
 

@@ -208,6 +208,7 @@ template <bool LAST>
 __global__ void __launch_bounds__(128) k_sum_count(LevelView<double> A, const unsigned char *__restrict__ act,
                                                    const double *__restrict__ v, RedOut red, int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     double s = 0.0, cnt = 0.0;
     if (in) {
@@ -225,6 +226,7 @@ template <bool LAST>
 __global__ void __launch_bounds__(128) k_center_norm(LevelView<double> A, const unsigned char *__restrict__ act,
                                                      double *__restrict__ b, RedOut red, int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     double s = 0.0;
     if (in) {
@@ -251,7 +253,7 @@ void active_mean(const LevelView<double> &A, const unsigned char *active, const 
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
     auto *k = red_last(nblocks(l)) ? k_sum_count<true> : k_sum_count<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, active, v, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, active, v, red_out(R), l.kz);
     *launches += 1;
     red_finish<RK_COUNT>(R, nblocks(l), false, st, launches);
 }
@@ -262,12 +264,12 @@ void rhs_prologue(const LevelView<double> &A, const unsigned char *active, doubl
     const March l = launch_march(A.n0, A.n1, A.n2);
     if (singular) {
         auto *k = red_last(nblocks(l)) ? k_sum_count<true> : k_sum_count<false>;
-        k<<<l.grid, l.block, 0, st>>>(A, active, b, red_out(R), l.kz);
+        launch_after(k, l.grid, l.block, 0, st, A, active, b, red_out(R), l.kz);
         *launches += 1;
         red_finish<RK_COUNT>(R, nblocks(l), false, st, launches);
     }
     auto *k = red_last(nblocks(l)) ? k_center_norm<true> : k_center_norm<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, active, b, red_out(R, singular), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, active, b, red_out(R, singular), l.kz);
     *launches += 1;
     red_finish<RK_BB>(R, nblocks(l), singular, st, launches);
 }
@@ -278,6 +280,7 @@ __global__ void __launch_bounds__(128) k_final_residual(LevelView<double> A, con
                                                         double *__restrict__ r, int singular, RedOut red,
                                                         int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     double s = 0.0, sx = 0.0;
     if (in) {
@@ -300,7 +303,7 @@ void final_residual(const LevelView<double> &A, const unsigned char *active, con
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
     auto *k = red_last(nblocks(l)) ? k_final_residual<true> : k_final_residual<false>;
-    k<<<l.grid, l.block, 0, st>>>(A, active, b, x, r, singular ? 1 : 0, red_out(R), l.kz);
+    launch_after(k, l.grid, l.block, 0, st, A, active, b, x, r, singular ? 1 : 0, red_out(R), l.kz);
     *launches += 1;
     red_finish<RK_RESIDUAL>(R, nblocks(l), false, st, launches);
 }
@@ -308,6 +311,7 @@ void final_residual(const LevelView<double> &A, const unsigned char *active, con
 __global__ void __launch_bounds__(128) k_shift(LevelView<double> A, const unsigned char *__restrict__ act,
                                                double *__restrict__ x, const double *__restrict__ scal, int kz)
 {
+    after_previous();
     ZCHUNK_IJK(A);
     if (!in) return;
     const double mu = scal[S_MEANX];
@@ -320,7 +324,7 @@ void shift_solution(const LevelView<double> &A, const unsigned char *active, dou
                     cudaStream_t st, int *launches)
 {
     const March l = launch_march(A.n0, A.n1, A.n2);
-    k_shift<<<l.grid, l.block, 0, st>>>(A, active, x, scal, l.kz);
+    launch_after(k_shift, l.grid, l.block, 0, st, A, active, x, scal, l.kz);
     *launches += 1;
 }
 
@@ -1182,6 +1186,7 @@ __global__ void __launch_bounds__(128) k_coarse_solve(const T *__restrict__ b, T
 template <typename T>
 __global__ void __launch_bounds__(256) k_coarsen_cpl(MgLevel<T> F, MgLevel<T> C)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -1212,6 +1217,7 @@ __global__ void __launch_bounds__(256) k_coarsen_cpl(MgLevel<T> F, MgLevel<T> C)
 template <typename T>
 __global__ void __launch_bounds__(256) k_coarsen_diag(MgLevel<T> C)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -1231,8 +1237,8 @@ template <typename T>
 void mg_coarsen(const MgLevel<T> &F, MgLevel<T> &C, cudaStream_t st, int *launches)
 {
     Launch3 l = launch_interior(C.n0, C.n1, C.n2);
-    k_coarsen_cpl<T><<<l.grid, l.block, 0, st>>>(F, C);
-    k_coarsen_diag<T><<<l.grid, l.block, 0, st>>>(C);
+    launch_after(k_coarsen_cpl<T>, l.grid, l.block, 0, st, F, C);
+    launch_after(k_coarsen_diag<T>, l.grid, l.block, 0, st, C);
     *launches += 2;
 }
 

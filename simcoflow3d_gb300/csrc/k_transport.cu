@@ -38,6 +38,7 @@
 
 #include "../../include/scf_clsvof.h"
 #include "transport_body.cuh"
+#include "scf_launch.cuh"
 #include "scf_devmem.h"
 #include "scf_stage.h"
 
@@ -170,6 +171,7 @@ __global__ void __launch_bounds__(32) k_partial_fluxes(const __grid_constant__ D
                                                        const unsigned *__restrict__ count, double *__restrict__ flo,
                                                        double *__restrict__ fhi)
 {
+    after_previous();
     const unsigned n = *count, per = min(32u, max(4u, (n + 152 * 3 - 1) / (152 * 3)));
     if (threadIdx.x >= per) return;
     for (unsigned long long q = (unsigned long long)blockIdx.x * per + threadIdx.x; q < n;
@@ -186,6 +188,7 @@ __global__ void __launch_bounds__(RB_THREADS) k_partial_fluxes_scan(const __grid
                                                                     const __grid_constant__ tr::SweepIn S,
                                                                     double *__restrict__ flo, double *__restrict__ fhi)
 {
+    after_previous();
     __shared__ unsigned short list[RB_CELLS];
     __shared__ int count;
     if (threadIdx.x == 0) count = 0;
@@ -236,6 +239,7 @@ __global__ void __launch_bounds__(NB_THREADS) k_normals(const __grid_constant__ 
                                                         const uint32_t *__restrict__ list,
                                                         const unsigned *__restrict__ count)
 {
+    after_previous();
     if (blockIdx.x < kNormalBlocks) {
         // thread t of block b takes entry t * blocks + b: neighbouring entries, and
         // with them the long chains, go to different SMs
@@ -289,6 +293,7 @@ __global__ void __launch_bounds__(SW_X) k_sweep_x(const __grid_constant__ Dims D
                                                   double *__restrict__ ls_out, uint32_t *__restrict__ list,
                                                   unsigned *__restrict__ count)
 {
+    after_previous();
     __shared__ tr::LineFace sh[SW_X];
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
@@ -329,6 +334,7 @@ __global__ void __launch_bounds__(NX) k_sweep_yz(const __grid_constant__ Dims D,
                                                  double *__restrict__ ls_out, uint32_t *__restrict__ list,
                                                  unsigned *__restrict__ count, int len)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int o = blockIdx.y * blockDim.y + threadIdx.y + 1;   // the other index: k or j
     const bool in = i <= D.I && o <= (AX == 1 ? D.K : D.J);
@@ -363,6 +369,7 @@ __global__ void __launch_bounds__(NX) k_sweep_yz(const __grid_constant__ Dims D,
 // BoundaryConditionLvsVof: blockIdx.y is the axis, x strides its planes.
 __global__ void k_walls(Dims D, Geo G, tr::WallIn W)
 {
+    after_previous();
     const int axis = blockIdx.y;
     const size_t np = D.plane_size(axis);
     for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < np; t += (size_t)gridDim.x * blockDim.x)
@@ -424,6 +431,7 @@ __global__ void __launch_bounds__(BP_THREADS) k_band_bound(Dims D, Geo G, const 
                                                            const unsigned *__restrict__ count, unsigned *ub,
                                                            uint8_t *fix)
 {
+    after_previous();
     __shared__ tr::BandFace faces[BP_WARPS][6];
     const unsigned long long items = (unsigned long long)*count * BP_PARTS;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
@@ -476,6 +484,7 @@ __global__ void __launch_bounds__(BP_THREADS, 4) k_band_pairs(const __grid_const
                                                               const unsigned *__restrict__ ub, unsigned long long *key,
                                                               uint8_t *fix)
 {
+    after_previous();
     __shared__ tr::BandFace faces[BP_WARPS][6];
     __shared__ uint32_t q_cell[BQ_CAP];
     __shared__ unsigned short q_off[BQ_CAP];
@@ -534,6 +543,7 @@ __global__ void k_band_value(Dims D, Geo G, const double *__restrict__ vfl, cons
                              const unsigned long long *__restrict__ key, const uint8_t *__restrict__ fix,
                              double *phi)
 {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1, k = blockIdx.z + 1;
     if (i > D.I) return;
     phi[D.g(i, j, k)] = tr::band_value(D, G, vfl, dis, i, j, k, key, fix);
@@ -655,17 +665,16 @@ int scheme_step(scf_clsvof_ctx *ctx, bool listed, int &launches, Timer &T)
             unsigned *count = ctx->npart + sw + 1;
             T.before(0);
             if (sw == 0 && !listed)
-                k_partial_fluxes_scan<<<rb_grid(D), RB_THREADS, 0, ctx->st>>>(D, G, S, ctx->flo, ctx->fhi);
+                launch_after(k_partial_fluxes_scan, rb_grid(D), RB_THREADS, 0, ctx->st, D, G, S, ctx->flo, ctx->fhi);
             else
-                k_partial_fluxes<<<kFluxBlocks, 32, 0, ctx->st>>>(D, G, S, ctx->part[sw & 1], ctx->npart + sw, ctx->flo,
+                launch_after(k_partial_fluxes, kFluxBlocks, 32, 0, ctx->st, D, G, S, ctx->part[sw & 1], ctx->npart + sw, ctx->flo,
                                                                   ctx->fhi);
             T.after();
             if ((rc = launch_check(ctx, "k_partial_fluxes")) != SCF_OK) return rc;
             T.before(1);
             if (ax == 0) {
                 const int bx = line_threads(D.I, SW_X), by = SW_X / bx;
-                (s ? k_sweep_x<true> : k_sweep_x<false>)<<<dim3((D.I + bx - 1) / bx, (D.J + by - 1) / by, D.K),
-                                                           dim3(bx, by), 0, ctx->st>>>(
+                launch_after(s ? k_sweep_x<true> : k_sweep_x<false>, dim3((D.I + bx - 1) / bx, (D.J + by - 1) / by, D.K), dim3(bx, by), 0, ctx->st, 
                     D, G, S, ctx->flo, ctx->fhi, ctx->vf[out], ctx->ls[out], list, count);
             } else {
                 const int bx = line_threads(D.I, NX), by = NX / bx, n = D.len(ax);
@@ -674,7 +683,7 @@ int scheme_step(scf_clsvof_ctx *ctx, bool listed, int &launches, Timer &T)
                 g.z = (n + len - 1) / len;
                 auto *kernel = ax == 1 ? (s ? k_sweep_yz<1, true> : k_sweep_yz<1, false>)
                                        : (s ? k_sweep_yz<2, true> : k_sweep_yz<2, false>);
-                kernel<<<g, dim3(bx, by), 0, ctx->st>>>(D, G, S, ctx->flo, ctx->fhi, ctx->vf[out], ctx->ls[out], list, count,
+                launch_after(kernel, g, dim3(bx, by), 0, ctx->st, D, G, S, ctx->flo, ctx->fhi, ctx->vf[out], ctx->ls[out], list, count,
                                               len);
             }
             T.after();
@@ -702,7 +711,7 @@ int scheme_step(scf_clsvof_ctx *ctx, bool listed, int &launches, Timer &T)
             W.vof_const[f] = ctx->vof_const[f];
         }
         T.before(2);
-        k_walls<<<dim3(blocks_for(pmax), 3), NT, 0, ctx->st>>>(D, G, W);
+        launch_after(k_walls, dim3(blocks_for(pmax), 3), NT, 0, ctx->st, D, G, W);
         T.after();
         if ((rc = launch_check(ctx, "k_walls")) != SCF_OK) return rc;
         const uint32_t *list = ctx->part[(3 * kk) & 1];
@@ -712,22 +721,22 @@ int scheme_step(scf_clsvof_ctx *ctx, bool listed, int &launches, Timer &T)
         O.key = ctx->key; O.fix = ctx->fix; O.cls = ctx->cls; O.ub = ctx->ub;
         const unsigned nb = kNormalBlocks + (unsigned)std::min<size_t>((size_t)D.J * D.K, 152 * 32);
         T.before(0);
-        k_normals<<<nb, NB_THREADS, 0, ctx->st>>>(D, G, ctx->vf[0], ctx->ls[0], O, list, count);
+        launch_after(k_normals, nb, NB_THREADS, 0, ctx->st, D, G, ctx->vf[0], ctx->ls[0], O, list, count);
         T.after();
         if ((rc = launch_check(ctx, "k_normals")) != SCF_OK) return rc;
         T.before(3);
-        k_band_bound<<<kBandBlocks, BP_THREADS, 0, ctx->st>>>(D, G, ctx->vf[0], ctx->nxl, ctx->nyl, ctx->nzl, ctx->dis,
+        launch_after(k_band_bound, kBandBlocks, BP_THREADS, 0, ctx->st, D, G, ctx->vf[0], ctx->nxl, ctx->nyl, ctx->nzl, ctx->dis,
                                                               ctx->cls, list, count, ctx->ub, ctx->fix);
         T.after();
         if ((rc = launch_check(ctx, "k_band_bound")) != SCF_OK) return rc;
         T.before(3);
-        k_band_pairs<<<kBandBlocks, BP_THREADS, 0, ctx->st>>>(D, G, ctx->vf[0], ctx->ls[0], ctx->nxl, ctx->nyl,
+        launch_after(k_band_pairs, kBandBlocks, BP_THREADS, 0, ctx->st, D, G, ctx->vf[0], ctx->ls[0], ctx->nxl, ctx->nyl,
                                                               ctx->nzl, ctx->dis, ctx->cls, list, count, ctx->ub,
                                                               ctx->key, ctx->fix);
         T.after();
         if ((rc = launch_check(ctx, "k_band_pairs")) != SCF_OK) return rc;
         T.before(3);
-        k_band_value<<<gin, NX, 0, ctx->st>>>(D, G, ctx->vf[0], ctx->dis, ctx->key, ctx->fix, ctx->ls[0]);
+        launch_after(k_band_value, gin, NX, 0, ctx->st, D, G, ctx->vf[0], ctx->dis, ctx->key, ctx->fix, ctx->ls[0]);
         T.after();
         if ((rc = launch_check(ctx, "k_band_value")) != SCF_OK) return rc;
         launches += 5;
