@@ -163,15 +163,11 @@ __device__ __forceinline__ void pass_end(A (&v)[red_sums(KIND)], const Red &R)
             for (int w = 0; w < NT / 32; ++w) a += sh[w][q];
             R.partials[4 * blk + q] = a;
         }
-        if (LAST) {
-            __threadfence();
-            last = atomicAdd(R.finished, 1u) == (unsigned)nb - 1u;
-        }
+        if (LAST) last = count_in(R.finished) == (unsigned)nb - 1u;
     }
     if constexpr (LAST) {
         __syncthreads();
         if (!last) return;
-        __threadfence();
         if (tid == 0) *R.finished = 0;
         red_tail<KIND>(R, nb);
     }

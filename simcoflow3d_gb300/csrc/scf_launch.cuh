@@ -37,3 +37,13 @@ inline cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, siz
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+
+// Counts a block in, by one thread after its block's results: the block that
+// gets the last count may read all the others' (release of its own, acquire
+// of theirs; a block barrier extends both to the other threads).
+__device__ __forceinline__ unsigned count_in(unsigned *counter)
+{
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(counter) : "memory");
+    return old;
+}

@@ -93,7 +93,6 @@ __device__ __forceinline__ void red_tail(const RedOut &o, int nb)
     constexpr int mail = KIND == RK_RR ? MAIL_RR : KIND == RK_RESIDUAL ? MAIL_RESIDUAL : KIND == RK_BB ? MAIL_BB : -1;
     if (mail >= 0 && t == 0) {
         *(volatile double *)(o.mail + (mail >= 0 ? mail : 0) * MAIL_STRIDE) = v[0];
-        __threadfence_system();
     }
     // lanes 0 and 1 form the two quotients of a kind in one division
     if constexpr (KIND == RK_ALPHA) {
@@ -139,13 +138,9 @@ __device__ __forceinline__ void red_end(const RedOut &o, double (&v)[red_sums(KI
     if constexpr (LAST) {
         __shared__ int last;
         const int nb = (int)(gridDim.x * gridDim.y * gridDim.z);
-        if (thread_linear() == 0) {
-            __threadfence();
-            last = atomicAdd(o.done, 1u) == (unsigned)nb - 1u;
-        }
+        if (thread_linear() == 0) last = count_in(o.done) == (unsigned)nb - 1u;
         __syncthreads();
         if (!last) return;
-        __threadfence();
         if (thread_linear() == 0) *o.done = 0;
         red_tail<KIND>(o, nb);
     }
