@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(128) k_pocoef(AsmArgs a)
 __global__ void __launch_bounds__(128) k_pocoef_groups(AsmArgs a, int ncol, int ngrp)
 {
     after_previous();
+    if (*a.stale_count == 0) return;
     const int g = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (g >= ngrp) return;
     const int c0 = g * 64;
@@ -291,32 +292,33 @@ __global__ void __launch_bounds__(128) k_pocoef_groups(AsmArgs a, int ncol, int 
 
 // Head cells: the carried value comes from the latest earlier segment (first
 // within the cell's group, then whole groups) that assigned the stream.
-__global__ void k_pocoef_heads(AsmArgs a, unsigned count)
+__global__ void k_pocoef_heads(AsmArgs a)
 {
     after_previous();
-    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
+    const unsigned count = min(*a.stale_count, a.stale_cap);
     const Dims &d = a.d;
-    const long long e = a.stale_list[t];
-    const int s = (int)(e & 15);
-    const int f = s >> 1;
-    const long long L = e >> 4;
-    const int col = (int)(L / d.K), k = (int)(L % d.K) + 1;
-    const int i = col / d.J + 1, j = col % d.J + 1;
-    const int nsk = (d.K + a.kseg - 1) / a.kseg;
-    const int seg = col * nsk + (k - 1) / a.kseg;
-    const unsigned bit = 1u << s;
-    double beta = a.stale_init;
-    bool found = false;
-    const int g = seg / 64;
-    for (int c = seg - 1; c >= g * 64; --c)
-        if (a.col_mask[c] & bit) { beta = a.col_val[(long long)c * 12 + s]; found = true; break; }
-    if (!found)
-        for (int q = g - 1; q >= 0; --q)
-            if (a.grp_mask[q] & bit) { beta = a.grp_val[(long long)q * 12 + s]; break; }
-    double dp, dg;
-    face_terms(a, f, i, j, k, dp, dg);
-    a.pocoef[nidx(d, i, j, k) + (long long)d.n * f] = coef_expr(dp, dg, a.betap, a.betam, beta);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+        const long long e = a.stale_list[t];
+        const int s = (int)(e & 15);
+        const int f = s >> 1;
+        const long long L = e >> 4;
+        const int col = (int)(L / d.K), k = (int)(L % d.K) + 1;
+        const int i = col / d.J + 1, j = col % d.J + 1;
+        const int nsk = (d.K + a.kseg - 1) / a.kseg;
+        const int seg = col * nsk + (k - 1) / a.kseg;
+        const unsigned bit = 1u << s;
+        double beta = a.stale_init;
+        bool found = false;
+        const int g = seg / 64;
+        for (int c = seg - 1; c >= g * 64; --c)
+            if (a.col_mask[c] & bit) { beta = a.col_val[(long long)c * 12 + s]; found = true; break; }
+        if (!found)
+            for (int q = g - 1; q >= 0; --q)
+                if (a.grp_mask[q] & bit) { beta = a.grp_val[(long long)q * 12 + s]; break; }
+        double dp, dg;
+        face_terms(a, f, i, j, k, dp, dg);
+        a.pocoef[nidx(d, i, j, k) + (long long)d.n * f] = coef_expr(dp, dg, a.betap, a.betam, beta);
+    }
 }
 
 // Boundary planes take the neighbouring plane (ProjectionP.f90:256-264).
@@ -620,7 +622,7 @@ __global__ void __launch_bounds__(OP_THREADS, 3) k_operator(AsmArgs a, OpArgs o)
 // ---------------------------------------------------------------------------
 // host launchers
 int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double *rho, double rho_ref,
-                    cudaStream_t st, unsigned *stale_count_host, int *launches)
+                    cudaStream_t st, int *launches)
 {
     const Dims &d = a.d;
     cudaMemsetAsync(a.stale_count, 0, sizeof(unsigned), st);
@@ -628,22 +630,16 @@ int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double 
         k_phase<<<2 * 152 * 8, 256, 0, st>>>(a);
         launch_pocoef_rho(a, rho, rho_ref, st, launches);
         *launches += 1;
-        *stale_count_host = 0;
     } else {
         dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + a.kseg - 1) / a.kseg);
         k_phase<<<2 * 152 * 8, 256, 0, st>>>(a);
         launch_after(k_pocoef, g, b, 0, st, a);
-        *launches += 2;
-        cudaMemcpyAsync(stale_count_host, a.stale_count, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-        cudaStreamSynchronize(st);
-    }
-    unsigned cnt = *stale_count_host;
-    if (cnt > a.stale_cap) cnt = a.stale_cap;
-    if (cnt) {
+        // (the count stays on the device: a host that read it here to skip
+        // these two would cost the GPU a round trip)
         const int ncol = d.I * d.J * ((d.K + a.kseg - 1) / a.kseg), ngrp = (ncol + 63) / 64;
         launch_after(k_pocoef_groups, (ngrp + 3) / 4, 128, 0, st, a, ncol, ngrp);
-        launch_after(k_pocoef_heads, (cnt + 127) / 128, 128, 0, st, a, cnt);
-        *launches += 2;
+        launch_after(k_pocoef_heads, 152 * 4, 128, 0, st, a);
+        *launches += 4;
     }
     {
         int m = d.J * d.K;

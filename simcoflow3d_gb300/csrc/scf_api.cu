@@ -339,8 +339,7 @@ int assemble(scf_ctx *ctx)
     o.diag_lo = ctx->diag_lo; o.cE_lo = ctx->cE_lo; o.cN_lo = ctx->cN_lo; o.cT_lo = ctx->cT_lo;
     o.extra32 = ctx->extra32;
     const double rho_ref = ctx->opts.rho_ref > 0.0 ? ctx->opts.rho_ref : ctx->opts.rho_l;
-    int e = launch_assemble(a, o, mixed, ctx->use_rho ? ctx->adj_rho : nullptr, rho_ref, ctx->st, ctx->h_u32,
-                            &ctx->launches);
+    int e = launch_assemble(a, o, mixed, ctx->use_rho ? ctx->adj_rho : nullptr, rho_ref, ctx->st, &ctx->launches);
     if (e) { set_err(ctx, "assembly launch: %s", cudaGetErrorString((cudaError_t)e)); return SCF_ERR_CUDA; }
     rc = check_flags(ctx);
     if (rc) return rc;

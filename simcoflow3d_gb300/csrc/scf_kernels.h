@@ -53,7 +53,7 @@ struct OpArgs {
 // rho: per-cell densities (ghosted) or nullptr for the reference's two-phase
 // coefficients.
 int launch_assemble(const AsmArgs &a, const OpArgs &o, bool mixed, const double *rho, double rho_ref,
-                    cudaStream_t st, unsigned *stale_count_host, int *launches);
+                    cudaStream_t st, int *launches);
 
 // ---- solver --------------------------------------------------------------
 template <typename T>
