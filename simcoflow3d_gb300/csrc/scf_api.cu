@@ -1039,10 +1039,12 @@ int scf_ctx_create(scf_ctx **out, int32_t imax, int32_t jmax, int32_t kmax, cons
     for (int q = 0; q < 6; ++q) A(ctx->bvar[q], plane_size(d, q));
     A(ctx->pocoef, 6 * n);
     A(ctx->stale_count, 1); A(ctx->flags, 4);
-    ctx->stale_cap = (unsigned)(n < (1LL << 30) ? n : (1LL << 30));
-    A(ctx->stale_list, ctx->stale_cap);
-    // per-segment summaries of the coefficient kernel
+    // per-segment summaries of the coefficient kernel; shorter segments list
+    // more of their first cells (at most every face)
     const int kseg = asm_kseg(imax, jmax, kmax);
+    const long long listed = kseg < 32 ? 6LL * n : n;
+    ctx->stale_cap = (unsigned)(listed < (1LL << 30) ? listed : (1LL << 30));
+    A(ctx->stale_list, ctx->stale_cap);
     const long long ncol = (long long)imax * jmax * ((kmax + kseg - 1) / kseg), ngrp = (ncol + 63) / 64;
     A(ctx->col_val, 12 * ncol); A(ctx->col_mask, ncol); A(ctx->grp_val, 12 * ngrp); A(ctx->grp_mask, ngrp);
     A(ctx->phase, ng);
