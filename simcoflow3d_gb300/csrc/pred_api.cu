@@ -69,6 +69,8 @@ void mom_err(scf_mom_ctx *c, const char *fmt, ...)
         }                                                                                   \
     } while (0)
 
+// Zeroed on the context's own stream: the legacy stream does not order before
+// its non-blocking ones, and may have the caller's work queued.
 template <typename P>
 int malloc0(scf_mom_ctx *ctx, P **ptr, size_t count)
 {
@@ -80,7 +82,7 @@ int malloc0(scf_mom_ctx *ctx, P **ptr, size_t count)
         return SCF_ERR_OUT_OF_MEMORY;
     }
     ctx->mem.push_back(p);
-    if (cudaMemset(p, 0, bytes) != cudaSuccess) return SCF_ERR_CUDA;
+    if (cudaMemsetAsync(p, 0, bytes, ctx->st) != cudaSuccess) return SCF_ERR_CUDA;
     *ptr = (P *)p;
     return SCF_OK;
 }
@@ -375,6 +377,7 @@ extern "C" int scf_mom_create(scf_mom_ctx **out, int32_t imax, int32_t jmax, int
     if (cudaMallocHost(&ctx->sc_host, sizeof(BcgScalars)) != cudaSuccess) return fail(SCF_ERR_OUT_OF_MEMORY);
     if (cudaMallocHost(&ctx->counts_host, 2 * sizeof(unsigned long long)) != cudaSuccess)
         return fail(SCF_ERR_OUT_OF_MEMORY);
+    if (cudaStreamSynchronize(ctx->st) != cudaSuccess) return fail(SCF_ERR_CUDA);   // the zeros, before any stream's work
     *out = ctx;
     return SCF_OK;
 }

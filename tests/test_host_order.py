@@ -1,0 +1,50 @@
+"""What the library's host code leaves unfinished on the GPU when a call returns,
+and the order in which it gives work to its streams, over a stand-in CUDA
+runtime (fake_cuda.h).  CPU only."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "simcoflow3d_gb300", "csrc")
+
+
+def build(tmp, name):
+    from simcoflow3d_gb300 import build as B
+    try:
+        nvcc = B.nvcc()
+    except RuntimeError:
+        pytest.skip("nvcc not found")
+    lib = os.path.join(str(tmp), name + ".so")
+    # only the calls that a path reaches are defined, so the rest is bound lazily
+    cmd = [nvcc, "-O1", "-std=c++17", "-shared", "-cudart", "none", *B.ARCH, "--expt-relaxed-constexpr", "-Xcompiler",
+           "-fPIC", "-I" + CSRC, "-I" + HERE, os.path.join(HERE, name + ".cu"), os.path.join(HERE, "fake_cuda.cpp"),
+           "-o", lib, "-Xlinker", "-z", "-Xlinker", "lazy", "-lpthread"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return lib
+
+
+def run(lib, *args):
+    """The words that the library's `scenario` prints, in a process of its own."""
+    code = ("import ctypes as C, sys\n"
+            "args = [a.encode() for a in sys.argv[2:]]\n"
+            "dl = C.CDLL(None)\n"
+            "dl.dlopen.restype = dl.dlsym.restype = C.c_void_p\n"
+            "dl.dlsym.argtypes = [C.c_void_p, C.c_char_p]\n"
+            "h = dl.dlopen(sys.argv[1].encode(), 1)\n"   # RTLD_LAZY
+            "f = C.CFUNCTYPE(None, C.c_char_p)(dl.dlsym(h, b'scenario'))\n"
+            "f(args[0] if args else b'')\n")
+    r = subprocess.run([sys.executable, "-c", code, lib, *args], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
+    return r.stdout.split()
+
+
+def test_predictor_create_leaves_nothing_to_other_streams(tmp_path):
+    """The counter that tells a pass's last block, and every other zeroed buffer,
+    before any of the context's three streams can use it."""
+    rc, left = run(build(tmp_path, "host_predictor"))
+    assert rc == "0" and left == "0"
