@@ -132,6 +132,8 @@ void set_err(scf_ctx *c, const char *fmt, ...)
         }                                                                                  \
     } while (0)
 
+// Zeroed on the context's own stream: the legacy stream does not order before
+// its non-blocking ones, and may have the caller's work queued.
 template <typename P>
 int dalloc(scf_ctx *ctx, DevBuf &mem, P **ptr, size_t count)
 {
@@ -143,8 +145,8 @@ int dalloc(scf_ctx *ctx, DevBuf &mem, P **ptr, size_t count)
         set_err(ctx, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
         return SCF_ERR_OUT_OF_MEMORY;
     }
-    cudaMemset(p, 0, bytes);
     mem.ptrs.push_back(p);
+    CK(cudaMemsetAsync(p, 0, bytes, ctx->st));
     *ptr = (P *)p;
     return SCF_OK;
 }
@@ -267,7 +269,8 @@ int ensure_mg(scf_ctx *ctx)
             for (int i = 1; i <= c0; ++i) hmap.push_back(i + sy * j + sz * k);
     DALLOC(ctx->mgmem, ctx->map, hmap.size());
     DALLOC(ctx->mgmem, ctx->ainv, (size_t)ctx->ncoarse * ctx->ncoarse);
-    CK(cudaMemcpy(ctx->map, hmap.data(), hmap.size() * sizeof(int), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(ctx->map, hmap.data(), hmap.size() * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
+    CK(cudaStreamSynchronize(ctx->st));   // (hmap goes away)
     ctx->mg_precision = prec;
     return SCF_OK;
 }
@@ -1028,6 +1031,7 @@ int scf_ctx_create(scf_ctx **out, int32_t imax, int32_t jmax, int32_t kmax, cons
     d.gx = imax + 2; d.gy = jmax + 2; d.gz = kmax + 2;
     d.ng = (int)ng; d.n = (int)n;
     auto fail = [&](int code) { scf_ctx_destroy(ctx); return code; };
+    if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) return fail(SCF_ERR_CUDA);
 #define A(ptr, cnt) do { if ((rc = dalloc(ctx, ctx->mem, &(ptr), (size_t)(cnt)))) return fail(rc); } while (0)
     A(ctx->pdx, n); A(ctx->pdy, n); A(ctx->pdz, n); A(ctx->udx, n); A(ctx->vdy, n); A(ctx->wdz, n);
     A(ctx->phil, ng); A(ctx->vofl, ng); A(ctx->vof, ng); A(ctx->ee, ng); A(ctx->ne, ng); A(ctx->te, ng);
@@ -1060,7 +1064,6 @@ int scf_ctx_create(scf_ctx **out, int32_t imax, int32_t jmax, int32_t kmax, cons
     A(ctx->R.scal, S_NUM);
     A(ctx->R.done, 1);
 #undef A
-    if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) return fail(SCF_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&ctx->cst, cudaStreamNonBlocking) != cudaSuccess) return fail(SCF_ERR_CUDA);
     if (cudaEventCreateWithFlags(&ctx->corr_ready, cudaEventDisableTiming) != cudaSuccess) return fail(SCF_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&ctx->ist, cudaStreamNonBlocking) != cudaSuccess) return fail(SCF_ERR_CUDA);

@@ -1,0 +1,104 @@
+// The projection's host code (scf_api.cu) over a stand-in CUDA runtime, with
+// launchers that give work to their stream and form the sums the host waits for.
+#include "fake_cuda.h"
+#include "scf_kernels.h"
+
+#include <cstdio>
+#include <sched.h>
+
+namespace {
+double rhs_sum = 4.0, step_sum = 0.0;     // (b, b), and (r, r) after a CG step
+std::vector<double> residuals;            // (r, r) of each residual, in order
+std::vector<std::function<void()>> in_flight;   // sums on their way to the host
+
+void land()
+{
+    for (auto &f : in_flight) f();
+    in_flight.clear();
+}
+void mailed(Reducer &R, Mail m, int slot, double v)
+{
+    R.scal[slot] = v;
+    if (R.mail) in_flight.push_back([=] { R.mail[m * MAIL_STRIDE] = v; });
+}
+}  // namespace
+
+extern "C" int sched_yield()
+{
+    ++fake::yields;
+    return 0;
+}
+
+void rhs_prologue(const LevelView<double> &, const unsigned char *, double *, bool, Reducer &R, cudaStream_t st, int *)
+{
+    fake::work("rhs", st);
+    mailed(R, MAIL_BB, S_BB, rhs_sum);
+}
+void final_residual(const LevelView<double> &, const unsigned char *, const double *, const double *, double *, bool,
+                    Reducer &R, cudaStream_t st, int *)
+{
+    fake::work("residual", st);
+    const double v = residuals.front();
+    residuals.erase(residuals.begin());
+    mailed(R, MAIL_RESIDUAL, S_RR, v);
+}
+template <>
+void mg_coarsen<double>(const MgLevel<double> &, MgLevel<double> &, cudaStream_t st, int *) { fake::work("coarsen", st); }
+template <>
+void mg_coarse_inverse<double>(const MgLevel<double> &, double *, int *, int, bool, cudaStream_t st, int *)
+{
+    fake::work("inverse", st);
+}
+template <>
+double *mg_vcycle<double>(MgLevel<double> *L, int, const ChebCoef &, const double *, const int *, int, bool, bool,
+                          cudaStream_t st, int *, KTimer *, cudaEvent_t ready)
+{
+    if (ready) cudaStreamWaitEvent(st, ready, 0);
+    fake::work("vcycle", st);
+    return L[0].xb;
+}
+template <>
+void cg_dot_rz<double>(const LevelView<double> &, const double *, const double *, const double *, Reducer &,
+                       cudaStream_t st, int *) { fake::work("dot", st); }
+template <>
+void cg_pupdate<double>(const LevelView<double> &, const double *, double *, const double *, bool, cudaStream_t st, int *)
+{
+    fake::work("p", st);
+}
+void cg_spmv_dot(const LevelView<double> &, const double *, double *, Reducer &, bool, cudaStream_t st, int *, KTimer *)
+{
+    fake::work("spmv", st);
+}
+template <>
+void cg_update<double>(const LevelView<double> &, double *, double *, const double *, const double *, double *,
+                       const LevelView<double> &, double *, double, Reducer &R, cudaStream_t st, int *, KTimer *)
+{
+    fake::work("update", st);
+    mailed(R, MAIL_RR, S_RR, step_sum);
+}
+cudaError_t coarse_cycle_attr() { return cudaSuccess; }
+cudaError_t pair_smem_attr() { return cudaSuccess; }
+int smoother_pairs_state() { return 1; }
+
+#include "scf_api.cu"   // after the specialisations
+
+extern "C" void scenario(const char *name)
+{
+    const std::string what = name;
+    fake::on_query = fake::on_wait = land;
+    scf_opts o;
+    scf_opts_default(&o);
+    o.warm_start = what == "warm";
+    o.coarse_max_cells = 8;
+    scf_ctx *ctx = nullptr;
+    if (scf_ctx_create(&ctx, 6, 5, 4, &o) != SCF_OK) return;
+    for (int q = 0; q < 6; ++q) ctx->bcp_flag[q] = 0;
+    scf_stats st{};
+    if (what == "replan") {   // zeroed buffers of a new plan and of the adjoint
+        o.coarse_max_cells = 16;
+        fake::outstanding.clear();
+        const int rc = scf_ctx_set_opts(ctx, &o), rc2 = ensure_adj(ctx);
+        std::printf("%d %d %d\n", rc, rc2, fake::left(nullptr));
+    }
+    std::fflush(stdout);
+}

@@ -48,3 +48,14 @@ def test_predictor_create_leaves_nothing_to_other_streams(tmp_path):
     before any of the context's three streams can use it."""
     rc, left = run(build(tmp_path, "host_predictor"))
     assert rc == "0" and left == "0"
+
+
+@pytest.fixture(scope="module")
+def projection(tmp_path_factory):
+    return build(tmp_path_factory.mktemp("host"), "host_projection")
+
+
+def test_projection_buffers_are_zeroed_on_its_own_stream(projection):
+    """Those made after the context (a new plan, the adjoint's) too: nothing is
+    left to the legacy stream, which its streams do not order after."""
+    assert run(projection, "replan") == ["0", "0", "0"]
