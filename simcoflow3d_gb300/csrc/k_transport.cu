@@ -744,6 +744,8 @@ int scheme_step(scf_clsvof_ctx *ctx, bool listed, int &launches, Timer &T)
     return SCF_OK;
 }
 
+// Zeroed on the context's stream: the legacy stream does not order before it,
+// and may have the caller's work queued.
 template <typename P>
 int alloc(scf_clsvof_ctx *ctx, P **ptr, size_t count)
 {
@@ -756,7 +758,7 @@ int alloc(scf_clsvof_ctx *ctx, P **ptr, size_t count)
     }
     ctx->mem.push_back(p);
     *ptr = (P *)p;
-    return cudaMemset(p, 0, bytes) == cudaSuccess ? SCF_OK : SCF_ERR_CUDA;
+    return cudaMemsetAsync(p, 0, bytes, ctx->st) == cudaSuccess ? SCF_OK : SCF_ERR_CUDA;
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b)

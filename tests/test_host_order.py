@@ -59,3 +59,8 @@ def test_projection_buffers_are_zeroed_on_its_own_stream(projection):
     """Those made after the context (a new plan, the adjoint's) too: nothing is
     left to the legacy stream, which its streams do not order after."""
     assert run(projection, "replan") == ["0", "0", "0"]
+
+
+def test_transport_buffers_are_zeroed_on_its_own_stream(tmp_path):
+    """A zero fill on the legacy stream could land on fields staged meanwhile."""
+    assert run(build(tmp_path, "host_transport")) == ["0", "0"]
