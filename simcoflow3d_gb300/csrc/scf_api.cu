@@ -617,6 +617,15 @@ void run_iteration(scf_ctx *ctx, MgLevel<T> *L, const ChebCoef &cc, bool singula
     iteration_kernels<T>(ctx, L, cc, singular);
 }
 
+// An error that ends a solve, with nothing of it left on the GPU: the sums that
+// the host waits for arrive ahead of the kernels queued behind them.
+int drained(scf_ctx *ctx, int rc)
+{
+    cudaStreamSynchronize(ctx->st);
+    cudaStreamSynchronize(ctx->ist);
+    return rc;
+}
+
 // Iterations without a new smallest CG residual after which a round of the
 // solve ends (the tolerance is below what FP64 can reach for the system).
 constexpr int kStallWindow = 50;
@@ -634,10 +643,7 @@ int solve_impl(scf_ctx *ctx, MgLevel<T> *L, scf_stats *stats)
     rhs_prologue(A, ctx->active, ctx->b, singular, ctx->R, ctx->st, &ctx->launches);
     {
         const int rh = build_hierarchy<T>(ctx, L);
-        if (rh) {
-            cudaStreamSynchronize(ctx->st);   // no sum is on its way when the next solve arms its mail
-            return rh;
-        }
+        if (rh) return drained(ctx, rh);
     }
     const double bb = await_mail(ctx, MAIL_BB, S_BB);
     const double bn = std::sqrt(bb);
@@ -653,7 +659,7 @@ int solve_impl(scf_ctx *ctx, MgLevel<T> *L, scf_stats *stats)
         stats->rounds = 1;
         stats->rel_residual = 0.0;
         stats->converged = 1;
-        return std::isfinite(bb) ? SCF_OK : SCF_ERR_NONFINITE;
+        return std::isfinite(bb) ? SCF_OK : drained(ctx, SCF_ERR_NONFINITE);
     }
     if (ctx->opts.warm_start && ctx->warm_ok) {
         final_residual(A, ctx->active, ctx->b, ctx->x, ctx->r, false, ctx->R, ctx->st, &ctx->launches);
@@ -697,7 +703,7 @@ int solve_impl(scf_ctx *ctx, MgLevel<T> *L, scf_stats *stats)
             if (!std::isfinite(rr)) {
                 set_err(ctx, "CG residual became non-finite at iteration %d", its);
                 stats->iterations = its;
-                return SCF_ERR_NONFINITE;
+                return drained(ctx, SCF_ERR_NONFINITE);
             }
             if (std::sqrt(rr) <= tol * bn) { conv = true; break; }
             // Below the rounding floor of the system (where the recursive
@@ -1329,7 +1335,7 @@ extern "C" int scf_loss_backward(scf_ctx *ctx, double *grad_u, double *grad_v, d
     else
         rc = solve_impl<float>(ctx, ctx->L32, stats);
     cudaEventRecord(ctx->ev[2], ctx->st);
-    if (rc) return rc;
+    if (rc) return drained(ctx, rc);
     // densities for the derivative: the given field or the phase densities
     if (!ctx->rho_given_last) fill_phase_density(ctx->phase, ctx->adj_rho, d.ng, ctx->opts.rho_l, ctx->opts.rho_g,
                                                  ctx->st, &ctx->launches);

@@ -100,5 +100,10 @@ extern "C" void scenario(const char *name)
         const int rc = scf_ctx_set_opts(ctx, &o), rc2 = ensure_adj(ctx);
         std::printf("%d %d %d\n", rc, rc2, fake::left(nullptr));
     }
+    if (what == "nonfinite_rhs" || what == "nonfinite_step") {   // what is left when the solve gives up
+        (what == "nonfinite_rhs" ? rhs_sum : step_sum) = std::nan("");
+        const int rc = solve_impl<double>(ctx, ctx->L64, &st);
+        std::printf("%d %d %d\n", rc == SCF_ERR_NONFINITE, fake::left(ctx->st), fake::left(ctx->ist));
+    }
     std::fflush(stdout);
 }

@@ -61,6 +61,12 @@ def test_projection_buffers_are_zeroed_on_its_own_stream(projection):
     assert run(projection, "replan") == ["0", "0", "0"]
 
 
+@pytest.mark.parametrize("where", ["nonfinite_rhs", "nonfinite_step"])
+def test_failed_solve_leaves_nothing_running(projection, where):
+    """Calls are synchronous, also those that end in an error."""
+    assert run(projection, where) == ["1", "0", "0"]
+
+
 def test_transport_buffers_are_zeroed_on_its_own_stream(tmp_path):
     """A zero fill on the legacy stream could land on fields staged meanwhile."""
     assert run(build(tmp_path, "host_transport")) == ["0", "0"]
