@@ -353,6 +353,10 @@ int assemble(scf_ctx *ctx)
 template <typename T>
 int build_hierarchy(scf_ctx *ctx, MgLevel<T> *L)
 {
+    if (ctx->inv_pending) {   // of a solve without a V-cycle (a zero right-hand side): it reads the levels
+        CK(cudaStreamSynchronize(ctx->ist));
+        ctx->inv_pending = false;
+    }
     for (int l = 0; l + 1 < ctx->nlev; ++l) mg_coarsen<T>(L[l], L[l + 1], ctx->st, &ctx->launches);
     CK(cudaEventRecord(ctx->inv_start, ctx->st));
     CK(cudaStreamWaitEvent(ctx->ist, ctx->inv_start, 0));

@@ -105,5 +105,20 @@ extern "C" void scenario(const char *name)
         const int rc = solve_impl<double>(ctx, ctx->L64, &st);
         std::printf("%d %d %d\n", rc == SCF_ERR_NONFINITE, fake::left(ctx->st), fake::left(ctx->ist));
     }
+    if (what == "zero_rhs") {   // a solve without a V-cycle, then one with: the levels wait for the first inverse
+        rhs_sum = 0.0;
+        const int rc = solve_impl<double>(ctx, ctx->L64, &st);
+        fake::log.clear();
+        rhs_sum = 4.0;
+        residuals = {0.0};
+        const int rc2 = solve_impl<double>(ctx, ctx->L64, &st);
+        const std::string joined = "sync " + std::to_string((uintptr_t)ctx->ist);
+        size_t wait = fake::log.size(), coarsen = wait;
+        for (size_t q = fake::log.size(); q-- > 0;) {
+            if (fake::log[q] == joined) wait = q;
+            if (fake::log[q].compare(0, 7, "coarsen") == 0) coarsen = q;
+        }
+        std::printf("%d %d %d\n", rc, rc2, wait < coarsen);
+    }
     std::fflush(stdout);
 }

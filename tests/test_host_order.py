@@ -67,6 +67,12 @@ def test_failed_solve_leaves_nothing_running(projection, where):
     assert run(projection, where) == ["1", "0", "0"]
 
 
+def test_hierarchy_waits_for_the_inverse_before_it(projection):
+    """A zero right-hand side ends a solve with the coarsest inverse still
+    reading the levels on its own stream."""
+    assert run(projection, "zero_rhs") == ["0", "0", "1"]
+
+
 def test_transport_buffers_are_zeroed_on_its_own_stream(tmp_path):
     """A zero fill on the legacy stream could land on fields staged meanwhile."""
     assert run(build(tmp_path, "host_transport")) == ["0", "0"]
