@@ -407,8 +407,8 @@ double read_scal(scf_ctx *ctx, int slot)
 }
 
 // The sums that the host waits for come through pinned memory: arm_mail before
-// the launches that form one (the device has written every earlier one by
-// then, in stream order), await_mail after.  A copy and a synchronisation took
+// the launches that form one, await_mail after.  Every sum that is sent is
+// waited for, so none is on its way when its slot is armed again.  A copy and a synchronisation took
 // some 7 us longer per CG iteration (a 40^3 projection 1001 -> 924 us).  They
 // remain with the kernel timers on, whose events the host reads next, and
 // where the stream ends without a value (an error).
@@ -666,7 +666,9 @@ int solve_impl(scf_ctx *ctx, MgLevel<T> *L, scf_stats *stats)
         return std::isfinite(bb) ? SCF_OK : drained(ctx, SCF_ERR_NONFINITE);
     }
     if (ctx->opts.warm_start && ctx->warm_ok) {
-        final_residual(A, ctx->active, ctx->b, ctx->x, ctx->r, false, ctx->R, ctx->st, &ctx->launches);
+        Reducer unread = ctx->R;   // the host takes no sum here
+        unread.mail = nullptr;
+        final_residual(A, ctx->active, ctx->b, ctx->x, ctx->r, false, unread, ctx->st, &ctx->launches);
     } else {
         CK(cudaMemsetAsync(ctx->x, 0, sizeof(double) * ctx->d.ng, ctx->st));
         CK(cudaMemcpyAsync(ctx->r, ctx->b, sizeof(double) * ctx->d.ng, cudaMemcpyDeviceToDevice, ctx->st));

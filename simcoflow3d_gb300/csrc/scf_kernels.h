@@ -86,7 +86,7 @@ struct Reducer {
     double *scal;        // ScfScalar slots
     int max_blocks;
     unsigned *done;      // blocks of the running launch that have finished (0 between launches)
-    double *mail;        // pinned host memory: the sums that the host waits for, MAIL_STRIDE apart
+    double *mail;        // pinned host memory: the sums that the host waits for, MAIL_STRIDE apart; or nullptr
 };
 // (r, r) of the CG update, of a residual, and (b, b).
 enum Mail { MAIL_RR, MAIL_RESIDUAL, MAIL_BB, MAIL_NUM };

@@ -91,9 +91,7 @@ __device__ __forceinline__ void red_tail(const RedOut &o, int nb)
     if (t > 1) return;
     // to the waiting host without a copy of its own (scf_api.cu, await_mail)
     constexpr int mail = KIND == RK_RR ? MAIL_RR : KIND == RK_RESIDUAL ? MAIL_RESIDUAL : KIND == RK_BB ? MAIL_BB : -1;
-    if (mail >= 0 && t == 0) {
-        *(volatile double *)(o.mail + (mail >= 0 ? mail : 0) * MAIL_STRIDE) = v[0];
-    }
+    if (mail >= 0 && t == 0 && o.mail) *(volatile double *)(o.mail + (mail >= 0 ? mail : 0) * MAIL_STRIDE) = v[0];
     // lanes 0 and 1 form the two quotients of a kind in one division
     if constexpr (KIND == RK_ALPHA) {
         // alpha = (r, z) / (p, q); for an all-Neumann system also the mean of

@@ -73,6 +73,12 @@ def test_hierarchy_waits_for_the_inverse_before_it(projection):
     assert run(projection, "zero_rhs") == ["0", "0", "1"]
 
 
+def test_warm_start_reads_its_own_residual(projection):
+    """The residual a warm start begins with goes to no slot that the host reads
+    later: nothing fences its write against the one the host waits for."""
+    assert run(projection, "warm") == ["0", "1", "0"]
+
+
 def test_transport_buffers_are_zeroed_on_its_own_stream(tmp_path):
     """A zero fill on the legacy stream could land on fields staged meanwhile."""
     assert run(build(tmp_path, "host_transport")) == ["0", "0"]
