@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <chrono>
+#include <thread>
 #include <vector>
 #include "scf_kernels.h"
 #include "../../include/scf_projection.h"
@@ -101,6 +102,7 @@ struct scf_ctx {
     // host pinned scratch
     double *h_scal = nullptr;
     unsigned *h_u32 = nullptr;
+    unsigned schedule = 0;     // how the caller has the host wait (cudaDeviceSchedule*), read at each solve
     cudaEvent_t ev[8];
     int launches = 0;
     // loss and adjoint (allocated on first use)
@@ -410,8 +412,10 @@ double read_scal(scf_ctx *ctx, int slot)
 // the launches that form one, await_mail after.  Every sum that is sent is
 // waited for, so none is on its way when its slot is armed again.  A copy and a synchronisation took
 // some 7 us longer per CG iteration (a 40^3 projection 1001 -> 924 us).  They
-// remain with the kernel timers on, whose events the host reads next, and
-// where the stream ends without a value (an error).
+// remain with the kernel timers on, whose events the host reads next, for a
+// caller that asked for blocking synchronisation (cudaSetDeviceFlags), and
+// where the stream ends without a value (an error); one that asked for yielding
+// gets a yield between reads.
 constexpr unsigned long long MAIL_EMPTY = 0xfff4a9e1c0ffee11ull;   // a NaN that no sum gives
 
 void arm_mail(scf_ctx *ctx, Mail m)
@@ -421,7 +425,7 @@ void arm_mail(scf_ctx *ctx, Mail m)
 
 double await_mail(scf_ctx *ctx, Mail m, int slot)
 {
-    if (ctx->kt.on) return read_scal(ctx, slot);
+    if (ctx->kt.on || ctx->schedule == cudaDeviceScheduleBlockingSync) return read_scal(ctx, slot);
     volatile unsigned long long *box = (volatile unsigned long long *)(ctx->R.mail + m * MAIL_STRIDE);
     for (unsigned n = 1;; ++n) {
         const unsigned long long b = *box;
@@ -430,6 +434,7 @@ double await_mail(scf_ctx *ctx, Mail m, int slot)
             memcpy(&v, &b, sizeof v);
             return v;
         }
+        if (ctx->schedule == cudaDeviceScheduleYield) std::this_thread::yield();
         if (n % 4096 == 0 && cudaStreamQuery(ctx->st) != cudaErrorNotReady && *box == MAIL_EMPTY)
             return read_scal(ctx, slot);
     }
@@ -643,6 +648,9 @@ int solve_impl(scf_ctx *ctx, MgLevel<T> *L, scf_stats *stats)
     float *rlow = mixed ? (float *)L[0].b : nullptr;
     const ChebCoef cc = cheb_for(ctx);
     auto t0 = std::chrono::steady_clock::now();
+    unsigned flags = 0;
+    CK(cudaGetDeviceFlags(&flags));
+    ctx->schedule = flags & cudaDeviceScheduleMask;
     arm_mail(ctx, MAIL_BB);
     rhs_prologue(A, ctx->active, ctx->b, singular, ctx->R, ctx->st, &ctx->launches);
     {

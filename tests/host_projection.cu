@@ -141,5 +141,13 @@ extern "C" void scenario(const char *name)
         const int rc = solve_impl<double>(ctx, ctx->L64, &st);
         std::printf("%d %d %g\n", rc, (int)st.rounds, st.rel_residual);
     }
+    if (what == "spin" || what == "yield" || what == "block") {   // as the device's flags ask
+        fake::device_flags = what == "yield" ? cudaDeviceScheduleYield : what == "block" ? cudaDeviceScheduleBlockingSync
+                                                                                         : cudaDeviceScheduleSpin;
+        residuals = {0.0};
+        fake::waits = 0;
+        const int rc = solve_impl<double>(ctx, ctx->L64, &st);
+        std::printf("%d %d %d %d\n", rc, fake::queries > 0, fake::yields > 0, fake::waits > 0);
+    }
     std::fflush(stdout);
 }

@@ -22,7 +22,7 @@ def build(tmp, name):
     # only the calls that a path reaches are defined, so the rest is bound lazily
     cmd = [nvcc, "-O1", "-std=c++17", "-shared", "-cudart", "none", *B.ARCH, "--expt-relaxed-constexpr", "-Xcompiler",
            "-fPIC", "-I" + CSRC, "-I" + HERE, os.path.join(HERE, name + ".cu"), os.path.join(HERE, "fake_cuda.cpp"),
-           "-o", lib, "-Xlinker", "-z", "-Xlinker", "lazy", "-lpthread"]
+           "-o", lib, "-Xlinker", "-z", "-Xlinker", "lazy", "-Xlinker", "-Bsymbolic", "-lpthread"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     return lib
@@ -77,6 +77,12 @@ def test_warm_start_reads_its_own_residual(projection):
     """The residual a warm start begins with goes to no slot that the host reads
     later: nothing fences its write against the one the host waits for."""
     assert run(projection, "warm") == ["0", "1", "0"]
+
+
+@pytest.mark.parametrize("how,polls,yields,waits", [("spin", 1, 0, 0), ("yield", 1, 1, 0), ("block", 0, 0, 1)])
+def test_waiting_follows_the_device_flags(projection, how, polls, yields, waits):
+    """A caller that chose blocking or yielding synchronisation gets it."""
+    assert run(projection, how) == ["0", str(polls), str(yields), str(waits)]
 
 
 def test_transport_buffers_are_zeroed_on_its_own_stream(tmp_path):
