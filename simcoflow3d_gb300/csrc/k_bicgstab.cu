@@ -87,14 +87,41 @@ __device__ __forceinline__ void scalars(BcgScalars *sc, const double (&s)[red_su
     }
 }
 
-// Sums the partials of nb blocks with 128 threads: 1024 strided sums, eight
-// per thread, then a tree over their index (512, 256, ... 1 apart), whose
-// first three levels are the thread's own.
+// The grid's sums from 1024 strided ones, a[q][j] of thread t < 128 being the
+// one that starts at block t + 128 j: a tree over their index (512, 256, ...
+// 1 apart), whose first three levels are the thread's own.
+template <int KIND>
+__device__ __forceinline__ void red_tree(const Red &R, double (&a)[red_sums(KIND)][8], int t)
+{
+    constexpr int Q = red_sums(KIND);
+    __shared__ double sh[Q][NT];
+    if (t < NT) {
+#pragma unroll
+        for (int d = 4; d > 0; d >>= 1)
+#pragma unroll
+            for (int q = 0; q < Q; ++q)
+#pragma unroll
+                for (int j = 0; j < d; ++j) a[q][j] += a[q][j + d];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) sh[q][t] = a[q][0];
+    }
+    __syncthreads();
+    if (t >= 32) return;
+    double s[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        s[q] = (sh[q][t] + sh[q][t + 64]) + (sh[q][t + 32] + sh[q][t + 96]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
+    }
+    scalars<KIND>(R.sc, s, R.want_bb);   // (s is the sums in lane 0)
+}
+
+// Sums the partials of nb blocks with 128 threads, eight strided sums each.
 template <int KIND>
 __device__ __forceinline__ void red_tail(const Red &R, int nb)
 {
     constexpr int Q = red_sums(KIND);
-    __shared__ double sh[Q][NT];
     const int t = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
     double a[Q][8];
 #pragma unroll
@@ -115,24 +142,7 @@ __device__ __forceinline__ void red_tail(const Red &R, int nb)
 #pragma unroll
                 for (int q = 0; q < Q; ++q) a[q][j] += p[q][j];
     }
-#pragma unroll
-    for (int d = 4; d > 0; d >>= 1)
-#pragma unroll
-        for (int q = 0; q < Q; ++q)
-#pragma unroll
-            for (int j = 0; j < d; ++j) a[q][j] += a[q][j + d];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) sh[q][t] = a[q][0];
-    __syncthreads();
-    if (t >= 32) return;
-    double s[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        s[q] = (sh[q][t] + sh[q][t + 64]) + (sh[q][t + 32] + sh[q][t + 96]);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
-    }
-    scalars<KIND>(R.sc, s, R.want_bb);   // (s is the sums in lane 0)
+    red_tree<KIND>(R, a, t);
 }
 
 // The end of a pass: the block's sums to its partials, and with LAST the
@@ -173,12 +183,54 @@ __device__ __forceinline__ void pass_end(A (&v)[red_sums(KIND)], const Red &R)
     }
 }
 
+// The sums of a grid of many blocks, in a launch of one block with a strided
+// sum per thread: the additions of red_tail in its order, with the partials'
+// loads spread over eight times the warps.  One / two sums back to back, by 128
+// threads and by 1024: 3.0 / 5.1 us and 3.3 / 5.0 at 1344 blocks, 6.7 / 14.6 and
+// 4.8 / 8.1 at 8192, where a predictor step (256^3 mixed) takes 38.9 ms, 43.5
+// before.
 template <int KIND>
-__global__ void __launch_bounds__(NT) k_red(Red R, int nb)
+__global__ void __launch_bounds__(8 * NT) k_red(Red R, int nb)
 {
     after_previous();
     if (KIND != BR_RESID && R.sc->done) return;
-    red_tail<KIND>(R, nb);
+    constexpr int Q = red_sums(KIND), U = 4;
+    __shared__ double strided[Q][8 * NT];
+    const int t = threadIdx.x;
+    double v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = 0.0;
+    for (int e = t; e < nb; e += U * 8 * NT) {
+        double p[U][Q];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const int b = e + u * 8 * NT;
+                p[u][q] = b < nb ? __ldcg(R.partials + 4 * (long long)b + q) : 0.0;
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (e - t + u * 8 * NT < nb)
+#pragma unroll
+                for (int q = 0; q < Q; ++q) v[q] += p[u][q];
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) strided[q][t] = v[q];
+    __syncthreads();
+    double a[Q][8];
+    if (t < NT)
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) a[q][j] = strided[q][t + NT * j];
+    red_tree<KIND>(R, a, t);
+}
+
+template <int KIND>
+void sum_blocks(const Red &R, int nb, cudaStream_t st)
+{
+    launch_after(k_red<KIND>, 1, 8 * NT, 0, st, R, nb);
 }
 
 template <typename T>
@@ -370,15 +422,15 @@ int bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first,
     if (ev) cudaEventRecord(ev[1], st);
     launch_after(kp, g, b, 0, st, d, M, p, V.r0, v, red);
     if (ev) cudaEventRecord(ev[2], st);
-    if (!last) launch_after(k_red<BR_ALPHA>, 1, NT, 0, st, red, R.nblocks);
+    if (!last) sum_blocks<BR_ALPHA>(red, R.nblocks, st);
     if (ev) cudaEventRecord(ev[3], st);
     launch_after(ks, g, b, 0, st, d, M, V.r, v, V.t, red);
     if (ev) cudaEventRecord(ev[4], st);
-    if (!last) launch_after(k_red<BR_OMEGA>, 1, NT, 0, st, red, R.nblocks);
+    if (!last) sum_blocks<BR_OMEGA>(red, R.nblocks, st);
     if (ev) cudaEventRecord(ev[5], st);
     launch_after(kx, g, b, 0, st, d, V.x, V.r, V.r0, p, v, V.t, red);
     if (ev) cudaEventRecord(ev[6], st);
-    if (!last_x) launch_after(k_red<BR_RHO>, 1, NT, 0, st, red, R.nblocks);
+    if (!last_x) sum_blocks<BR_RHO>(red, R.nblocks, st);
     return 4 + (last ? 0 : 2) + (last_x ? 0 : 1);
 }
 
@@ -389,7 +441,7 @@ int resid64(const Dims &d, const double *const m[6], const double *b, const doub
     const bool last = R.nblocks <= LAST_MAX_X;
     auto *k = last ? k_resid64<true> : k_resid64<false>;
     launch_after(k, solver_grid(d), solver_block(), 0, st, d, m6(m), b, x, r64, r32, red);
-    if (!last) launch_after(k_red<BR_RESID>, 1, NT, 0, st, red, R.nblocks);
+    if (!last) sum_blocks<BR_RESID>(red, R.nblocks, st);
     return last ? 1 : 2;
 }
 
