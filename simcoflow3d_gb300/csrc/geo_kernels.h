@@ -28,6 +28,26 @@ struct GeoFam {
                         (k = q_ / ((d).I * (d).J) + 1), true);                               \
          q_ += gridDim.x * blockDim.x)
 
+// Cells per column segment of the face kernel: the longest of 32, 16, .., 2 that
+// gives two waves of its three blocks per SM.  A segment start evaluates one
+// face more, a long segment is a serial chain of loads and queue barriers:
+// 96^3 (host call) 10.8 ms at 32 cells, 9.7 at 4, 9.8 at 2.  Segments of two
+// are not for flat grids whose columns alone give two blocks to each SM: two
+// segments of four hide as much as four of two, which start twice as often
+// (the four families' face kernels at 200x200x8: 0.93 ms at 8 cells, 0.89 at 4,
+// 1.05 at 2; 220x220x8 0.90, 0.90 and 1.08; with K <= 6 two cells stay better,
+// 300x150x6 1.00 ms at 4 cells and 0.92 at 2).
+inline int geo_kseg(int I, int J, int K)
+{
+    const long long cols = (long long)((I + 31) / 32) * ((J + 3) / 4);
+    int kseg = 32;
+    while (kseg > 2 && cols * ((K + kseg - 1) / kseg) < 152 * 6) {
+        if (kseg == 4 && cols >= 152 * 2 && K > 6) break;
+        kseg /= 2;
+    }
+    return kseg;
+}
+
 // DefineCell + CellGeoCal of one family; when ev is given, ev[0] and ev[1]
 // are recorded around the face kernel.
 void launch_cell_geo(const GeoFam &t, const Dims &d, int *exact_count, cudaStream_t st, int *launches,

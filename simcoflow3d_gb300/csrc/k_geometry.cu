@@ -724,13 +724,7 @@ void launch_cell_geo(const GeoFam &t, const Dims &d, int *exact_count, cudaStrea
                      cudaEvent_t *ev)
 {
     k_geo_define<<<grid_for(d.ng, 256), 256, 0, st>>>(t, d);
-    // Cells per segment: the longest of 32, 16, .., 2 that gives two waves of
-    // the face kernel's three blocks per SM.  A segment start evaluates one
-    // face more, a long segment is a serial chain of loads and queue barriers:
-    // 96^3 (host call) 10.8 ms at 32 cells, 9.7 at 4, 9.8 at 2.
-    const long long cols = (long long)((d.I + 31) / 32) * ((d.J + 3) / 4);
-    int kseg = 32;
-    while (kseg > 2 && cols * ((d.K + kseg - 1) / kseg) < 152 * 6) kseg /= 2;
+    const int kseg = geo_kseg(d.I, d.J, d.K);
     dim3 b(32, 4), g((d.I + 31) / 32, (d.J + 3) / 4, (d.K + kseg - 1) / kseg);
     if (ev) cudaEventRecord(ev[0], st);
     k_geo_faces<<<g, b, 0, st>>>(t, d, exact_count, kseg);
