@@ -974,8 +974,11 @@ __device__ __forceinline__ float band_sqrt(float a)   // within 2^-23 relative
     return r;
 }
 #else
-TR_HD float band_fma(float a, float b, float c) { return a * b + c; }
-TR_HD float band_sqrt(float a) { return sqrtf(a); }
+TR_HD float band_fma(float a, float b, float c) { return fmaf(a, b, c); }
+#if !defined(TR_SQRT_ERROR)
+#define TR_SQRT_ERROR 0.0   // host checks: the approximate square root's relative error
+#endif
+TR_HD float band_sqrt(float a) { return (float)((double)sqrtf(a) * (1.0 + TR_SQRT_ERROR)); }
 #endif
 
 // v[q] by selects: the arrays stay in registers.
