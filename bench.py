@@ -956,7 +956,7 @@ def clsvof_workload(n: int):
 
 # algorithmic bytes per interior cell of one launch: the fields a kernel must
 # read and write once (neighbours come from cache)
-CLSVOF_BYTES = {"sweep_first": 40, "sweep_later": 56, "normals": 54}
+CLSVOF_BYTES = {"sweep_first": 40, "sweep_later": 56}
 
 
 def clsvof_cpu_ms(n_full: int, sample_n: int = 64):
@@ -975,7 +975,7 @@ def run_clsvof(args):
     planes, the reconstruction and the redistancing) on the reference's
     3-D deformation test scaled to 256^3: device time with the state
     resident, the host-array call end to end, the live roofline of the
-    heaviest kernel kind, and the oracle on the host cores.  One JSON line."""
+    sweeps, and the oracle on the host cores.  One JSON line."""
     import numpy as np
     from simcoflow3d_gb300.projection import load_library
     from simcoflow3d_gb300.transport import ClsvofScheme
@@ -1008,14 +1008,11 @@ def run_clsvof(args):
     cells = n ** 3
     kinds = ("reconstruct", "sweep", "walls", "redistance")
     kms = {k: sum(t["ms_kernels"][q] for t in timed) / len(timed) for q, k in enumerate(kinds)}
-    # per step: 18 sweeps (6 first, 12 later) and 24 reconstructions, of which
-    # the 18 before the sweeps touch the partly filled cells only
+    # per step 18 sweeps (6 first, 12 later), the heaviest kind of one kernel; the
+    # reconstruction's time is that of two, most of whose launches touch the
+    # partly filled cells only
     sweep_bytes = 6 * cells * (CLSVOF_BYTES["sweep_first"] + 2 * CLSVOF_BYTES["sweep_later"])
-    rec_bytes = 6 * cells * CLSVOF_BYTES["normals"]
-    top = max(("sweep", "reconstruct"), key=lambda k: kms[k])
-    tb = {"sweep": sweep_bytes, "reconstruct": rec_bytes}[top]
-    launches = {"sweep": 18, "reconstruct": 24}[top]
-    achieved = tb / (kms[top] * 1e-3) / 1e9
+    achieved = sweep_bytes / (kms["sweep"] * 1e-3) / 1e9
     peak, peak_kind = measured_peaks()
     cpu = None
     if not args.no_cpu:
@@ -1039,10 +1036,13 @@ def run_clsvof(args):
                 "h2d_bytes_per_step": int(e2e[-1]["bytes_h2d"]), "d2h_bytes_per_step": int(e2e[-1]["bytes_d2h"]),
                 "ms_h2d": round(statistics.mean(r["ms_h2d"] for r in e2e), 3),
                 "ms_d2h": round(statistics.mean(r["ms_d2h"] for r in e2e), 3)},
-        "roofline": {"bound": "hbm", "kernel": {"sweep": "k_sweep", "reconstruct": "k_normals"}[top],
+        "roofline": {"bound": "hbm", "kernel": "k_sweep",
                      "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
-                     "peak_kind": peak_kind, "bytes_per_launch": tb // launches,
-                     "ms_per_launch": round(kms[top] / launches, 5),
+                     "peak_kind": peak_kind, "bytes_per_launch": sweep_bytes // 18,
+                     "ms_per_launch": round(kms["sweep"] / 18, 5),
+                     "kinds_launches": {"reconstruct": "18 k_partial_fluxes, 6 k_normals", "sweep": "18 k_sweep",
+                                        "walls": "6 k_walls",
+                                        "redistance": "6 each of k_band_bound, k_band_pairs, k_band_value"},
                      "kinds_ms_per_step": {k: round(v, 4) for k, v in kms.items()},
                      "timing": "CUDA events around every kernel of 2 steps", "traffic": None},
         "clocks": clocks,
