@@ -16,8 +16,7 @@
 // reproducible) and the scalars updated, which stay in device memory: by the
 // block that finishes last on grids up to LAST_MAX, else by a launch of one
 // block.  (The launches were 4 to 5 us each, three per iteration: a predictor
-// step at 67x53x75 in FP64 2570 us with them, 2280 without; at 128x112x96
-// mixed 4457 and 4205.)  The reduction after X sets `done` when
+// step at 67x53x75 in FP64 2570 us with them, 2280 without.)  The reduction after X sets `done` when
 // ||r||^2 <= target or on a breakdown, and every kernel after that returns at
 // once, so the host enqueues several iterations and reads the scalars once
 // per batch.
@@ -41,10 +40,17 @@ struct Red {
     BcgScalars *sc;
     int want_bb;
 };
-// Blocks up to which the last one sums a pass: one resident wave of P and S
-// (16 blocks per SM), half of that of X and the residual, where a block's
-// fence waits for more stores.  Beyond, the fences cost more than a launch.
-constexpr int LAST_MAX = 152 * 16, LAST_MAX_X = 152 * 8;
+// Blocks up to which the last one sums a pass.  The tail's registers (55 to 72
+// against 32 to 40 without) leave room for nine FP32 blocks of P and S per SM
+// and eight of X, and the FP32 passes live on warps in flight: beyond one such
+// wave a launch costs less (a predictor step, mixed: 128x176x128, 1408 blocks,
+// 7.36 ms with the sums in the last block of P and S and 6.31 without;
+// 320x96x130, 2160 blocks, 11.9 and 11.0; X at 128x112x96, 1344 blocks, +9%).
+// FP64 P and S are bound by their arithmetic and gain (320x96x130 24.4 ms with
+// launches, 22.6 without; 128x176x128 13.4 and 13.7).
+template <typename T>
+constexpr int LAST_MAX = sizeof(T) == 4 ? 152 * 9 : 152 * 16;
+constexpr int LAST_MAX_X = 152 * 8;
 
 // The scalars from a pass's sums, by one warp (which divides in one go).
 template <int KIND>
@@ -89,13 +95,14 @@ __device__ __forceinline__ void scalars(BcgScalars *sc, const double (&s)[red_su
 
 // The grid's sums from 1024 strided ones, a[q][j] of thread t < 128 being the
 // one that starts at block t + 128 j: a tree over their index (512, 256, ...
-// 1 apart), whose first three levels are the thread's own.
-template <int KIND>
+// 1 apart), whose first three levels are the thread's own.  WIDE: the block has
+// more threads, which hold none.
+template <int KIND, bool WIDE>
 __device__ __forceinline__ void red_tree(const Red &R, double (&a)[red_sums(KIND)][8], int t)
 {
     constexpr int Q = red_sums(KIND);
     __shared__ double sh[Q][NT];
-    if (t < NT) {
+    if (!WIDE || t < NT) {
 #pragma unroll
         for (int d = 4; d > 0; d >>= 1)
 #pragma unroll
@@ -142,7 +149,7 @@ __device__ __forceinline__ void red_tail(const Red &R, int nb)
 #pragma unroll
                 for (int q = 0; q < Q; ++q) a[q][j] += p[q][j];
     }
-    red_tree<KIND>(R, a, t);
+    red_tree<KIND, false>(R, a, t);
 }
 
 // The end of a pass: the block's sums to its partials, and with LAST the
@@ -224,7 +231,7 @@ __global__ void __launch_bounds__(8 * NT) k_red(Red R, int nb)
         for (int q = 0; q < Q; ++q)
 #pragma unroll
             for (int j = 0; j < 8; ++j) a[q][j] = strided[q][t + NT * j];
-    red_tree<KIND>(R, a, t);
+    red_tree<KIND, true>(R, a, t);
 }
 
 template <int KIND>
@@ -415,7 +422,7 @@ int bcg_iteration(const Dims &d, const T *const m[6], BcgVecs<T> &V, bool first,
     if (ev) cudaEventRecord(ev[0], st);
     launch_after(k_bcg_u<T>, g, b, 0, st, d, V.r, p, v, sc, first ? 1 : 0);
     const Red red{R.partials, R.finished, sc, 0};
-    const bool last = R.nblocks <= LAST_MAX, last_x = R.nblocks <= LAST_MAX_X;
+    const bool last = R.nblocks <= LAST_MAX<T>, last_x = R.nblocks <= LAST_MAX_X;
     auto *kp = last ? k_bcg_p<T, true> : k_bcg_p<T, false>;
     auto *ks = last ? k_bcg_s<T, true> : k_bcg_s<T, false>;
     auto *kx = last_x ? k_bcg_x<T, true> : k_bcg_x<T, false>;
