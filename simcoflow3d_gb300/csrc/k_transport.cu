@@ -8,11 +8,11 @@
 //                                  own two faces (no scatter, no atomics)
 //                                  with the divergence term fused in;
 //   k_walls                        the wall planes and ghosts;
-//   k_normals                      liquid normals and centre distances, the
-//                                  redistancing's resets and the list of the
-//                                  interface cells;
-//   k_band_bound, k_band_pairs,    the redistancing over the listed cells'
-//   k_band_value                   9^3 band pairs: FP32 bounds of every
+//   k_normals                      liquid normals and centre distances, and
+//                                  the redistancing's resets;
+//   k_band_bound, k_band_pairs,    the redistancing over the 9^3 band pairs of
+//   k_band_value                   the interface cells, which the last sweep
+//                                  has listed: FP32 bounds of every
 //                                  pair's distance leave each target its
 //                                  least upper bound, then only the pairs
 //                                  whose lower bound does not exceed it are
@@ -241,8 +241,8 @@ __global__ void __launch_bounds__(NB_THREADS) k_normals(const __grid_constant__ 
 {
     after_previous();
     if (blockIdx.x < kNormalBlocks) {
-        // thread t of block b takes entry t * blocks + b: neighbouring entries, and
-        // with them the long chains, go to different SMs
+        // 32 neighbouring entries to a warp, a warp of every block before the next
+        // of any: a short list is spread over all SMs
         const unsigned n = *count;
         for (unsigned long long q = (unsigned long long)(threadIdx.x >> 5) * kNormalBlocks * 32 + blockIdx.x * 32 +
                                     (threadIdx.x & 31);

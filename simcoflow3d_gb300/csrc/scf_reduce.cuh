@@ -3,11 +3,13 @@
 //
 // Up to one resident wave of blocks, the block that finishes last adds the
 // partials itself, so a dot product costs no launch of its own; with more
-// blocks a kernel of one block does.  (There the fence and the atomic of every
-// block, and the registers of the tail, cost more than the launch: at 256^3
-// k_cg_update_df 177 -> 217 us, k_dot_rz_df 79 -> 93.  At 40^3 a projection
-// takes 1018 us with the launches and 1001 without, at 64^3 in FP64, 1024
-// blocks, 2193 and 2175.)
+// blocks a kernel of one block does.  (There the count of every block, which
+// waits for the block's stores, and the registers of the tail cost more than
+// the launch.  A projection, mixed, with the sums in launches / in the last
+// block at any number of blocks: 256^3, 4096 blocks, 13.47 / 13.62 ms;
+// 512x256x256 27.5 / 27.7; 147x93x121, 1920 blocks, 3.20 / 3.24; 192^3 and
+// 256x128x128 the same.  At 40^3 it takes 1018 us with the launches and 1001
+// without, at 64^3 in FP64, 1024 blocks, 2193 and 2175.)
 // Either way the order of the additions is fixed: 1024 strided sums, then a
 // tree over each 32 of them and one over the 32 results.  128 threads form it
 // with the trees' upper levels as additions of registers -- 36 FP64 warp
